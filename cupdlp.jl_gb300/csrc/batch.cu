@@ -45,7 +45,8 @@ void build_seg_items(const std::vector<int32_t>& off, std::vector<SegItem>& item
   begin.assign(count + 1, 0);
   for (int k = 0; k < count; ++k) {
     begin[k] = (int32_t)items.size();
-    for (int32_t s = off[k]; s < off[k + 1]; s += kSegLen) items.push_back({s, std::min(off[k + 1], s + kSegLen), k});
+    const int32_t step = seg_len(off[k + 1] - off[k]);
+    for (int32_t s = off[k]; s < off[k + 1]; s += step) items.push_back({s, std::min(off[k + 1], s + step), k});
   }
   begin[count] = (int32_t)items.size();
   if (items.empty()) items.push_back({0, 0, 0});
@@ -310,7 +311,7 @@ struct BatchWorkspace {
   DBuf<T> y0, y1, kx0, kx1, sy, skx, ay, akx, ry, rkx;
   DBuf<StepState> st_dev;
   PinnedBuf<StepState> st_host;
-  DBuf<double> part_p, part_d, red_part, red_out;
+  DBuf<double> part_p, part_d, red_part_n, red_part_m, red_out;
   DBuf<double> rvar, rcon;   // 1 / variable and 1 / constraint rescaling (evaluation divisions)
   PinnedBuf<double> red_host;
   TilePlan<T> plan_p, plan_d;   // tiles of the packed A' and A, instance by instance
@@ -318,7 +319,7 @@ struct BatchWorkspace {
   // launched CTAs: those of instances not yet retired (rebuilt when their count halves)
   DBuf<int32_t> map_p, map_d;
   int grid_p = 0, grid_d = 0;
-  DBuf<uint8_t> flags;             // 4 x count: active, use_current, to_avg, restart
+  DBuf<uint8_t> flags;             // 3 x count: evaluated, to_avg, restart
   PinnedBuf<uint8_t> flags_host;
   cudaGraphExec_t graphs[kBatchLevels] = {};
   long long launches = 0;
@@ -338,8 +339,8 @@ struct BatchWorkspace {
   }
 
   explicit BatchWorkspace(gpdhg_batch* b_) : B(b_), count(b_->count), N(b_->N), M(b_->M),
-                                             st_host(b_->count), red_host((size_t)b_->count * 32),
-                                             flags_host(4 * (size_t)b_->count) {
+                                             st_host(b_->count), red_host((size_t)b_->count * kEvalStride),
+                                             flags_host(3 * (size_t)b_->count) {
     PhaseTrace tr;
     cudaStream_t s = B->stream;
     if constexpr (sizeof(T) == sizeof(double)) {
@@ -379,9 +380,10 @@ struct BatchWorkspace {
     part_d.alloc(2 * (size_t)plan_d.num_ctas);
     part_p_split.alloc(std::max(plan_p.num_splits, 1));
     part_d_split.alloc(2 * (size_t)std::max(plan_d.num_splits, 1));
-    red_part.alloc((size_t)16 * std::max(B->nseg_n, B->nseg_m));
-    red_out.alloc((size_t)count * 32);
-    flags.alloc(4 * (size_t)count);
+    red_part_n.alloc((size_t)kPassNQ * B->nseg_n);
+    red_part_m.alloc((size_t)kPassMQ * B->nseg_m);
+    red_out.alloc((size_t)count * kEvalStride);
+    flags.alloc(3 * (size_t)count);
     compact(std::vector<char>(count, 0));
     tr.mark("batch ws: CTA maps, graphs");
   }
@@ -473,31 +475,33 @@ struct BatchWorkspace {
     CK(cudaStreamSynchronize(B->stream));
   }
   void push_flags() {
-    CK(cudaMemcpyAsync(flags.get(), flags_host.p, 4 * (size_t)count, cudaMemcpyHostToDevice, B->stream));
+    CK(cudaMemcpyAsync(flags.get(), flags_host.p, 3 * (size_t)count, cudaMemcpyHostToDevice, B->stream));
     CK(cudaStreamSynchronize(B->stream));
   }
   uint8_t* active() { return flags.get(); }
-  uint8_t* use_current() { return flags.get() + count; }
-  uint8_t* to_avg() { return flags.get() + 2 * count; }
-  uint8_t* restart() { return flags.get() + 3 * count; }
+  uint8_t* to_avg() { return flags.get() + count; }
+  uint8_t* restart() { return flags.get() + 2 * count; }
   BatchVecArgs<T> vn(const uint8_t* flag) const { return BatchVecArgs<T>{B->col_inst.get(), flag, st_dev.get(), N}; }
   BatchVecArgs<T> vm(const uint8_t* flag) const { return BatchVecArgs<T>{B->row_inst.get(), flag, st_dev.get(), M}; }
   int grid(int len) const { return std::max(1, std::min(ceil_div(len, kBlock), 4096)); }
 
+  // one side's pass over the segments of the evaluated instances (StepState::eval_active)
   template <int Q, unsigned MAXMASK, class F>
-  void seg_reduce(bool n_side, F f, int out_offset) {
+  void seg_reduce(bool n_side, F f) {
     const int nit = n_side ? B->nseg_n : B->nseg_m;
-    const SegItem* items = n_side ? B->seg_n.get() : B->seg_m.get();
-    const int32_t* beg = n_side ? B->seg_n_begin.get() : B->seg_m_begin.get();
-    seg_reduce_kernel<Q, MAXMASK, F><<<nit, kBlock, 0, B->stream>>>(items, active(), f, red_part.get(), nit);
+    seg_reduce_kernel<Q, MAXMASK, F><<<nit, kBlock, 0, B->stream>>>(
+        n_side ? B->seg_n.get() : B->seg_m.get(), st_dev.get(), f, n_side ? red_part_n.get() : red_part_m.get(), nit);
     CK_LAUNCH();
-    seg_finalize_kernel<Q, MAXMASK><<<count, kBlock, 0, B->stream>>>(beg, active(), red_part.get(), nit,
-                                                                      red_out.get() + out_offset, 32);
-    CK_LAUNCH();
-    launches += 2;
+    ++launches;
   }
-  void fetch() {
-    CK(cudaMemcpyAsync(red_host.p, red_out.get(), sizeof(double) * 32 * count, cudaMemcpyDeviceToHost, B->stream));
+  void finish_reductions() {
+    const SegSide m{B->seg_m_begin.get(), red_part_m.get(), red_out.get(), B->nseg_m, kPassMQ, kEvalMMax};
+    const SegSide n{B->seg_n_begin.get(), red_part_n.get(), red_out.get() + kEvalOutN, B->nseg_n, kPassNQ, kEvalNMax};
+    seg_finalize_kernel<<<dim3(kPassMQ + kPassNQ, count), kBlock, 0, B->stream>>>(m, n, st_dev.get());
+    CK_LAUNCH();
+    ++launches;
+    CK(cudaMemcpyAsync(red_host.p, red_out.get(), sizeof(double) * kEvalStride * count, cudaMemcpyDeviceToHost,
+                       B->stream));
     CK(cudaStreamSynchronize(B->stream));
   }
 };
@@ -522,6 +526,7 @@ static void run_batch(gpdhg_batch* B, BatchWorkspace<T>& W, const gpdhg_params& 
   CK(cudaMemcpyAsync(W.rgrad.get(), W.c, sizeof(T) * N, cudaMemcpyDeviceToDevice, s));
   std::vector<long long> iteration(K, 1);
   std::vector<RestartMemory> mem(K);
+  std::vector<RestartKkt> restart_kkt(K);
   std::vector<char> retired(K, 0), due(K, 1);
   std::vector<double> basic(K, 0.0);
   StepState* st = W.st_host.p;
@@ -550,62 +555,55 @@ static void run_batch(gpdhg_batch* B, BatchWorkspace<T>& W, const gpdhg_params& 
   long long rounds = 0;
   while (alive > 0) {
     // ---- evaluate every instance that reached its evaluation point ----
-    std::memset(fh, 0, 4 * (size_t)K);
+    std::memset(fh, 0, 3 * (size_t)K);
     bool any = false;
-    for (int k = 0; k < K; ++k)
-      if (!retired[k] && due[k]) {
-        fh[k] = 1;
-        fh[K + k] = (st[k].numerical_error || st[k].count_primal == 0 || st[k].count_dual == 0) ? 1 : 0;
-        if (!fh[K + k]) {
-          st[k].rcp_w_primal = 1.0 / st[k].sum_w_primal;
-          st[k].rcp_w_dual = 1.0 / st[k].sum_w_dual;
-        }
-        st[k].kkt_passes += 2.0;
-        st[k].done = 0;
-        any = true;
-      } else {
-        st[k].done = 1;  // not being evaluated: keep its kernels idle
-      }
+    for (int k = 0; k < K; ++k) {
+      StepState& q = st[k];
+      q.eval_active = !retired[k] && due[k] ? 1 : 0;
+      q.done = q.eval_active ? 0 : 1;  // not being evaluated: keep its kernels idle
+      if (!q.eval_active) continue;
+      fh[k] = 1;
+      q.eval_current = (q.numerical_error || q.count_primal == 0 || q.count_dual == 0) ? 1 : 0;
+      q.eval_restart = restart_kkt[k].valid ? 0 : 1;
+      q.rcp_w_primal = q.eval_current ? 0.0 : 1.0 / q.sum_w_primal;
+      q.rcp_w_dual = q.eval_current ? 0.0 : 1.0 / q.sum_w_dual;
+      q.kkt_passes += 2.0;
+      any = true;
+    }
     if (any) {
       W.push_state();
       W.push_flags();
-      W.launch_pair(kStepCommitOnly);
-      CK_LAUNCH();
-      for (int k = 0; k < K; ++k)
-        if (fh[k]) st[k].pending_commit = 0;
-      // y-bar first, then the averages' K'y = A' y-bar of the instances evaluated now (as the
-      // lone solve forms it), then x-bar and the average gradient
-      if (M) {
-        batch_average_m_kernel<T><<<W.grid(M), kBlock, 0, s>>>(W.vm(W.active()), W.use_current(), W.sy.get(),
-                                                               W.skx.get(), W.y0.get(), W.y1.get(), W.kx0.get(),
-                                                               W.kx1.get(), W.ay.get(), W.akx.get());
-        CK_LAUNCH();
-      }
+      // as the lone solve: the pending step's column side, the row pass, A' y-bar, the column pass
+      launch_step(primal_step_kernel<T>, W.grid_p, s, W.pargs(kStepCommitOnly));
+      W.template seg_reduce<kPassMQ, kEvalMMax>(
+          false, EvalPassM<T>{B->con.get(), W.rcon.get(), B->ob.get(), W.b, W.y0.get(), W.y1.get(), W.kx0.get(),
+                              W.kx1.get(), W.ry.get(), W.rkx.get(), W.sy.get(), W.skx.get(), W.ay.get(), W.akx.get(), 0,
+                              B->ineq_flag.get()});
       if (B->At.num_items > 0) {
         spmv_kernel<T><<<B->At.num_items, kBlock, 0, s>>>(B->At.view<T>(), W.ay.get(), W.aty.get(), B->col_inst.get(),
                                                           W.active());
         CK_LAUNCH();
       }
-      batch_average_n_kernel<T><<<W.grid(N), kBlock, 0, s>>>(W.vn(W.active()), W.use_current(), W.sx.get(),
-                                                             W.aty.get(), W.c, W.x.get(), W.grad.get(), W.ax.get(),
-                                                             W.agrad.get());
-      CK_LAUNCH();
-      W.launches += 3;
-      W.template seg_reduce<kEvalNQ, kEvalNMax>(
-          true, EvalN<T>{W.ax.get(), W.agrad.get(), B->var.get(), W.rvar.get(), B->ol.get(), B->ou.get(), B->oc.get()},
-          0);
-      W.template seg_reduce<kEvalMQ, kEvalMMax>(
-          false, EvalM<T>{W.ay.get(), W.akx.get(), B->con.get(), W.rcon.get(), B->ob.get(), 0, B->ineq_flag.get()},
-          16);
-      W.fetch();
-      bool any_restart_check = false;
-      std::vector<char> check(K, 0);
+      W.launches += 2;
+      W.template seg_reduce<kPassNQ, kEvalNMax>(
+          true, EvalPassN<T>{B->var.get(), W.rvar.get(), B->ol.get(), B->ou.get(), B->oc.get(), W.l, W.u, W.c,
+                             W.x.get(), W.sx.get(), W.aty.get(), W.kty.get(), W.rx.get(), W.rgrad.get(), W.ax.get(),
+                             W.agrad.get(), W.grad.get()});
+      W.finish_reductions();
+      bool any_restart = false;
+      std::vector<uint8_t> ta(K, 0), rs(K, 0);
       for (int k = 0; k < K; ++k) {
         if (!fh[k]) continue;
-        const double* en = W.red_host.p + (size_t)32 * k;
+        st[k].pending_commit = 0;
+        const double* em = W.red_host.p + (size_t)kEvalStride * k;
+        const double* en = em + kEvalOutN;
+        double kn[kKktNQ], km[kKktMQ];
+        std::memcpy(kn, en + kEvalNQ, sizeof(kn));
+        std::memcpy(km, em + kEvalMQ, sizeof(km));
+        restart_kkt[k].keep_or_fill(kn, km);
         gpdhg_iteration_stats stats;
         std::memset(&stats, 0, sizeof(stats));
-        assemble_stats(B->info[k], prm, en, en + 16, stats);
+        assemble_stats(B->info[k], prm, en, em, stats);
         const long long it = iteration[k];
         stats.iteration_number = (int32_t)(it - 1);
         stats.cumulative_kkt_matrix_passes = st[k].kkt_passes;
@@ -651,78 +649,38 @@ static void run_batch(gpdhg_batch* B, BatchWorkspace<T>& W, const gpdhg_params& 
           if (on_retire) (*on_retire)(k);
           continue;
         }
-        if (st[k].count_primal > 0 && st[k].count_dual > 0) {
-          check[k] = 1;
-          any_restart_check = true;
-        }
+        // run_restart_scheme for the instances that have an average
+        if (st[k].count_primal == 0 || st[k].count_dual == 0) continue;
+        const RestartDecision dec =
+            decide_restart(prm, B->info[k], st[k].count_primal, st[k].tau, st[k].omega, iteration[k] - 1, kn, km, mem[k]);
+        if (dec.restart_used == GPDHG_RESTART_CHOICE_NO_RESTART) continue;
+        rs[k] = 1;
+        ta[k] = dec.reset_to_average ? 1 : 0;
+        restart_kkt[k].valid = false;
+        st[k].count_primal = st[k].count_dual = 0;
+        st[k].sum_w_primal = st[k].sum_w_dual = 0.0;
+        st[k].omega = dec.new_omega;
+        any_restart = true;
       }
-      // buffer_primal_gradient = c - K'y (:742) for every instance that goes on
-      for (int k = 0; k < K; ++k) fh[k] = (!retired[k] && due[k]) ? 1 : 0;
-      W.push_flags();
-      batch_grad_kernel<T><<<W.grid(N), kBlock, 0, s>>>(W.vn(W.active()), W.c, W.kty.get(), W.grad.get());
-      CK_LAUNCH();
-      ++W.launches;
-      // run_restart_scheme for the instances that have an average
-      for (int k = 0; k < K; ++k) fh[k] = check[k];
-      if (any_restart_check) {
-        W.push_flags();
-        KktN<T> kn{W.l, W.u, W.c, W.x.get(), W.ax.get(), W.rx.get(), W.grad.get(), W.agrad.get(), W.rgrad.get()};
-        W.template seg_reduce<kKktNQ, 0u>(true, kn, 0);
-        W.fetch();
-        std::vector<double> knv((size_t)32 * K);
-        std::memcpy(knv.data(), W.red_host.p, sizeof(double) * 32 * K);
-        // m side: one launch per buffer parity, so each instance reads its current y and K x
-        for (int par = 0; par < 2; ++par) {
-          bool have = false;
-          for (int k = 0; k < K; ++k) {
-            fh[k] = check[k] && st[k].parity == par;
-            have |= fh[k] != 0;
-          }
-          if (!have) continue;
-          W.push_flags();
-          KktM<T> km{W.b, par ? W.y1.get() : W.y0.get(), W.ay.get(), W.ry.get(),
-                     par ? W.kx1.get() : W.kx0.get(), W.akx.get(), W.rkx.get(), 0, B->ineq_flag.get()};
-          W.template seg_reduce<kKktMQ, 0u>(false, km, 16);
-        }
-        for (int k = 0; k < K; ++k) fh[k] = check[k];
-        W.fetch();
-        bool any_restart = false;
-        std::vector<uint8_t> ta(K, 0), rs(K, 0);
+      if (any_restart) {
         for (int k = 0; k < K; ++k) {
-          if (!check[k]) continue;
-          const double* kn = knv.data() + (size_t)32 * k;
-          const double* kmv = W.red_host.p + (size_t)32 * k + 16;
-          const RestartDecision dec =
-              decide_restart(prm, B->info[k], st[k].count_primal, st[k].tau, st[k].omega, iteration[k] - 1, kn, kmv, mem[k]);
-          if (dec.restart_used != GPDHG_RESTART_CHOICE_NO_RESTART) {
-            rs[k] = 1;
-            ta[k] = dec.reset_to_average ? 1 : 0;
-            st[k].count_primal = st[k].count_dual = 0;
-            st[k].sum_w_primal = st[k].sum_w_dual = 0.0;
-            st[k].omega = dec.new_omega;
-            any_restart = true;
-          }
+          fh[k] = rs[k];
+          fh[K + k] = ta[k];
         }
-        if (any_restart) {
-          for (int k = 0; k < K; ++k) {
-            fh[k] = rs[k];
-            fh[2 * K + k] = ta[k];
-          }
-          W.push_flags();
-          W.push_state();  // restart kernels read each instance's parity
-          batch_restart_n_kernel<T><<<W.grid(N), kBlock, 0, s>>>(W.vn(W.active()), W.to_avg(), W.ax.get(),
-                                                                 W.agrad.get(), W.c, W.x.get(), W.kty.get(),
-                                                                 W.grad.get(), W.sx.get(), W.rx.get(), W.rgrad.get());
+        W.push_flags();
+        W.push_state();  // restart kernels read each instance's parity
+        batch_restart_n_kernel<T><<<W.grid(N), kBlock, 0, s>>>(W.vn(W.active()), W.to_avg(), W.ax.get(),
+                                                               W.agrad.get(), W.c, W.x.get(), W.kty.get(),
+                                                               W.grad.get(), W.sx.get(), W.rx.get(), W.rgrad.get());
+        CK_LAUNCH();
+        if (M) {
+          batch_restart_m_kernel<T><<<W.grid(M), kBlock, 0, s>>>(W.vm(W.active()), W.to_avg(), W.ay.get(),
+                                                                 W.akx.get(), W.y0.get(), W.y1.get(), W.kx0.get(),
+                                                                 W.kx1.get(), W.sy.get(), W.skx.get(), W.ry.get(),
+                                                                 W.rkx.get());
           CK_LAUNCH();
-          if (M) {
-            batch_restart_m_kernel<T><<<W.grid(M), kBlock, 0, s>>>(W.vm(W.active()), W.to_avg(), W.ay.get(),
-                                                                   W.akx.get(), W.y0.get(), W.y1.get(), W.kx0.get(),
-                                                                   W.kx1.get(), W.sy.get(), W.skx.get(), W.ry.get(),
-                                                                   W.rkx.get());
-            CK_LAUNCH();
-          }
-          W.launches += 2;
         }
+        W.launches += 2;
       }
       // re-arm: take_step! calls until each instance's next evaluation
       for (int k = 0; k < K; ++k) {

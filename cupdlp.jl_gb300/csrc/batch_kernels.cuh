@@ -1,5 +1,5 @@
 // batch_kernels.cuh — step and evaluation kernels for many LPs packed into one
-// block-diagonal ("segmented") CSR.
+// block-diagonal ("segmented") CSR; a lone LP is evaluated by the same kernels.
 //
 // Every row-block item of the packed A and A' belongs to exactly one instance, and an
 // instance's items are built exactly as for a lone solve, so each instance sees the same
@@ -15,44 +15,59 @@
 namespace gpdhg {
 
 // ---- segmented FP64 reductions --------------------------------------------------
-// A segment item is a contiguous element range of one instance; partials are written
-// per item, and one CTA per instance reduces its items in order.
+// A segment item is a contiguous element range of one instance, reduced by one CTA into its
+// partials; then one CTA per instance and quantity reduces the instance's items in order. (One
+// CTA per instance for all quantities took 15-34 us on 1,000-2,000 items, its loads of 25
+// quantities one after the other; one CTA each takes 6 us.) st NULL: every instance is active.
+// The passes are bound by the FP64 pipe (62-84% busy) and the latency of a thread's dozen loads,
+// so 3 CTAs per SM (80 registers, 50 bytes spilled in the column pass; 2 CTAs: 107 us against
+// 70). Cold-cache times, plainly written FP64 arithmetic -> now: column pass of the transportation
+// LP (1M columns, FP64) 194 -> 70 us, of the power-law LP (2M, FP32) 428 -> 138 us, its row pass
+// (1M rows) 127 -> 63-70 us.
 template <int Q, unsigned MAXMASK, class F>
-__global__ void __launch_bounds__(kBlock) seg_reduce_kernel(const SegItem* items, const uint8_t* active, F f,
+__global__ void __launch_bounds__(kBlock, 3) seg_reduce_kernel(const SegItem* items, const StepState* st, F f,
                                                             double* partials, int num_items) {
   __shared__ double sh[(Q < kRedChunk ? Q : kRedChunk) * kBlock];
   __shared__ double res[Q];
   const SegItem it = items[blockIdx.x];
-  if (!active[it.inst]) return;
+  if (st && !st[it.inst].eval_active) return;
+  const typename F::Params p(st, it.inst);
   double acc[Q];
 #pragma unroll
   for (int q = 0; q < Q; ++q) acc[q] = 0.0;
-  for (int i = it.begin + threadIdx.x; i < it.end; i += kBlock) f((long long)i, acc);
+  for (int i = it.begin + threadIdx.x; i < it.end; i += kBlock) f(p, i, acc);
   const double r = block_reduce_q<Q, MAXMASK>(acc, sh, res);
   if ((int)threadIdx.x < Q) partials[(size_t)threadIdx.x * num_items + blockIdx.x] = r;
 }
 
-template <int Q, unsigned MAXMASK>
-__global__ void __launch_bounds__(kBlock) seg_finalize_kernel(const int32_t* inst_item_begin, const uint8_t* active,
-                                                              const double* partials, int num_items, double* out,
-                                                              int out_stride) {
-  __shared__ double sh[(Q < kRedChunk ? Q : kRedChunk) * kBlock];
-  __shared__ double res[Q];
-  const int inst = blockIdx.x;
-  if (!active[inst]) return;
-  const int k0 = inst_item_begin[inst], k1 = inst_item_begin[inst + 1];
-  double acc[Q];
-#pragma unroll
-  for (int q = 0; q < Q; ++q) acc[q] = 0.0;
-  for (int k = k0 + threadIdx.x; k < k1; k += kBlock) {
-#pragma unroll
-    for (int q = 0; q < Q; ++q) {
-      const double v = partials[(size_t)q * num_items + k];
-      acc[q] = ((MAXMASK >> q) & 1u) ? nan_max(acc[q], v) : acc[q] + v;
-    }
-  }
-  const double r = block_reduce_q<Q, MAXMASK>(acc, sh, res);
-  if ((int)threadIdx.x < Q) out[(size_t)inst * out_stride + threadIdx.x] = r;
+// Where one side's partials lie and where its results go (quantity q of instance k at
+// out[k * kEvalStride + q]).
+struct SegSide {
+  const int32_t* inst_item_begin;
+  const double* partials;
+  double* out;
+  int num_items;
+  int quantities;
+  unsigned maxmask;
+};
+constexpr int kEvalStride = 64;   // results per instance: rows' at 0, columns' at kEvalOutN
+constexpr int kEvalOutN = 32;
+// Grid (quantities of both sides, instances).
+inline __global__ void __launch_bounds__(kBlock) seg_finalize_kernel(SegSide a, SegSide b, const StepState* st) {
+  __shared__ double sh[32];
+  const int inst = blockIdx.y;
+  if (st && !st[inst].eval_active) return;
+  const bool second = (int)blockIdx.x >= a.quantities;
+  const SegSide& s = second ? b : a;
+  const int q = (int)blockIdx.x - (second ? a.quantities : 0);
+  const bool is_max = (s.maxmask >> q) & 1u;
+  const double* p = s.partials + (size_t)q * s.num_items;
+  const int k1 = s.inst_item_begin[inst + 1];
+  double acc = 0.0;
+  for (int k = s.inst_item_begin[inst] + (int)threadIdx.x; k < k1; k += kBlock)
+    acc = is_max ? nan_max(acc, p[k]) : acc + p[k];
+  acc = is_max ? block_nan_max(acc, sh) : block_sum(acc, sh);
+  if (threadIdx.x == 0) s.out[(size_t)inst * kEvalStride + q] = acc;
 }
 
 // Per-element helpers driven by per-instance flags / weights.
@@ -63,51 +78,6 @@ struct BatchVecArgs {
   const StepState* st;
   int len;
 };
-
-// compute_average! (or the current point when the instance has no average yet), the average's
-// K'y given as aty = A' y-bar
-template <class T>
-__global__ void batch_average_n_kernel(BatchVecArgs<T> v, const uint8_t* use_current, const T* sx, const T* aty,
-                                       const T* c, const T* x, const T* grad, T* ax, T* agrad) {
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < v.len; j += gridDim.x * blockDim.x) {
-    const int k = v.inst_of[j];
-    if (!v.flag[k]) continue;
-    if (use_current[k]) {
-      ax[j] = x[j];
-      agrad[j] = grad[j];
-    } else {
-      const StepState& q = v.st[k];
-      ax[j] = (T)div_rcp((double)sx[j], q.sum_w_primal, q.rcp_w_primal);
-      agrad[j] = c[j] - aty[j];  // aty = A' y-bar
-    }
-  }
-}
-
-template <class T>
-__global__ void batch_average_m_kernel(BatchVecArgs<T> v, const uint8_t* use_current, const T* sy, const T* skx,
-                                       const T* y0, const T* y1, const T* kx0, const T* kx1, T* ay, T* akx) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < v.len; i += gridDim.x * blockDim.x) {
-    const int k = v.inst_of[i];
-    if (!v.flag[k]) continue;
-    if (use_current[k]) {
-      const int p = v.st[k].parity;
-      ay[i] = p ? y1[i] : y0[i];
-      akx[i] = p ? kx1[i] : kx0[i];
-    } else {
-      const StepState& q = v.st[k];
-      ay[i] = (T)div_rcp((double)sy[i], q.sum_w_dual, q.rcp_w_dual);
-      akx[i] = (T)div_rcp((double)skx[i], q.sum_w_primal, q.rcp_w_primal);
-    }
-  }
-}
-
-template <class T>
-__global__ void batch_grad_kernel(BatchVecArgs<T> v, const T* c, const T* kty, T* grad) {
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < v.len; j += gridDim.x * blockDim.x) {
-    if (!v.flag[v.inst_of[j]]) continue;
-    grad[j] = c[j] - kty[j];
-  }
-}
 
 // Restart actions (src/saddle_point_gpu.jl:575-614) for the instances with flag set:
 // to_avg[k] selects reset-to-average; sums are cleared; the restart point is stored.

@@ -117,8 +117,11 @@ struct StepState {
   double half_w_dx2;       // 0.5 * omega * ||dx|| * ||dx||: the primal part of the movement
   double half_over_omega;  // 0.5 / omega
   double f1, f2;           // step-size factors for this attempt's counter
-  // 1 / sum_w_primal and 1 / sum_w_dual, set by the host before an evaluation averages
+  // set by the host before an evaluation: 1 / sum_w_primal and 1 / sum_w_dual, whether the
+  // instance is evaluated, whether it has no average yet (the current point stands in), and
+  // whether the last restart point's KKT ingredients are needed
   double rcp_w_primal, rcp_w_dual;
+  int eval_active, eval_current, eval_restart, pad;
 };
 
 // ----------------------------------------------------------------------------------

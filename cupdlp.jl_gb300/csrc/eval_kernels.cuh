@@ -14,28 +14,64 @@
 
 namespace gpdhg {
 
+// A double's bits and back through a move the compiler does not look into: given a plain bit cast
+// it recognises masks of the sign bit as |v| and -v, and range tests as FP64 comparisons, and emits
+// FP64-pipe instructions for them (7 of the 14 that a column of gpdhg_convergence_noalloc took).
+__device__ __forceinline__ unsigned long long bits_of(double v) {
+  unsigned long long b;
+  asm("mov.b64 %0, %1;" : "=l"(b) : "d"(v));
+  return b;
+}
+__device__ __forceinline__ double of_bits(unsigned long long b) {
+  double v;
+  asm("mov.b64 %0, %1;" : "=d"(v) : "l"(b));
+  return v;
+}
+constexpr unsigned long long kSignBit = 0x8000000000000000ULL;
+constexpr unsigned long long kInfBits = 0x7ff0000000000000ULL;
+
 // The evaluation's max-quantities are all magnitudes (|v|, or a positive part): their
 // NaN-propagating maximum is the integer maximum of the bit patterns with the sign cleared
 // (+0 < ... < +inf < NaN), done on the integer pipe instead of GB300's narrow FP64 pipe.
 __device__ __forceinline__ double nan_max(double a, double b) {
-  const unsigned long long ua = (unsigned long long)__double_as_longlong(a) & 0x7fffffffffffffffULL;
-  const unsigned long long ub = (unsigned long long)__double_as_longlong(b) & 0x7fffffffffffffffULL;
-  return __longlong_as_double((long long)(ua > ub ? ua : ub));
+  const unsigned long long ua = bits_of(a) & ~kSignBit, ub = bits_of(b) & ~kSignBit;
+  return of_bits(ua > ub ? ua : ub);
 }
 
-__device__ __forceinline__ bool bits_nan(long long b) { return (b & 0x7fffffffffffffffLL) > 0x7ff0000000000000LL; }
+__device__ __forceinline__ bool bits_nan(double v) { return (bits_of(v) & ~kSignBit) > kInfBits; }
+__device__ __forceinline__ bool bits_zero(double v) { return (bits_of(v) << 1) == 0; }
+__device__ __forceinline__ bool bits_negative(double v) { return (long long)bits_of(v) < 0; }
+__device__ __forceinline__ bool bits_finite(double v) { return (bits_of(v) & kInfBits) != kInfBits; }
+__device__ __forceinline__ double negate_bits(double v) { return of_bits(bits_of(v) ^ kSignBit); }
 
-// Julia's max(v, 0) and min(v, 0) (NaN-propagating), by sign and NaN tests on the bits.
+// Julia's max(v, 0) (NaN-propagating), by sign and NaN tests on the bits.
 __device__ __forceinline__ double pos_part(double v) {
-  const long long b = __double_as_longlong(v);
-  return (b > 0 || bits_nan(b)) ? v : 0.0;  // +x (x != 0) and NaN kept; -x, -0, +0 -> +0
+  const unsigned long long b = bits_of(v);
+  return of_bits((long long)b > 0 || bits_nan(v) ? b : 0);  // +x (x != 0) and NaN kept; -x, -0, +0 -> +0
 }
-__device__ __forceinline__ double neg_part(double v) {
-  const long long b = __double_as_longlong(v);
-  return ((b < 0 && (b & 0x7fffffffffffffffLL) != 0) || bits_nan(b)) ? v : 0.0;
+
+// (double)v. A float's conversion runs on the FP64 pipe; the exponent is re-biased on the integer
+// pipe instead (a subnormal is first made normal by an exact FP32 product with 2^24).
+__device__ __forceinline__ double widen(double v) { return v; }
+__device__ __forceinline__ double widen(float v) {
+  unsigned mag = __float_as_uint(v) & 0x7fffffffu, bias = 0x38000000u;
+  if (mag < 0x00800000u) {
+    mag = __float_as_uint(__uint_as_float(mag) * 16777216.0f);
+    bias = mag ? 0x38000000u - (24u << 20) : 0u;
+  } else if (mag >= 0x7f800000u) {
+    bias = 0x70000000u;   // infinite and NaN: to the top exponent
+  }
+  const unsigned hi = (__float_as_uint(v) & 0x80000000u) | ((mag >> 3) + bias);
+  return of_bits((unsigned long long)hi << 32 | (unsigned)(mag << 29));
 }
-__device__ __forceinline__ bool bits_finite(double v) {
-  return (__double_as_longlong(v) & 0x7ff0000000000000LL) != 0x7ff0000000000000LL;
+// c += a b where p holds, skipped by a warp in which it holds nowhere. (Written as a plain
+// condition, a predicated instruction or a vote around the C expression, the FMA is moved out and
+// computed for every element; a volatile one stays behind the vote.)
+__device__ __forceinline__ void fma_if(bool p, double a, double b, double& c) {
+  if (!__any_sync(__activemask(), p)) return;
+  a = of_bits(p ? bits_of(a) : 0ULL);
+  b = of_bits(p ? bits_of(b) : 0ULL);
+  asm volatile("fma.rn.f64 %0, %1, %2, %0;" : "+d"(c) : "d"(a), "d"(b));
 }
 
 __device__ __forceinline__ double warp_nan_max(double v) {
@@ -98,249 +134,248 @@ __device__ __forceinline__ double block_reduce_q(const double* acc, double* sh, 
 // are returned as they are, which keeps the quotient's sign and infinities.
 __device__ __forceinline__ double div_rcp(double a, double b, double r) {
   const double q = a * r;
-  const long long bq = __double_as_longlong(q) & 0x7fffffffffffffffLL;
-  if (bq == 0 || bq >= 0x7ff0000000000000LL) return q;
+  if (!bits_finite(q) || bits_zero(q)) return q;
   const double e = fma(-q, b, a);
   return fma(e, r, q);
 }
 
-__device__ __forceinline__ double reduced_cost(double g, bool fl, bool fu) {
-  // src/iteration_stats_utils_gpu.jl:168: max(g,0)*isfinite(l) + min(g,0)*isfinite(u). At
-  // most one term is nonzero unless g is NaN (then the sum is NaN), so the sum is a select.
-  const double p = fl ? pos_part(g) : 0.0;
-  const double q = fu ? neg_part(g) : 0.0;
-  const long long bp = __double_as_longlong(p);
-  return (bp != 0) ? p : q;  // p is +0 or a positive value / NaN
+// The statistics below are written so that the FP64 pipe (2 lanes per SM and cycle: a warp-wide
+// FP64 instruction takes it for 16 cycles) only sees operations whose result is not known from the
+// operands' bits. Measured on the transportation LP (1M columns, FP64): 79 FP64 operations per
+// column when written plainly, the negations and absolute values among them (both compile to
+// FP64 additions), the pipe 81% busy.
+
+// Squared and largest violation of l <= x <= u: (l - x)+ and (x - u)+
+// (src/iteration_stats_utils_gpu.jl:71-90). A projected iterate, or an average of some, violates
+// its bounds by rounding at most, so the arithmetic sits behind a comparison of order keys; it
+// also runs for non-finite operands, which then propagate as in the plain form.
+__device__ __forceinline__ long long bits_key(double v) {   // order_key without a bit cast
+  const long long b = (long long)bits_of(v);
+  return b ^ (long long)((unsigned long long)(b >> 63) >> 1);
 }
-__device__ __forceinline__ double rc_contribution(double rc, double l, double u) {
-  // src/iteration_stats_utils_gpu.jl:120-126 (rc > 0, rc < 0 tested on the bits)
-  const long long b = __double_as_longlong(rc);
-  if (bits_nan(b) || (b & 0x7fffffffffffffffLL) == 0) return 0.0;  // neither rc > 0 nor rc < 0
-  return b > 0 ? l * rc : u * rc;
+__device__ __forceinline__ void add_violation(double x, double l, double u, double& sq, double& mx) {
+  const long long k = bits_key(x);
+  const bool below = k < bits_key(l), above = bits_key(u) < k;
+  const bool plain = !bits_finite(x) || bits_nan(l) || bits_nan(u) || (below && above);
+  if (!(below || above || plain)) return;
+  if (plain) {
+    const double lv = pos_part(l - x), uv = pos_part(x - u);
+    sq += lv * lv + uv * uv;
+    mx = nan_max(mx, nan_max(lv, uv));
+  } else {
+    const double v = of_bits(bits_of(below ? l : x)) - of_bits(bits_of(below ? x : u));
+    sq = fma(v, v, sq);
+    mx = nan_max(mx, v);
+  }
+}
+__device__ __forceinline__ void add_square(double v, double& sq) {
+  fma_if(!bits_zero(v), v, v, sq);
 }
 
-// Unscaled primal-side statistics of the averaged iterate (original problem).
+// Reduced cost of gradient g: max(g, 0) isfinite(l) + min(g, 0) isfinite(u)
+// (src/iteration_stats_utils_gpu.jl:168) is g itself or 0, so it and the dual residual g - rc are
+// selections (NaN where the plain form is: g NaN, or infinite and kept).
+__device__ __forceinline__ bool keeps_cost(double g, bool fl, bool fu) {
+  if (bits_nan(g)) return fl || fu;
+  return !bits_zero(g) && (bits_negative(g) ? fu : fl);
+}
+__device__ __forceinline__ double cost_residual(double g, bool kept) {
+  return of_bits(!kept ? bits_of(g) : bits_finite(g) ? 0ULL : kInfBits | 1ULL << 51);
+}
+// Adds the dual objective's term of a kept reduced cost (:120-126): l rc for rc > 0, u rc for
+// rc < 0, nothing for NaN; a zero bound adds nothing to a finite rc.
+__device__ __forceinline__ void add_bound_term(double g, bool kept, double l, double u, double& sum) {
+  const double bound = of_bits(bits_negative(g) ? bits_of(u) : bits_of(l));
+  fma_if(kept && !bits_nan(g) && (!bits_zero(bound) || !bits_finite(g)), bound, g, sum);
+}
+// The constraint violation b - Kx, or its positive part on an inequality row (:26-45).
+__device__ __forceinline__ double row_violation(double d, bool ineq) {
+  return of_bits(bits_of(ineq ? pos_part(d) : d));
+}
+// (-y)+ of an inequality row's dual (:198-211): a bit flip of a negative (or NaN) y
+__device__ __forceinline__ double dual_violation(double y, bool ineq) {
+  return of_bits(ineq && (bits_negative(y) || bits_nan(y)) && !bits_zero(y) ? bits_of(y) ^ kSignBit : 0ULL);
+}
+
+// One evaluation's quantities. Columns: the unscaled statistics of the average (kN_*), then at
+// kEvalNQ the weighted-KKT ingredients (src/saddle_point_gpu.jl:250-278) of the current, average
+// and last-restart points (4 each: bound violation, c'x, dual residual, bound terms) and
+// ||avg - last restart||^2. Rows: kM_*, then 3 per point (violation, dual violation, b'y) and the
+// distance.
 enum EvalNQ {
   kN_LuSq = 0, kN_LuMax, kN_Cx, kN_XMax, kN_XSq, kN_RcvSq, kN_RcvMax, kN_Contrib,
   kN_RayLuMax, kN_RayRcvMax, kN_RayContrib, kN_RayRcMax, kEvalNQ
 };
 constexpr unsigned kEvalNMax = (1u << kN_LuMax) | (1u << kN_XMax) | (1u << kN_RcvMax) | (1u << kN_RayLuMax) |
                                (1u << kN_RayRcvMax) | (1u << kN_RayRcMax);
+enum EvalMQ { kM_CvSq = 0, kM_CvMax, kM_DrSq, kM_DrMax, kM_By, kM_YMax, kM_YSq, kM_RayCvMax, kEvalMQ };
+constexpr unsigned kEvalMMax = (1u << kM_CvMax) | (1u << kM_DrMax) | (1u << kM_YMax) | (1u << kM_RayCvMax);
+constexpr int kKktNQ = 13;
+constexpr int kKktMQ = 10;
+constexpr int kPassNQ = kEvalNQ + kKktNQ;
+constexpr int kPassMQ = kEvalMQ + kKktMQ;
 
+// What an instance's passes need of its StepState, read once per CTA.
 template <class T>
-struct EvalN {
-  const T* ax;
-  const T* agrad;
-  const double* var;   // variable_rescaling (D)
-  const double* rvar;  // 1 / D
-  const double* ol;
-  const double* ou;
-  const double* oc;
-  __device__ __forceinline__ void operator()(long long j, double* a) const { stats(j, ax[j], agrad[j], a); }
-  // the statistics of element j of the scaled point (axv, agv)
-  __device__ __forceinline__ void stats(long long j, T axv, T agv, double* a) const {
-    const double x = div_rcp((double)axv, var[j], rvar[j]);   // :470-471
-    const double g = (double)agv * var[j];         // :472-473
-    const double l = ol[j], u = ou[j], c = oc[j];
-    const bool fl = bits_finite(l), fu = bits_finite(u);
-    const double lv = pos_part(l - x), uv = pos_part(x - u);
-    a[kN_LuSq] += lv * lv + uv * uv;
-    a[kN_LuMax] = nan_max(a[kN_LuMax], nan_max(fabs(lv), fabs(uv)));
-    a[kN_Cx] += c * x;
-    a[kN_XMax] = nan_max(a[kN_XMax], fabs(x));
-    a[kN_XSq] += x * x;
-    const double rc = reduced_cost(g, fl, fu);
-    const double rcv = g - rc;
-    a[kN_RcvSq] += rcv * rcv;
-    a[kN_RcvMax] = nan_max(a[kN_RcvMax], fabs(rcv));
-    a[kN_Contrib] += rc_contribution(rc, l, u);
-    // primal ray, before division by ||x||_inf: bounds 0 where finite (:335-336)
-    const double lr = fl ? pos_part(-x) : 0.0, ur = fu ? pos_part(x) : 0.0;
-    a[kN_RayLuMax] = nan_max(a[kN_RayLuMax], nan_max(lr, ur));
-    // dual ray: objective set to zero, gradient - c (:346-354)
-    const double gr = g - c;
-    const double rcr = reduced_cost(gr, fl, fu);
-    a[kN_RayRcvMax] = nan_max(a[kN_RayRcvMax], fabs(gr - rcr));
-    a[kN_RayContrib] += rc_contribution(rcr, l, u);
-    a[kN_RayRcMax] = nan_max(a[kN_RayRcMax], fabs(rcr));
+struct EvalParams {
+  double wx, wy, rwx, rwy;
+  T commit_weight;
+  bool parity, pending, current, restart;
+  __device__ __forceinline__ EvalParams(const StepState* st, int inst) {
+    const StepState& s = st[inst];
+    wx = s.sum_w_primal;
+    wy = s.sum_w_dual;
+    rwx = s.rcp_w_primal;
+    rwy = s.rcp_w_dual;
+    commit_weight = (T)s.commit_weight;
+    parity = s.parity != 0;
+    pending = s.pending_commit != 0;
+    current = s.eval_current != 0;
+    restart = s.eval_restart != 0;
   }
 };
 
-enum EvalMQ { kM_CvSq = 0, kM_CvMax, kM_DrSq, kM_DrMax, kM_By, kM_YMax, kM_YSq, kM_RayCvMax, kEvalMQ };
-constexpr unsigned kEvalMMax = (1u << kM_CvMax) | (1u << kM_DrMax) | (1u << kM_YMax) | (1u << kM_RayCvMax);
-
+// The row pass of an evaluation (optimize(), src/primal_dual_hybrid_gradient_gpu.jl:633-760): the
+// commit of the last accepted step's Sigma y and Sigma Kx, the average y and Kx
+// (compute_average!, src/saddle_point_gpu.jl:226-240; the current point when there is no average),
+// the unscaled statistics and the KKT ingredients. The instance's weights, buffer parity and
+// what to do come from its StepState. The last restart point's ingredients depend on that
+// point alone, so they are formed only when it moved (eval_restart).
 template <class T>
-struct EvalM {
-  const T* ay;
-  const T* akx;
+struct EvalPassM {
+  using Params = EvalParams<T>;
   const double* con;   // constraint_rescaling (E)
   const double* rcon;  // 1 / E
   const double* ob;
-  int neq;
-  const uint8_t* ineq_flag;  // per-row '>=' flag (packed batches); NULL: rows >= neq
-  __device__ __forceinline__ void operator()(long long i, double* a) const { stats(i, ay[i], akx[i], a); }
-  __device__ __forceinline__ void stats(long long i, T ayv, T akv, double* a) const {
-    const double y = div_rcp((double)ayv, con[i], rcon[i]);   // :474-475
-    const double kx = (double)akv * con[i];        // :476-477
-    const double b = ob[i];
-    const bool ineq = ineq_flag ? ineq_flag[i] != 0 : i >= neq;
-    double cv = b - kx;                            // :26-45
-    if (ineq) cv = pos_part(cv);
-    a[kM_CvSq] += cv * cv;
-    a[kM_CvMax] = nan_max(a[kM_CvMax], fabs(cv));
-    if (ineq) {
-      const double dr = pos_part(-y);             // :198-211
-      a[kM_DrSq] += dr * dr;
-      a[kM_DrMax] = nan_max(a[kM_DrMax], dr);
-    }
-    a[kM_By] += b * y;
-    a[kM_YMax] = nan_max(a[kM_YMax], fabs(y));
-    a[kM_YSq] += y * y;
-    double cvr = -kx;                              // ray: right-hand side 0 (:338)
-    if (ineq) cvr = pos_part(cvr);
-    a[kM_RayCvMax] = nan_max(a[kM_RayCvMax], fabs(cvr));
-  }
-};
-
-// Scaled weighted-KKT ingredients (src/saddle_point_gpu.jl:250-278) of three points:
-// 0 = current, 1 = average, 2 = last restart; plus ||avg - last restart||^2.
-constexpr int kKktNQ = 13;
-constexpr int kKktMQ = 10;
-
-template <class T>
-struct KktN {
-  const T* l;
-  const T* u;
-  const T* c;
-  const T* x0; const T* x1; const T* x2;
-  const T* g0; const T* g1; const T* g2;
-  __device__ __forceinline__ void operator()(long long j, double* a) const {
-    at(j, x0[j], g0[j], x1[j], g1[j], true, a);
-  }
-  // the three points' ingredients from the values of the current (xc, gc) and average
-  // (xa, ga) points; the last restart point's (quantities 8-11) only when with_restart
-  __device__ __forceinline__ void at(long long j, T xc, T gc, T xa, T ga, bool with_restart, double* a) const {
-    const double l = (double)this->l[j], u = (double)this->u[j], c = (double)this->c[j];
-    const bool fl = bits_finite(l), fu = bits_finite(u);
-    value_point(0, xc, gc, l, u, c, fl, fu, a);
-    value_point(1, xa, ga, l, u, c, fl, fu, a);
-    const T xr = x2[j];
-    if (with_restart) value_point(2, xr, g2[j], l, u, c, fl, fu, a);
-    const double d = (double)xa - (double)xr;
-    a[12] += d * d;
-  }
-  __device__ __forceinline__ void value_point(int p, T xv, T gv, double l, double u, double c, bool fl, bool fu,
-                                              double* a) const {
-    const double x = (double)xv, g = (double)gv;
-    const double lv = pos_part(l - x), uv = pos_part(x - u);
-    a[4 * p + 0] += lv * lv + uv * uv;
-    a[4 * p + 1] += c * x;
-    const double rc = reduced_cost(g, fl, fu);
-    const double rcv = g - rc;
-    a[4 * p + 2] += rcv * rcv;
-    a[4 * p + 3] += rc_contribution(rc, l, u);
-  }
-};
-
-template <class T>
-struct KktM {
   const T* b;
-  const T* y0; const T* y1; const T* y2;
-  const T* k0; const T* k1; const T* k2;
-  int neq;
-  const uint8_t* ineq_flag;  // as in EvalM
-  __device__ __forceinline__ void value_point(int p, T yv, T kv, double b, bool ineq, double* a) const {
-    const double y = (double)yv, kx = (double)kv;
-    double cv = b - kx;
-    if (ineq) cv = pos_part(cv);
-    a[3 * p + 0] += cv * cv;
-    if (ineq) {
-      const double dr = pos_part(-y);
-      a[3 * p + 1] += dr * dr;
-    }
-    a[3 * p + 2] += b * y;
-  }
-  __device__ __forceinline__ void operator()(long long i, double* a) const { at(i, y0[i], k0[i], y1[i], k1[i], true, a); }
-  __device__ __forceinline__ void at(long long i, T yc, T kc, T ya, T ka, bool with_restart, double* a) const {
-    const double b = (double)this->b[i];
-    const bool ineq = ineq_flag ? ineq_flag[i] != 0 : i >= neq;
-    value_point(0, yc, kc, b, ineq, a);
-    value_point(1, ya, ka, b, ineq, a);
-    const T yr = y2[i];
-    if (with_restart) value_point(2, yr, k2[i], b, ineq, a);
-    const double d = (double)ya - (double)yr;
-    a[9] += d * d;
-  }
-};
-
-// One evaluation's column pass (optimize(), src/primal_dual_hybrid_gradient_gpu.jl:633-760):
-// the average (compute_average!, src/saddle_point_gpu.jl:226-240, with the average's K'y
-// given as aty = A' y-bar, computed after the row pass formed y-bar; or the current point when
-// there is none, which takes the gradient buffer as it stood), its unscaled statistics
-// (EvalN), buffer_primal_gradient = c - K'y (:742), and the KKT ingredients of the current,
-// average and last-restart points (KktN). The last restart point's ingredients depend on
-// that point alone, so the caller recomputes them (with_restart) only after it changed.
-// Per element the arithmetic is that of the separate kernels, so the sums are the same.
-template <class T>
-struct EvalPassN {
-  EvalN<T> en;   // its ax / agrad are not read: the average comes from sx and aty here
-  KktN<T> kn;    // kn.x0 = x, kn.x2 = rx, kn.g2 = rgrad
-  const T* sx;
-  const T* aty;  // A' y-bar
-  const T* kty;
-  T* ax;         // the average, written
-  T* agrad;
-  T* grad;
-  double wx, wy, rwx, rwy;
-  int use_current;
-  int with_restart;
-  __device__ __forceinline__ void operator()(long long j, double* a) const {
-    const T c = kn.c[j];
-    const T gold = grad[j];
-    const T xc = kn.x0[j];
-    T xa, ga;
-    if (use_current) {
-      xa = xc;
-      ga = gold;
-    } else {
-      xa = (T)div_rcp((double)sx[j], wx, rwx);
-      ga = c - aty[j];
-    }
-    ax[j] = xa;
-    agrad[j] = ga;
-    const T gc = c - kty[j];
-    grad[j] = gc;
-    en.stats(j, xa, ga, a);
-    kn.at(j, xc, gc, xa, ga, with_restart != 0, a + kEvalNQ);
-  }
-};
-
-// The row pass of the same evaluation: average (or current) y and K x, EvalM, KktM.
-template <class T>
-struct EvalPassM {
-  EvalM<T> em;   // its ay / akx are not read
-  KktM<T> km;    // km.y0 / km.k0 = current y / K x, km.y2 / km.k2 = restart point
-  const T* sy;
-  const T* skx;
+  const T* y0; const T* y1; const T* kx0; const T* kx1;
+  const T* ry; const T* rkx;
+  T* sy;
+  T* skx;
   T* ay;         // the average, written
   T* akx;
-  double wx, wy, rwx, rwy;
-  int use_current;
-  int with_restart;
-  __device__ __forceinline__ void operator()(long long i, double* a) const {
-    const T yc = km.y0[i], kc = km.k0[i];
-    T ya, ka;
-    if (use_current) {
-      ya = yc;
-      ka = kc;
-    } else {
-      ya = (T)div_rcp((double)sy[i], wy, rwy);
-      ka = (T)div_rcp((double)skx[i], wx, rwx);
+  int neq;
+  const uint8_t* ineq_flag;  // per-row '>=' flag (packed batches); NULL: rows >= neq
+  __device__ __forceinline__ void point(T yv, T kv, double b, bool ineq, double* a) const {
+    const double y = widen(yv);
+    add_square(row_violation(b - widen(kv), ineq), a[0]);
+    add_square(dual_violation(y, ineq), a[1]);
+    a[2] = fma(b, y, a[2]);
+  }
+  __device__ __forceinline__ void operator()(const Params& s, int i, double* a) const {
+    const T yc = (s.parity ? y1 : y0)[i], kc = (s.parity ? kx1 : kx0)[i];
+    const bool ineq = ineq_flag ? ineq_flag[i] != 0 : i >= neq;
+    T ya = yc, ka = kc;
+    if (!s.current) {
+      T vy = sy[i], vk = skx[i];
+      if (s.pending) {
+        vy = fma(yc, s.commit_weight, vy);
+        vk = fma(kc, s.commit_weight, vk);
+        sy[i] = vy;
+        skx[i] = vk;
+      }
+      ya = (T)div_rcp(widen(vy), s.wy, s.rwy);
+      ka = (T)div_rcp(widen(vk), s.wx, s.rwx);
     }
     ay[i] = ya;
     akx[i] = ka;
-    em.stats(i, ya, ka, a);
-    km.at(i, yc, kc, ya, ka, with_restart != 0, a + kEvalMQ);
+    {
+      const double y = div_rcp(widen(ya), con[i], rcon[i]);   // :474-475
+      const double kx = widen(ka) * con[i];                   // :476-477
+      const double b = ob[i];
+      const double cv = row_violation(b - kx, ineq);
+      add_square(cv, a[kM_CvSq]);
+      a[kM_CvMax] = nan_max(a[kM_CvMax], cv);
+      const double dr = dual_violation(y, ineq);
+      add_square(dr, a[kM_DrSq]);
+      a[kM_DrMax] = nan_max(a[kM_DrMax], dr);
+      a[kM_By] = fma(b, y, a[kM_By]);
+      a[kM_YMax] = nan_max(a[kM_YMax], y);
+      a[kM_YSq] = fma(y, y, a[kM_YSq]);
+      // ray: right-hand side 0 (:338)
+      a[kM_RayCvMax] = nan_max(a[kM_RayCvMax], row_violation(negate_bits(kx), ineq));
+    }
+    double* k = a + kEvalMQ;
+    const double b = widen(this->b[i]);
+    point(yc, kc, b, ineq, k);
+    point(ya, ka, b, ineq, k + 3);
+    const T yr = ry[i];
+    if (s.restart) point(yr, rkx[i], b, ineq, k + 6);
+    const double d = widen(ya) - widen(yr);
+    k[9] = fma(d, d, k[9]);
+  }
+};
+
+// The column pass: the average x, its gradient c - A' y-bar (aty, formed after the row pass;
+// the current point takes the gradient buffer as it stood), buffer_primal_gradient = c - K'y
+// (:742), the statistics and the KKT ingredients.
+template <class T>
+struct EvalPassN {
+  using Params = EvalParams<T>;
+  const double* var;   // variable_rescaling (D)
+  const double* rvar;  // 1 / D
+  const double* ol; const double* ou; const double* oc;
+  const T* l; const T* u; const T* c;
+  const T* x; const T* sx; const T* aty; const T* kty;
+  const T* rx; const T* rgrad;
+  T* ax;         // the average, written
+  T* agrad;
+  T* grad;
+  __device__ __forceinline__ void point(T xv, T gv, double l, double u, double c, bool fl, bool fu, double* a) const {
+    const double x = widen(xv), g = widen(gv);
+    double unused = 0.0;
+    add_violation(x, l, u, a[0], unused);
+    a[1] = fma(c, x, a[1]);
+    const bool kept = keeps_cost(g, fl, fu);
+    add_square(cost_residual(g, kept), a[2]);
+    add_bound_term(g, kept, l, u, a[3]);
+  }
+  __device__ __forceinline__ void operator()(const Params& s, int j, double* a) const {
+    const T cs = c[j], xc = x[j];
+    T xa = xc, ga;
+    if (s.current) {
+      ga = grad[j];
+    } else {
+      xa = (T)div_rcp(widen(sx[j]), s.wx, s.rwx);
+      ga = cs - aty[j];
+    }
+    ax[j] = xa;
+    agrad[j] = ga;
+    const T gc = cs - kty[j];
+    grad[j] = gc;
+    {
+      const double x = div_rcp(widen(xa), var[j], rvar[j]);   // :470-471
+      const double g = widen(ga) * var[j];                    // :472-473
+      const double l = ol[j], u = ou[j], c = oc[j];
+      const bool fl = bits_finite(l), fu = bits_finite(u);
+      add_violation(x, l, u, a[kN_LuSq], a[kN_LuMax]);
+      a[kN_Cx] = fma(c, x, a[kN_Cx]);
+      a[kN_XMax] = nan_max(a[kN_XMax], x);
+      a[kN_XSq] = fma(x, x, a[kN_XSq]);
+      const bool kept = keeps_cost(g, fl, fu);
+      const double rcv = cost_residual(g, kept);
+      add_square(rcv, a[kN_RcvSq]);
+      a[kN_RcvMax] = nan_max(a[kN_RcvMax], rcv);
+      add_bound_term(g, kept, l, u, a[kN_Contrib]);
+      // primal ray, before division by ||x||_inf: bounds 0 where finite (:335-336)
+      const bool xnan = bits_nan(x);
+      if (xnan ? fl || fu : (bits_negative(x) ? fl : fu)) a[kN_RayLuMax] = nan_max(a[kN_RayLuMax], x);
+      // dual ray: objective set to zero, gradient - c (:346-354)
+      const double gr = g - c;
+      const bool keptr = keeps_cost(gr, fl, fu);
+      a[kN_RayRcvMax] = nan_max(a[kN_RayRcvMax], cost_residual(gr, keptr));
+      add_bound_term(gr, keptr, l, u, a[kN_RayContrib]);
+      if (keptr) a[kN_RayRcMax] = nan_max(a[kN_RayRcMax], gr);
+    }
+    double* k = a + kEvalNQ;
+    const double l = widen(this->l[j]), u = widen(this->u[j]), c = widen(cs);
+    const bool fl = bits_finite(l), fu = bits_finite(u);
+    point(xc, gc, l, u, c, fl, fu, k);
+    point(xa, ga, l, u, c, fl, fu, k + 4);
+    const T xr = rx[j];
+    if (s.restart) point(xr, rgrad[j], l, u, c, fl, fu, k + 8);
+    const double d = widen(xa) - widen(xr);
+    k[12] = fma(d, d, k[12]);
   }
 };
 

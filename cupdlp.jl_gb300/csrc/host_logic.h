@@ -36,6 +36,24 @@ struct RestartMemory {
   double pdist = 0.0, ddist = 0.0, ratio_last = 1.0;
 };
 
+// KKT ingredients of the last restart point (quantities 8-11 of a column pass, 6-8 of a row
+// pass), kept until the restart point moves.
+struct RestartKkt {
+  bool valid = false;
+  double n[4] = {}, m[3] = {};
+  // fills the kept values into an evaluation's kn / km, or keeps the ones just computed there
+  void keep_or_fill(double* kn, double* km) {
+    if (valid) {
+      std::memcpy(kn + 8, n, sizeof(n));
+      std::memcpy(km + 6, m, sizeof(m));
+    } else {
+      std::memcpy(n, kn + 8, sizeof(n));
+      std::memcpy(m, km + 6, sizeof(m));
+      valid = true;
+    }
+  }
+};
+
 inline double jmax_h(double a, double b) {
   if (a != a || b != b) return a + b;
   return a > b ? a : b;
@@ -132,7 +150,7 @@ struct RestartDecision {
   double new_omega = 0.0;
 };
 
-// kn / km: the KktN / KktM reductions (points 0 = current, 1 = average, 2 = last restart;
+// kn / km: an evaluation's KKT ingredients (points 0 = current, 1 = average, 2 = last restart;
 // kn[12] = ||avg x - last x||^2, km[9] = ||avg y - last y||^2). `count_primal` is
 // sum_primal_solutions_count, `tau`/`omega` the current step size and primal weight.
 inline RestartDecision decide_restart(const gpdhg_params& prm, const InstanceInfo& qi, long long count_primal,

@@ -20,6 +20,7 @@
 // module and its symbol are reloaded then). Every call reuses the same array: each call
 // overwrites all partials it reads, so nothing needs clearing, and calls that overlap on the
 // GPU (two streams, or two host threads) race on it.
+#include <algorithm>
 #include <cmath>
 #include <cstring>
 #include <mutex>
@@ -30,9 +31,13 @@
 namespace gpdhg {
 namespace {
 
-constexpr int kNoallocItem = 4096;                                     // elements per CTA
 constexpr long long kNoallocMaxLength = 1LL << 24;                     // n and m at most
-constexpr int kNoallocMaxItems = (int)(kNoallocMaxLength / kNoallocItem);
+constexpr int kNoallocMaxItems = 4096;                                 // CTAs per side at most
+// Elements per CTA: as few as one per thread, and one wave of 4 CTAs on each of 152 SMs for both
+// sides together on long vectors.
+int noalloc_item(long long n, long long m) {
+  return kBlock * (int)std::max<long long>(1, (n + m + kBlock * 600LL - 1) / (kBlock * 600LL));
+}
 constexpr int kQn = 10, kQm = 9;
 constexpr int kScratchDoubles = (kQn + kQm) * kNoallocMaxItems + 32;
 
@@ -46,82 +51,96 @@ constexpr unsigned kBMax = (1u << kB_CvMax) | (1u << kB_DrMax) | (1u << kB_YMax)
 // Column side: bound violations, objective, reduced costs of g = c - A'y (the statistics of
 // compute_primal_residual!, primal_obj and compute_dual_stats!, src/iteration_stats_utils_gpu.jl:71-238).
 struct ColumnStats {
+  static constexpr int kQ = kQn;
+  static constexpr unsigned kMax = kAMax;
   const double *l, *u, *c, *x, *aty;
   __device__ __forceinline__ void operator()(long long j, double* a) const {
-    const double xv = x[j], lv_ = l[j], uv_ = u[j], cv = c[j];
-    const bool fl = isfinite(lv_), fu = isfinite(uv_);
-    const double lv = jmax(lv_ - xv, 0.0), uv = jmax(xv - uv_, 0.0);
-    a[kA_LuSq] += lv * lv + uv * uv;
-    a[kA_LuMax] = nan_max(a[kA_LuMax], nan_max(lv, uv));
-    a[kA_Cx] += cv * xv;
-    a[kA_XMax] = nan_max(a[kA_XMax], fabs(xv));
-    a[kA_XSq] += xv * xv;
+    const double xv = x[j], lv = l[j], uv = u[j], cv = c[j];
+    const bool fl = bits_finite(lv), fu = bits_finite(uv);
+    add_violation(xv, lv, uv, a[kA_LuSq], a[kA_LuMax]);
+    a[kA_Cx] = fma(cv, xv, a[kA_Cx]);
+    a[kA_XMax] = nan_max(a[kA_XMax], xv);
+    a[kA_XSq] = fma(xv, xv, a[kA_XSq]);
     const double g = cv - aty[j];
-    const double rc = reduced_cost(g, fl, fu);
-    const double rcv = g - rc;
-    a[kA_RcvSq] += rcv * rcv;
-    a[kA_RcvMax] = nan_max(a[kA_RcvMax], fabs(rcv));
-    a[kA_Contrib] += rc_contribution(rc, lv_, uv_);
-    a[kA_CSq] += cv * cv;
-    a[kA_CMax] = nan_max(a[kA_CMax], fabs(cv));
+    const bool kept = keeps_cost(g, fl, fu);
+    const double rcv = cost_residual(g, kept);
+    add_square(rcv, a[kA_RcvSq]);
+    a[kA_RcvMax] = nan_max(a[kA_RcvMax], rcv);
+    add_bound_term(g, kept, lv, uv, a[kA_Contrib]);
+    a[kA_CSq] = fma(cv, cv, a[kA_CSq]);
+    a[kA_CMax] = nan_max(a[kA_CMax], cv);
   }
 };
 
 // Row side: constraint violations of A x, dual sign violations, b'y.
 struct RowStats {
+  static constexpr int kQ = kQm;
+  static constexpr unsigned kMax = kBMax;
   const double *b, *y, *ax;
   int neq;
   __device__ __forceinline__ void operator()(long long i, double* a) const {
     const double bv = b[i], yv = y[i];
     const bool ineq = i >= neq;
-    double cv = bv - ax[i];
-    if (ineq) cv = jmax(cv, 0.0);
-    a[kB_CvSq] += cv * cv;
-    a[kB_CvMax] = nan_max(a[kB_CvMax], fabs(cv));
-    if (ineq) {
-      const double dr = jmax(-yv, 0.0);
-      a[kB_DrSq] += dr * dr;
-      a[kB_DrMax] = nan_max(a[kB_DrMax], dr);
-    }
-    a[kB_By] += bv * yv;
-    a[kB_YMax] = nan_max(a[kB_YMax], fabs(yv));
-    a[kB_YSq] += yv * yv;
-    a[kB_BSq] += bv * bv;
-    a[kB_BMax] = nan_max(a[kB_BMax], fabs(bv));
+    const double cv = row_violation(bv - ax[i], ineq);
+    add_square(cv, a[kB_CvSq]);
+    a[kB_CvMax] = nan_max(a[kB_CvMax], cv);
+    const double dr = dual_violation(yv, ineq);
+    add_square(dr, a[kB_DrSq]);
+    a[kB_DrMax] = nan_max(a[kB_DrMax], dr);
+    a[kB_By] = fma(bv, yv, a[kB_By]);
+    a[kB_YMax] = nan_max(a[kB_YMax], yv);
+    a[kB_YSq] = fma(yv, yv, a[kB_YSq]);
+    a[kB_BSq] = fma(bv, bv, a[kB_BSq]);
+    a[kB_BMax] = nan_max(a[kB_BMax], bv);
   }
 };
 
-// The segmented reduction of the solver with its item list implied by the block index
-// (item k = [k * 4096, (k + 1) * 4096)) and its partials in the caller-free scratch.
-template <int Q, unsigned MAXMASK, class F>
-__global__ void __launch_bounds__(kBlock) noalloc_reduce_kernel(long long len, F f, double* partials, int nitems) {
-  __shared__ double sh[32];
-  double acc[Q];
+// One side's elements, its CTAs and their partials in the scratch.
+template <class F>
+struct NoallocSide {
+  F f;
+  long long len;
+  int item;         // elements per CTA
+  int items;
+  double* partials; // quantity q of CTA k at partials[q * items + k]
+};
+
+template <class F>
+__device__ __forceinline__ void noalloc_item_sums(const NoallocSide<F>& s, int item, double* sh, double* res) {
+  double acc[F::kQ];
 #pragma unroll
-  for (int q = 0; q < Q; ++q) acc[q] = 0.0;
-  const long long b = (long long)blockIdx.x * kNoallocItem;
-  const long long e = b + kNoallocItem < len ? b + kNoallocItem : len;
-  for (long long i = b + threadIdx.x; i < e; i += kBlock) f(i, acc);
-#pragma unroll
-  for (int q = 0; q < Q; ++q) {
-    const double r = ((MAXMASK >> q) & 1u) ? block_nan_max(acc[q], sh) : block_sum(acc[q], sh);
-    if (threadIdx.x == 0) partials[(size_t)q * nitems + blockIdx.x] = r;
-  }
+  for (int q = 0; q < F::kQ; ++q) acc[q] = 0.0;
+  const long long b = (long long)item * s.item;
+  const long long e = b + s.item < s.len ? b + s.item : s.len;
+  for (long long i = b + threadIdx.x; i < e; i += kBlock) s.f(i, acc);
+  const double r = block_reduce_q<F::kQ, F::kMax>(acc, sh, res);
+  if ((int)threadIdx.x < F::kQ) s.partials[(size_t)threadIdx.x * s.items + item] = r;
 }
 
-template <int Q, unsigned MAXMASK>
-__global__ void __launch_bounds__(kBlock) noalloc_finalize_kernel(const double* partials, int nitems, double* out) {
+// Both sides in one launch: the columns' CTAs, then the rows'. Bound by the FP64 pipe (88% busy;
+// 104 MB at HBM rate would take 15 us): n = 2M, m = 1M took 163 + 47 us in two launches with a
+// shuffle tree per quantity and plainly written arithmetic, and takes 50 us.
+__global__ void __launch_bounds__(kBlock, 4) noalloc_reduce_kernel(NoallocSide<ColumnStats> n, NoallocSide<RowStats> m) {
+  __shared__ double sh[kQn * kBlock];
+  __shared__ double res[kQn];
+  if ((int)blockIdx.x < n.items) noalloc_item_sums(n, blockIdx.x, sh, res);
+  else noalloc_item_sums(m, (int)blockIdx.x - n.items, sh, res);
+}
+
+// 19 + 15 us as two CTAs over all quantities in turn, 5 us as one CTA per quantity.
+// One CTA per quantity (columns' then rows'), its items in order; rows' results from out + 16.
+__global__ void __launch_bounds__(kBlock) noalloc_finalize_kernel(const double* part_n, int items_n,
+                                                                  const double* part_m, int items_m, double* out) {
   __shared__ double sh[32];
-  for (int q = 0; q < Q; ++q) {
-    const bool is_max = (MAXMASK >> q) & 1u;
-    double a = 0.0;
-    for (int k = threadIdx.x; k < nitems; k += kBlock) {
-      const double v = partials[(size_t)q * nitems + k];
-      a = is_max ? nan_max(a, v) : a + v;
-    }
-    a = is_max ? block_nan_max(a, sh) : block_sum(a, sh);
-    if (threadIdx.x == 0) out[q] = a;
-  }
+  const bool rows = (int)blockIdx.x >= kQn;
+  const int q = rows ? (int)blockIdx.x - kQn : (int)blockIdx.x;
+  const bool is_max = ((rows ? kBMax : kAMax) >> q) & 1u;
+  const int items = rows ? items_m : items_n;
+  const double* p = (rows ? part_m : part_n) + (size_t)q * items;
+  double a = 0.0;
+  for (int k = threadIdx.x; k < items; k += kBlock) a = is_max ? nan_max(a, p[k]) : a + p[k];
+  a = is_max ? block_nan_max(a, sh) : block_sum(a, sh);
+  if (threadIdx.x == 0) out[(rows ? 16 : 0) + q] = a;
 }
 
 using CtxGetIdFn = int (*)(void* ctx, unsigned long long* id);   // cuCtxGetId
@@ -200,17 +219,13 @@ void convergence_noalloc(int32_t n, int32_t m, int32_t neq, double obj_const, co
   double* part_n = base;
   double* part_m = base + (size_t)kQn * kNoallocMaxItems;
   double* outs = base + (size_t)(kQn + kQm) * kNoallocMaxItems;
-  const int in = (int)((n + kNoallocItem - 1) / kNoallocItem);
-  const int im = (int)((m + kNoallocItem - 1) / kNoallocItem);
-  noalloc_reduce_kernel<kQn, kAMax><<<in, kBlock, 0, s>>>(n, ColumnStats{l, u, c, x, aty}, part_n, in);
+  const int item = noalloc_item(n, m);
+  const int in = (n + item - 1) / item, im = (m + item - 1) / item;
+  noalloc_reduce_kernel<<<in + im, kBlock, 0, s>>>(
+      NoallocSide<ColumnStats>{ColumnStats{l, u, c, x, aty}, n, item, in, part_n},
+      NoallocSide<RowStats>{RowStats{b, y, ax, neq}, m, item, im, part_m});
   CK_LAUNCH();
-  if (im > 0) {
-    noalloc_reduce_kernel<kQm, kBMax><<<im, kBlock, 0, s>>>(m, RowStats{b, y, ax, neq}, part_m, im);
-    CK_LAUNCH();
-  }
-  noalloc_finalize_kernel<kQn, kAMax><<<1, kBlock, 0, s>>>(part_n, in, outs);
-  CK_LAUNCH();
-  noalloc_finalize_kernel<kQm, kBMax><<<1, kBlock, 0, s>>>(part_m, im, outs + 16);
+  noalloc_finalize_kernel<<<kQn + kQm, kBlock, 0, s>>>(part_n, in, part_m, im, outs);
   CK_LAUNCH();
   double h[32];
   CK(cudaMemcpyAsync(h, outs, sizeof(h), cudaMemcpyDeviceToHost, s));

@@ -58,7 +58,12 @@ template <class T>
 struct DotF {
   const T* a;
   const T* b;
-  __device__ __forceinline__ void operator()(long long i, double* acc) const { acc[0] += (double)a[i] * (double)b[i]; }
+  struct Params {
+    __device__ Params(const StepState*, int) {}
+  };
+  __device__ __forceinline__ void operator()(const Params&, int i, double* acc) const {
+    acc[0] += (double)a[i] * (double)b[i];
+  }
 };
 
 // Step graphs hold 1, 2, 4, ..., 64 [primal, dual] pairs; a chunk launches the smallest one
@@ -114,17 +119,13 @@ struct Workspace {
   DBuf<T> y0, y1, kx0, kx1, sy, skx, ay, akx, ry, rkx, tmp_m;
   DBuf<StepState> st_dev;
   PinnedBuf<StepState> st_host;
-  DBuf<double> part_p, part_d, red_part, red_out;
+  DBuf<double> part_p, part_d, red_part_n, red_part_m, red_out;
   DBuf<double> rvar, rcon;   // 1 / variable and 1 / constraint rescaling (evaluation divisions)
   PinnedBuf<double> red_host;
-  // KKT ingredients of the last restart point (KktN quantities 8-11, KktM 6-8), valid until
-  // the restart point moves
-  bool restart_kkt_valid = false;
-  double restart_kkt_n[4] = {}, restart_kkt_m[3] = {};
+  RestartKkt restart_kkt;
   // segmented reductions over [0, n) and [0, m): the same layout a batch uses per instance
   DBuf<SegItem> seg_n, seg_m;
   DBuf<int32_t> seg_n_begin, seg_m_begin;
-  DBuf<uint8_t> one;
   int nseg_n = 1, nseg_m = 1;
   cudaGraphExec_t graphs[kGraphLevels] = {};
   // profiled variants: an event between every pair of kernels
@@ -137,7 +138,7 @@ struct Workspace {
   TilePlan<T> plan_p, plan_d;
   DBuf<double> part_p_split, part_d_split;
 
-  explicit Workspace(gpdhg_problem* p) : P(p), n(p->n), m(p->m), st_host(1), red_host(64) {
+  explicit Workspace(gpdhg_problem* p) : P(p), n(p->n), m(p->m), st_host(1), red_host(kEvalStride) {
     PhaseTrace tr;
     const size_t N = std::max(n, 1), M = std::max(m, 1);
     cudaStream_t s = P->stream;
@@ -192,7 +193,7 @@ struct Workspace {
     part_d.alloc(2 * (size_t)plan_d.num_ctas);
     part_p_split.alloc(std::max(plan_p.num_splits, 1));
     part_d_split.alloc(2 * (size_t)std::max(plan_d.num_splits, 1));
-    red_out.alloc(64);
+    red_out.alloc(kEvalStride);
     {
       std::vector<SegItem> it;
       std::vector<int32_t> beg;
@@ -207,9 +208,8 @@ struct Workspace {
       };
       upload(seg_n, seg_n_begin, n, nseg_n);
       upload(seg_m, seg_m_begin, m, nseg_m);
-      red_part.alloc((size_t)32 * std::max(nseg_n, nseg_m));
-      one.alloc(1);
-      CK(cudaMemsetAsync(one.get(), 1, 1, s));
+      red_part_n.alloc((size_t)kPassNQ * nseg_n);
+      red_part_m.alloc((size_t)kPassMQ * nseg_m);
     }
     CK(cudaEventCreate(&ev0));
     CK(cudaEventCreate(&ev1));
@@ -305,28 +305,33 @@ struct Workspace {
     ++P->launches;
   }
 
-  // FP64 reduction of Q quantities over [0, n) (n_side) or [0, m), into red_out[out_offset..)
+  // one side's pass over its segments into its partials
   template <int Q, unsigned MAXMASK, class F>
-  void reduce(bool n_side, F f, int out_offset) {
+  void reduce(bool n_side, F f, const StepState* st) {
     const int nit = n_side ? nseg_n : nseg_m;
-    seg_reduce_kernel<Q, MAXMASK, F><<<nit, kBlock, 0, P->stream>>>(n_side ? seg_n.get() : seg_m.get(), one.get(), f,
-                                                                     red_part.get(), nit);
+    seg_reduce_kernel<Q, MAXMASK, F><<<nit, kBlock, 0, P->stream>>>(n_side ? seg_n.get() : seg_m.get(), st, f,
+                                                                     n_side ? red_part_n.get() : red_part_m.get(), nit);
     CK_LAUNCH();
-    seg_finalize_kernel<Q, MAXMASK><<<1, kBlock, 0, P->stream>>>(n_side ? seg_n_begin.get() : seg_m_begin.get(),
-                                                                  one.get(), red_part.get(), nit,
-                                                                  red_out.get() + out_offset, 32);
-    CK_LAUNCH();
-    P->launches += 2;
+    ++P->launches;
   }
-  void fetch_reductions(int count) {
-    CK(cudaMemcpyAsync(red_host.p, red_out.get(), sizeof(double) * count, cudaMemcpyDeviceToHost, P->stream));
+  SegSide side(bool n_side, int quantities, unsigned maxmask) {
+    return SegSide{n_side ? seg_n_begin.get() : seg_m_begin.get(), n_side ? red_part_n.get() : red_part_m.get(),
+                   red_out.get() + (n_side ? kEvalOutN : 0), n_side ? nseg_n : nseg_m, quantities, maxmask};
+  }
+  // the partials of both sides reduced (a side without quantities is skipped) and read back
+  void finish_reductions(SegSide a, SegSide b, const StepState* st) {
+    seg_finalize_kernel<<<dim3(a.quantities + b.quantities, 1), kBlock, 0, P->stream>>>(a, b, st);
+    CK_LAUNCH();
+    ++P->launches;
+    CK(cudaMemcpyAsync(red_host.p, red_out.get(), sizeof(double) * kEvalStride, cudaMemcpyDeviceToHost, P->stream));
     CK(cudaStreamSynchronize(P->stream));
   }
 
   double dot(const T* a, const T* b2, long long len) {
-    reduce<1, 0u>(len == n, DotF<T>{a, b2}, 0);
-    fetch_reductions(1);
-    return red_host.p[0];
+    const bool n_side = len == n;
+    reduce<1, 0u>(n_side, DotF<T>{a, b2}, nullptr);
+    finish_reductions(side(n_side, 1, 0u), SegSide{}, nullptr);
+    return red_host.p[n_side ? kEvalOutN : 0];
   }
 
   int grid_for(long long len) const { return std::max(1, std::min(ceil_div(len, kBlock), 4096)); }
@@ -398,57 +403,46 @@ bool run_phase(gpdhg_problem* P, Workspace<T>& W, const gpdhg_params& prm, LoopS
     if (eval_due(it, freq, it_limit, st.numerical_error != 0)) {
       st.kkt_passes += 2.0;  // KKT_PASSES_PER_TERMINATION_EVALUATION
       st.done = 0;
-      push_state();
+      // The average, or the current point (src/primal_dual_hybrid_gradient_gpu.jl:635-642)
+      st.eval_active = 1;
+      st.eval_current = (st.numerical_error || st.count_primal == 0 || st.count_dual == 0) ? 1 : 0;
+      st.eval_restart = W.restart_kkt.valid ? 0 : 1;
+      st.rcp_w_primal = st.eval_current ? 0.0 : 1.0 / st.sum_w_primal;
+      st.rcp_w_dual = st.eval_current ? 0.0 : 1.0 / st.sum_w_dual;
+      push_state_async();
+      // the accepted step still to be applied: its K'y, x and Sigma x here, Sigma y and Sigma Kx
+      // in the row pass
       if (st.pending_commit) {
-        W.launch_pair(kStepCommitOnly, s);
+        W.launch_primal(kStepCommitOnly, s);
         CK_LAUNCH();
-        st.pending_commit = 0;
+        ++P->launches;
       }
       const int p = st.parity;
-      // One pass per side (EvalPassM, then EvalPassN): the average, or the current point
-      // (src/primal_dual_hybrid_gradient_gpu.jl:635-642); its unscaled statistics
-      // (src/iteration_stats_utils_gpu.jl:447-502); buffer_primal_gradient = c - K'y (:742);
-      // and the restart scheme's KKT ingredients, those of the last restart point only when
-      // it moved since they were computed. Between them the average's K'y = A' y-bar (the
-      // reference sums the steps' K'y with the averaging weights instead,
-      // src/saddle_point_gpu.jl:176-189; the two agree in exact arithmetic). One read-back
-      // for all of them.
-      const bool use_current = st.numerical_error || st.count_primal == 0 || st.count_dual == 0;
-      const double wx = st.sum_w_primal, wy = st.sum_w_dual;
-      const double rwx = use_current ? 0.0 : 1.0 / wx, rwy = use_current ? 0.0 : 1.0 / wy;
-      const bool with_restart = !W.restart_kkt_valid;
-      W.template reduce<kEvalMQ + kKktMQ, kEvalMMax>(
+      // One pass per side: the row pass forms the averages y-bar and Kx-bar with their unscaled
+      // statistics (src/iteration_stats_utils_gpu.jl:447-502) and restart-scheme ingredients;
+      // then the average's K'y = A' y-bar (the reference sums the steps' K'y with the averaging
+      // weights instead, src/saddle_point_gpu.jl:176-189; the two agree in exact arithmetic)
+      // and the column pass. One read-back for all of them.
+      W.template reduce<kPassMQ, kEvalMMax>(
           false,
-          EvalPassM<T>{EvalM<T>{W.ay.get(), W.akx.get(), P->con.get(), W.rcon.get(), P->ob.get(), P->neq, nullptr},
-                       KktM<T>{W.b, W.ycur(p), W.ay.get(), W.ry.get(), W.kxcur(p), W.akx.get(), W.rkx.get(), P->neq,
-                               nullptr},
-                       W.sy.get(), W.skx.get(), W.ay.get(), W.akx.get(), wx, wy, rwx, rwy, use_current ? 1 : 0,
-                       with_restart ? 1 : 0},
-          32);
-      if (!use_current) W.spmv(P->At, W.ay.get(), W.tmp_n.get());
-      W.template reduce<kEvalNQ + kKktNQ, kEvalNMax>(
+          EvalPassM<T>{P->con.get(), W.rcon.get(), P->ob.get(), W.b, W.y0.get(), W.y1.get(), W.kx0.get(), W.kx1.get(),
+                       W.ry.get(), W.rkx.get(), W.sy.get(), W.skx.get(), W.ay.get(), W.akx.get(), P->neq, nullptr},
+          W.st_dev.get());
+      if (!st.eval_current) W.spmv(P->At, W.ay.get(), W.tmp_n.get());
+      W.template reduce<kPassNQ, kEvalNMax>(
           true,
-          EvalPassN<T>{EvalN<T>{W.ax.get(), W.agrad.get(), P->var.get(), W.rvar.get(), P->ol.get(), P->ou.get(),
-                                P->oc.get()},
-                       KktN<T>{W.l, W.u, W.c, W.x.get(), W.ax.get(), W.rx.get(), W.grad.get(), W.agrad.get(),
-                               W.rgrad.get()},
-                       W.sx.get(), W.tmp_n.get(), W.kty.get(), W.ax.get(), W.agrad.get(), W.grad.get(), wx, wy, rwx,
-                       rwy, use_current ? 1 : 0, with_restart ? 1 : 0},
-          0);
-      W.fetch_reductions(32 + kEvalMQ + kKktMQ);
-      const double* en = W.red_host.p;            // EvalN, then KktN at kEvalNQ
-      const double* em = W.red_host.p + 32;       // EvalM, then KktM at kEvalMQ
+          EvalPassN<T>{P->var.get(), W.rvar.get(), P->ol.get(), P->ou.get(), P->oc.get(), W.l, W.u, W.c, W.x.get(),
+                       W.sx.get(), W.tmp_n.get(), W.kty.get(), W.rx.get(), W.rgrad.get(), W.ax.get(), W.agrad.get(),
+                       W.grad.get()},
+          W.st_dev.get());
+      W.finish_reductions(W.side(false, kPassMQ, kEvalMMax), W.side(true, kPassNQ, kEvalNMax), W.st_dev.get());
+      st.pending_commit = 0;
+      const double* em = W.red_host.p;               // kM_*, then the rows' KKT ingredients
+      const double* en = W.red_host.p + kEvalOutN;   // kN_*, then the columns'
       double kn[kKktNQ], km[kKktMQ];
       std::memcpy(kn, en + kEvalNQ, sizeof(kn));
       std::memcpy(km, em + kEvalMQ, sizeof(km));
-      if (with_restart) {
-        std::memcpy(W.restart_kkt_n, kn + 8, sizeof(W.restart_kkt_n));
-        std::memcpy(W.restart_kkt_m, km + 6, sizeof(W.restart_kkt_m));
-        W.restart_kkt_valid = true;
-      } else {
-        std::memcpy(kn + 8, W.restart_kkt_n, sizeof(W.restart_kkt_n));
-        std::memcpy(km + 6, W.restart_kkt_m, sizeof(W.restart_kkt_m));
-      }
+      W.restart_kkt.keep_or_fill(kn, km);
       gpdhg_iteration_stats stats;
       std::memset(&stats, 0, sizeof(stats));
       assemble_stats(qi, prm, en, em, stats);
@@ -539,7 +533,7 @@ bool run_phase(gpdhg_problem* P, Workspace<T>& W, const gpdhg_params& prm, LoopS
               CK(cudaMemcpyAsync(W.kxcur_mut(p), W.akx.get(), sizeof(T) * m, cudaMemcpyDeviceToDevice, s));
             }
           }
-          W.restart_kkt_valid = false;  // the restart point moves below
+          W.restart_kkt.valid = false;  // the restart point moves below
           // reset_solution_weighted_average!
           CK(cudaMemsetAsync(W.sx.get(), 0, sizeof(T) * n, s));
           if (m) {
@@ -691,7 +685,7 @@ void init_state(gpdhg_problem* P, Workspace<T>& W, const gpdhg_params& prm, Loop
   }
   st.iter_start_tau = st.tau;
   // create_last_restart_info
-  W.restart_kkt_valid = false;
+  W.restart_kkt.valid = false;
   CK(cudaMemcpyAsync(W.rx.get(), W.x.get(), sizeof(T) * n, cudaMemcpyDeviceToDevice, s));
   CK(cudaMemcpyAsync(W.rgrad.get(), W.grad.get(), sizeof(T) * n, cudaMemcpyDeviceToDevice, s));
   if (m) {
@@ -734,7 +728,7 @@ void handoff_to_fp64(gpdhg_problem* P, Workspace<float>& F, Workspace<double>& D
   grad_kernel<double><<<D.grid_for(n), kBlock, 0, s>>>(n, D.c, D.kty.get(), D.grad.get());
   CK_LAUNCH();
   ++P->launches;
-  D.restart_kkt_valid = false;
+  D.restart_kkt.valid = false;
   CK(cudaMemcpyAsync(D.rx.get(), D.x.get(), sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
   CK(cudaMemcpyAsync(D.rgrad.get(), D.grad.get(), sizeof(double) * n, cudaMemcpyDeviceToDevice, s));
   if (m) {
