@@ -45,8 +45,7 @@ void build_seg_items(const std::vector<int32_t>& off, std::vector<SegItem>& item
   begin.assign(count + 1, 0);
   for (int k = 0; k < count; ++k) {
     begin[k] = (int32_t)items.size();
-    const int32_t step = seg_len(off[k + 1] - off[k]);
-    for (int32_t s = off[k]; s < off[k + 1]; s += step) items.push_back({s, std::min(off[k + 1], s + step), k});
+    for (int32_t s = off[k]; s < off[k + 1]; s += kSegLen) items.push_back({s, std::min(off[k + 1], s + kSegLen), k});
   }
   begin[count] = (int32_t)items.size();
   if (items.empty()) items.push_back({0, 0, 0});
@@ -444,24 +443,18 @@ struct BatchWorkspace {
     return PrimalArgs<T>{B->At.view<T>(), view_p(), c, l, u, x.get(), dx.get(), kty.get(), sx.get(),
                          y0.get(), y1.get(), st_dev.get(), part_p.get(), part_p_split.get(), mode, direct};
   }
-  DualArgs<T> dargs(int mode) {
+  DualArgs<T> dargs() {
     return DualArgs<T>{B->A.view<T>(), view_d(), plan_p.inst_cta_begin.get(), plan_p.inst_split_begin.get(),
                        dx.get(), b, y0.get(), y1.get(), kx0.get(), kx1.get(), sy.get(), skx.get(), st_dev.get(),
-                       part_p.get(), part_p_split.get(), part_d.get(), part_d_split.get(), mode, direct};
+                       part_p.get(), part_p_split.get(), part_d.get(), part_d_split.get(), direct};
   }
-  void launch_pair(int mode, cudaStream_t s) {
-    launch_step(primal_step_kernel<T>, grid_p, s, pargs(mode));
-    launch_step(dual_step_kernel<T>, grid_d, s, dargs(mode));
-    launches += 2;
-  }
-  void launch_pair(int mode) { launch_pair(mode, B->stream); }
   cudaGraphExec_t capture(int pairs) {
     cudaStream_t s = B->stream;
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     for (int k = 0; k < pairs; ++k) {
       launch_step(primal_step_kernel<T>, grid_p, s, pargs(kStepNormal));
-      launch_step(dual_step_kernel<T>, grid_d, s, dargs(kStepNormal));
+      launch_step(dual_step_kernel<T>, grid_d, s, dargs());
     }
     cudaMemcpyAsync(st_host.p, st_dev.get(), sizeof(StepState) * count, cudaMemcpyDeviceToHost, s);
     CK(cudaStreamEndCapture(s, &g));
@@ -692,6 +685,8 @@ static void run_batch(gpdhg_batch* B, BatchWorkspace<T>& W, const gpdhg_params& 
         st[k].attempts_in_chunk = 0;
         st[k].max_attempts_in_chunk = 1 << 30;
         st[k].iter_start_tau = st[k].tau;
+        st[k].half_over_omega = 0.5 / st[k].omega;
+        st[k].tto = st[k].tau / st[k].omega;
         st[k].arrive = 0;
         due[k] = 0;
       }

@@ -12,15 +12,7 @@
 
 namespace gpdhg {
 
-// Elements per segmented-reduction item (one CTA each) of an instance's side of `len` elements: a
-// small side spreads over the GPU (one or two elements per thread; an element's FP64 chain takes
-// about 1 us), a large one is cut into one wave of 3 CTAs on each of 152 SMs, so that no partly
-// filled wave follows (the transportation LP's column pass: 977 CTAs 97 us) and a CTA's own
-// reduction is small beside its elements.
-constexpr int seg_len(int len) {
-  const int per_thread = (len + 256 * 456 - 1) / (256 * 456);
-  return 256 * (per_thread < 2 && len > (1 << 15) ? 2 : (per_thread < 1 ? 1 : per_thread));
-}
+constexpr int kSegLen = 1024;   // elements per segmented-reduction item (one CTA each)
 
 template <class T>
 struct BatchWorkspace;
@@ -29,7 +21,7 @@ struct BatchWorkspaceDeleter {
   void operator()(BatchWorkspace<float>* w) const;
 };
 
-// Splits [off[k], off[k+1]) of every instance into seg_len-element items.
+// Splits [off[k], off[k+1]) of every instance into kSegLen-element items.
 void build_seg_items(const std::vector<int32_t>& off, std::vector<SegItem>& items, std::vector<int32_t>& begin);
 
 }  // namespace gpdhg

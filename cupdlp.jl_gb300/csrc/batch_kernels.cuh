@@ -19,11 +19,12 @@ namespace gpdhg {
 // partials; then one CTA per instance and quantity reduces the instance's items in order. (One
 // CTA per instance for all quantities took 15-34 us on 1,000-2,000 items, its loads of 25
 // quantities one after the other; one CTA each takes 6 us.) st NULL: every instance is active.
-// The passes are bound by the FP64 pipe (62-84% busy) and the latency of a thread's dozen loads,
-// so 3 CTAs per SM (80 registers, 50 bytes spilled in the column pass; 2 CTAs: 107 us against
-// 70). Cold-cache times, plainly written FP64 arithmetic -> now: column pass of the transportation
-// LP (1M columns, FP64) 194 -> 70 us, of the power-law LP (2M, FP32) 428 -> 138 us, its row pass
-// (1M rows) 127 -> 63-70 us.
+// The passes are bound by the FP64 pipe (62-81% busy) and the latency of a thread's dozen loads, so
+// 3 CTAs per SM (80 registers, some spilled in the column pass; 2 CTAs: 110 and 212 us for the two
+// column passes below). Cold-cache times, FP64 arithmetic plainly written -> as it is: column pass
+// of the transportation LP (1M columns, FP64) 194 -> 101 us, of the power-law LP (2M, FP32) 428 ->
+// 189 us, its row pass (1M rows) 127 -> 93 us. (Longer segments, in one wave of CTAs, take 70, 138
+// and 70 us, but add the restart scores in another order.)
 template <int Q, unsigned MAXMASK, class F>
 __global__ void __launch_bounds__(kBlock, 3) seg_reduce_kernel(const SegItem* items, const StepState* st, F f,
                                                             double* partials, int num_items) {
@@ -53,8 +54,8 @@ struct SegSide {
 constexpr int kEvalStride = 64;   // results per instance: rows' at 0, columns' at kEvalOutN
 constexpr int kEvalOutN = 32;
 // Grid (quantities of both sides, instances).
-inline __global__ void __launch_bounds__(kBlock) seg_finalize_kernel(SegSide a, SegSide b, const StepState* st) {
-  __shared__ double sh[32];
+static __global__ void __launch_bounds__(kBlock) seg_finalize_kernel(SegSide a, SegSide b, const StepState* st) {
+  __shared__ double sh[kBlock], res[1];
   const int inst = blockIdx.y;
   if (st && !st[inst].eval_active) return;
   const bool second = (int)blockIdx.x >= a.quantities;
@@ -63,11 +64,11 @@ inline __global__ void __launch_bounds__(kBlock) seg_finalize_kernel(SegSide a, 
   const bool is_max = (s.maxmask >> q) & 1u;
   const double* p = s.partials + (size_t)q * s.num_items;
   const int k1 = s.inst_item_begin[inst + 1];
-  double acc = 0.0;
+  double acc[1] = {0.0};
   for (int k = s.inst_item_begin[inst] + (int)threadIdx.x; k < k1; k += kBlock)
-    acc = is_max ? nan_max(acc, p[k]) : acc + p[k];
-  acc = is_max ? block_nan_max(acc, sh) : block_sum(acc, sh);
-  if (threadIdx.x == 0) s.out[(size_t)inst * kEvalStride + q] = acc;
+    acc[0] = is_max ? nan_max(acc[0], p[k]) : acc[0] + p[k];
+  const double r = is_max ? block_reduce_q<1, 1u>(acc, sh, res) : block_reduce_q<1, 0u>(acc, sh, res);
+  if (threadIdx.x == 0) s.out[(size_t)inst * kEvalStride + q] = r;
 }
 
 // Per-element helpers driven by per-instance flags / weights.

@@ -113,10 +113,8 @@ struct StepState {
   long long primal_spmv;   // attempts whose primal kernel also ran A'y (a commit)
   const double* pow_table; // [1-(k+1)^-r, 1+(k+1)^-g] for k < pow_table_len (device)
   long long pow_table_len;
-  // written in every attempt by the instance's first dual CTA, for the deciding CTA:
-  double half_w_dx2;       // 0.5 * omega * ||dx|| * ||dx||: the primal part of the movement
-  double half_over_omega;  // 0.5 / omega
-  double f1, f2;           // step-size factors for this attempt's counter
+  double half_over_omega;  // 0.5 / omega, set by the host with omega
+  double tto;              // tau / omega, kept by whoever changes tau or omega (the host, the step decision)
   // set by the host before an evaluation: 1 / sum_w_primal and 1 / sum_w_dual, whether the
   // instance is evaluated, whether it has no average yet (the current point stands in), and
   // whether the last restart point's KKT ingredients are needed

@@ -64,14 +64,21 @@ __device__ __forceinline__ double widen(float v) {
   const unsigned hi = (__float_as_uint(v) & 0x80000000u) | ((mag >> 3) + bias);
   return of_bits((unsigned long long)hi << 32 | (unsigned)(mag << 29));
 }
-// c += a b where p holds, skipped by a warp in which it holds nowhere. (Written as a plain
-// condition, a predicated instruction or a vote around the C expression, the FMA is moved out and
-// computed for every element; a volatile one stays behind the vote.)
+// Sums skipped by a warp in which p holds nowhere: c += a b with one rounding, and with the product
+// rounded first. (Written as a plain condition, a predicated instruction or a vote around the C
+// expression, the arithmetic is moved out and done for every element; a volatile one stays behind
+// the vote.)
 __device__ __forceinline__ void fma_if(bool p, double a, double b, double& c) {
   if (!__any_sync(__activemask(), p)) return;
   a = of_bits(p ? bits_of(a) : 0ULL);
   b = of_bits(p ? bits_of(b) : 0ULL);
   asm volatile("fma.rn.f64 %0, %1, %2, %0;" : "+d"(c) : "d"(a), "d"(b));
+}
+__device__ __forceinline__ void add_product_if(bool p, double a, double b, double& c) {
+  if (!__any_sync(__activemask(), p)) return;
+  a = of_bits(p ? bits_of(a) : 0ULL);
+  b = of_bits(p ? bits_of(b) : 0ULL);
+  asm volatile("{\n\t.reg .f64 t;\n\tmul.rn.f64 t, %1, %2;\n\tadd.rn.f64 %0, %0, t;\n\t}" : "+d"(c) : "d"(a), "d"(b));
 }
 
 __device__ __forceinline__ double warp_nan_max(double v) {
@@ -153,6 +160,8 @@ __device__ __forceinline__ long long bits_key(double v) {   // order_key without
   const long long b = (long long)bits_of(v);
   return b ^ (long long)((unsigned long long)(b >> 63) >> 1);
 }
+// kFused: the square is added with one rounding, else rounded first.
+template <bool kFused>
 __device__ __forceinline__ void add_violation(double x, double l, double u, double& sq, double& mx) {
   const long long k = bits_key(x);
   const bool below = k < bits_key(l), above = bits_key(u) < k;
@@ -160,11 +169,11 @@ __device__ __forceinline__ void add_violation(double x, double l, double u, doub
   if (!(below || above || plain)) return;
   if (plain) {
     const double lv = pos_part(l - x), uv = pos_part(x - u);
-    sq += lv * lv + uv * uv;
+    sq = __dadd_rn(sq, __fma_rn(lv, lv, __dmul_rn(uv, uv)));
     mx = nan_max(mx, nan_max(lv, uv));
   } else {
     const double v = of_bits(bits_of(below ? l : x)) - of_bits(bits_of(below ? x : u));
-    sq = fma(v, v, sq);
+    sq = kFused ? fma(v, v, sq) : __dadd_rn(sq, __dmul_rn(v, v));
     mx = nan_max(mx, v);
   }
 }
@@ -184,9 +193,12 @@ __device__ __forceinline__ double cost_residual(double g, bool kept) {
 }
 // Adds the dual objective's term of a kept reduced cost (:120-126): l rc for rc > 0, u rc for
 // rc < 0, nothing for NaN; a zero bound adds nothing to a finite rc.
+template <bool kFused>
 __device__ __forceinline__ void add_bound_term(double g, bool kept, double l, double u, double& sum) {
   const double bound = of_bits(bits_negative(g) ? bits_of(u) : bits_of(l));
-  fma_if(kept && !bits_nan(g) && (!bits_zero(bound) || !bits_finite(g)), bound, g, sum);
+  const bool counts = kept && !bits_nan(g) && (!bits_zero(bound) || !bits_finite(g));
+  if constexpr (kFused) fma_if(counts, bound, g, sum);
+  else add_product_if(counts, bound, g, sum);
 }
 // The constraint violation b - Kx, or its positive part on an inequality row (:26-45).
 __device__ __forceinline__ double row_violation(double d, bool ineq) {
@@ -324,11 +336,11 @@ struct EvalPassN {
   __device__ __forceinline__ void point(T xv, T gv, double l, double u, double c, bool fl, bool fu, double* a) const {
     const double x = widen(xv), g = widen(gv);
     double unused = 0.0;
-    add_violation(x, l, u, a[0], unused);
+    add_violation<false>(x, l, u, a[0], unused);
     a[1] = fma(c, x, a[1]);
     const bool kept = keeps_cost(g, fl, fu);
     add_square(cost_residual(g, kept), a[2]);
-    add_bound_term(g, kept, l, u, a[3]);
+    add_bound_term<false>(g, kept, l, u, a[3]);
   }
   __device__ __forceinline__ void operator()(const Params& s, int j, double* a) const {
     const T cs = c[j], xc = x[j];
@@ -348,7 +360,7 @@ struct EvalPassN {
       const double g = widen(ga) * var[j];                    // :472-473
       const double l = ol[j], u = ou[j], c = oc[j];
       const bool fl = bits_finite(l), fu = bits_finite(u);
-      add_violation(x, l, u, a[kN_LuSq], a[kN_LuMax]);
+      add_violation<true>(x, l, u, a[kN_LuSq], a[kN_LuMax]);
       a[kN_Cx] = fma(c, x, a[kN_Cx]);
       a[kN_XMax] = nan_max(a[kN_XMax], x);
       a[kN_XSq] = fma(x, x, a[kN_XSq]);
@@ -356,7 +368,7 @@ struct EvalPassN {
       const double rcv = cost_residual(g, kept);
       add_square(rcv, a[kN_RcvSq]);
       a[kN_RcvMax] = nan_max(a[kN_RcvMax], rcv);
-      add_bound_term(g, kept, l, u, a[kN_Contrib]);
+      add_bound_term<true>(g, kept, l, u, a[kN_Contrib]);
       // primal ray, before division by ||x||_inf: bounds 0 where finite (:335-336)
       const bool xnan = bits_nan(x);
       if (xnan ? fl || fu : (bits_negative(x) ? fl : fu)) a[kN_RayLuMax] = nan_max(a[kN_RayLuMax], x);
@@ -364,7 +376,7 @@ struct EvalPassN {
       const double gr = g - c;
       const bool keptr = keeps_cost(gr, fl, fu);
       a[kN_RayRcvMax] = nan_max(a[kN_RayRcvMax], cost_residual(gr, keptr));
-      add_bound_term(gr, keptr, l, u, a[kN_RayContrib]);
+      add_bound_term<true>(gr, keptr, l, u, a[kN_RayContrib]);
       if (keptr) a[kN_RayRcMax] = nan_max(a[kN_RayRcMax], gr);
     }
     double* k = a + kEvalNQ;

@@ -57,7 +57,7 @@ struct ColumnStats {
   __device__ __forceinline__ void operator()(long long j, double* a) const {
     const double xv = x[j], lv = l[j], uv = u[j], cv = c[j];
     const bool fl = bits_finite(lv), fu = bits_finite(uv);
-    add_violation(xv, lv, uv, a[kA_LuSq], a[kA_LuMax]);
+    add_violation<true>(xv, lv, uv, a[kA_LuSq], a[kA_LuMax]);
     a[kA_Cx] = fma(cv, xv, a[kA_Cx]);
     a[kA_XMax] = nan_max(a[kA_XMax], xv);
     a[kA_XSq] = fma(xv, xv, a[kA_XSq]);
@@ -66,7 +66,7 @@ struct ColumnStats {
     const double rcv = cost_residual(g, kept);
     add_square(rcv, a[kA_RcvSq]);
     a[kA_RcvMax] = nan_max(a[kA_RcvMax], rcv);
-    add_bound_term(g, kept, lv, uv, a[kA_Contrib]);
+    add_bound_term<true>(g, kept, lv, uv, a[kA_Contrib]);
     a[kA_CSq] = fma(cv, cv, a[kA_CSq]);
     a[kA_CMax] = nan_max(a[kA_CMax], cv);
   }

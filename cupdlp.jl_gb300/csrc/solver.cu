@@ -234,19 +234,13 @@ struct Workspace {
     return PrimalArgs<T>{P->At.view<T>(), plan_p.view(), c, l, u, x.get(), dx.get(), kty.get(), sx.get(),
                          y0.get(), y1.get(), st_dev.get(), part_p.get(), part_p_split.get(), mode, direct};
   }
-  DualArgs<T> dual_args(int mode) {
+  DualArgs<T> dual_args() {
     return DualArgs<T>{P->A.view<T>(), plan_d.view(), plan_p.inst_cta_begin.get(), plan_p.inst_split_begin.get(),
                        dx.get(), b, y0.get(), y1.get(), kx0.get(), kx1.get(), sy.get(), skx.get(), st_dev.get(),
-                       part_p.get(), part_p_split.get(), part_d.get(), part_d_split.get(), mode, direct};
+                       part_p.get(), part_p_split.get(), part_d.get(), part_d_split.get(), direct};
   }
   void launch_primal(int mode, cudaStream_t s) { launch_step(primal_step_kernel<T>, plan_p.num_ctas, s, primal_args(mode)); }
-  void launch_dual(int mode, cudaStream_t s) { launch_step(dual_step_kernel<T>, plan_d.num_ctas, s, dual_args(mode)); }
-
-  void launch_pair(int mode, cudaStream_t s) {
-    launch_primal(mode, s);
-    launch_dual(mode, s);
-    P->launches += 2;
-  }
+  void launch_dual(cudaStream_t s) { launch_step(dual_step_kernel<T>, plan_d.num_ctas, s, dual_args()); }
 
   cudaGraphExec_t capture(int pairs) {
     cudaStream_t s = P->stream;
@@ -254,7 +248,7 @@ struct Workspace {
     CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     for (int k = 0; k < pairs; ++k) {
       launch_primal(kStepNormal, s);
-      launch_dual(kStepNormal, s);
+      launch_dual(s);
     }
     cudaMemcpyAsync(st_host.p, st_dev.get(), sizeof(StepState), cudaMemcpyDeviceToHost, s);
     cudaError_t e = cudaStreamEndCapture(s, &g);
@@ -280,7 +274,7 @@ struct Workspace {
     for (int k = 0; k < pairs; ++k) {
       launch_primal(kStepNormal, s);
       CK(cudaEventRecord(pev[2 * k + 1], s));
-      launch_dual(kStepNormal, s);
+      launch_dual(s);
       CK(cudaEventRecord(pev[2 * k + 2], s));
     }
     CK_LAUNCH();
@@ -386,14 +380,8 @@ bool run_phase(gpdhg_problem* P, Workspace<T>& W, const gpdhg_params& prm, LoopS
   qi.obj_const = P->obj_const;
   qi.linf_c = P->linf_c; qi.linf_b = P->linf_b; qi.l2_c = P->l2_c; qi.l2_b = P->l2_b;
 
-  // The pinned mirror is edited right after this call, so the copy must have landed.
-  auto push_state = [&]() {
-    CK(cudaMemcpyAsync(W.st_dev.get(), W.st_host.p, sizeof(StepState), cudaMemcpyHostToDevice, s));
-    CK(cudaStreamSynchronize(s));
-  };
-  // The same copy when the mirror stays untouched until the stream has passed it (the step
-  // graphs that follow end by copying the state back into the mirror, and the host reads it
-  // only after synchronising with them).
+  // The state to the device. The mirror stays untouched until the stream has passed the copy: the
+  // host edits it only after synchronising with the work that follows.
   auto push_state_async = [&]() {
     CK(cudaMemcpyAsync(W.st_dev.get(), W.st_host.p, sizeof(StepState), cudaMemcpyHostToDevice, s));
   };
@@ -564,6 +552,8 @@ bool run_phase(gpdhg_problem* P, Workspace<T>& W, const gpdhg_params& prm, LoopS
     st.attempts_in_chunk = 0;
     st.max_attempts_in_chunk = 1 << 30;
     st.iter_start_tau = st.tau;
+    st.half_over_omega = 0.5 / st.omega;
+    st.tto = st.tau / st.omega;
     st.arrive = 0;
     push_state_async();
     const auto tb = Clock::now();

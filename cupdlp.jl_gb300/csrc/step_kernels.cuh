@@ -92,32 +92,35 @@ struct DualArgs {
   const double* part_p_split;
   double* part_d;        // [interaction | ||dy||^2] per CTA (num_ctas each)
   double* part_d_split;  // (interaction, ||dy||^2) of each split row
-  int mode;
   int direct;            // dx holds x^ and the row sums are K x^ (see above)
 };
 
-// Sums over the CTA of Q per-thread partials in a fixed order, valid in thread 0; `sh`
-// holds Q * kBlock doubles and may be reused by consecutive calls. FP64 partials go through
-// shared memory: lane l of warp 0 adds entry l of every warp in warp order, then one shuffle
-// tree finishes (12 warp-wide FP64 adds per quantity, where a shuffle tree in every warp
-// takes 40: GB300 issues FP64 at 2 lanes per SM and cycle). FP32 partials: a shuffle tree
-// per warp in FP32, the warp sums added in FP64.
-template <int Q, class T>
-__device__ __forceinline__ void cta_sums(const T (&v)[Q], double (&out)[Q], double* sh) {
+// Sums over the CTA of Q <= 8 per-thread partials in a fixed order: out[q] in shared memory, complete
+// after the final barrier; `sh` holds Q * kBlock doubles and may be reused by consecutive calls. An
+// FP64 addition takes 64 cycles and the pipe 2 lanes per SM and cycle, so FP64 partials go through
+// shared memory and warp q adds quantity q: lane l entry l of every warp in warp order, then a
+// shuffle tree (12 dependent additions; two quantities one after the other took 2,300 cycles). FP32
+// partials: a shuffle tree per warp in FP32, the warp sums added in FP64 in warp order.
+// post(q, sum), run by the one thread that has sum q, gives what out[q] takes.
+struct KeepSum {
+  __device__ __forceinline__ double operator()(int, double sum) const { return sum; }
+};
+template <int Q, class T, class Post = KeepSum>
+__device__ __forceinline__ void cta_sums(const T (&v)[Q], double* out, double* sh, Post post = Post()) {
+  static_assert(Q <= kBlock / 32, "one warp per quantity");
   const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
-  __syncthreads();  // a previous call's readers are done with sh
+  __syncthreads();  // a previous call's readers are done with sh and out
   if constexpr (sizeof(T) == 8) {
 #pragma unroll
     for (int q = 0; q < Q; ++q) sh[q * kBlock + t] = v[q];
     __syncthreads();
-    if (t < 32) {
+    if (warp < Q) {
+      const double* c = sh + warp * kBlock + lane;
+      double sum = c[0];
 #pragma unroll
-      for (int q = 0; q < Q; ++q) {
-        double s = sh[q * kBlock + lane];
-#pragma unroll
-        for (int w = 1; w < kBlock / 32; ++w) s += sh[q * kBlock + w * 32 + lane];
-        out[q] = warp_sum(s);
-      }
+      for (int w = 1; w < kBlock / 32; ++w) sum += c[32 * w];
+      sum = warp_sum(sum);
+      if (lane == 0) out[warp] = post(warp, sum);
     }
   } else {
 #pragma unroll
@@ -126,15 +129,14 @@ __device__ __forceinline__ void cta_sums(const T (&v)[Q], double (&out)[Q], doub
       if (lane == 0) sh[q * 32 + warp] = (double)ws;
     }
     __syncthreads();
-    if (t == 0) {
+    if (warp < Q && lane == 0) {
+      double sum = sh[warp * 32];
 #pragma unroll
-      for (int q = 0; q < Q; ++q) {
-        double s = 0.0;
-        for (int w = 0; w < kBlock / 32; ++w) s += sh[q * 32 + w];
-        out[q] = s;
-      }
+      for (int w = 1; w < kBlock / 32; ++w) sum += sh[warp * 32 + w];
+      out[warp] = post(warp, sum);
     }
   }
+  __syncthreads();
 }
 
 // One lane's epilogue inputs for its row of a tile (issued with the tile's matrix loads).
@@ -161,61 +163,83 @@ constexpr bool kDenseEpilogue = sizeof(T) == 8;
 template <class T>
 constexpr int kDenseSlots = kDenseEpilogue<T> ? kTilesPerCtaMax * kTileRows : 1;
 
+// What a primal pass takes from its instance's state: whether an accepted step waits for its
+// commit, that step's averaging weight, step_size / primal_weight and the current dual.
 template <class T>
-__global__ void __launch_bounds__(kBlock, kPrimalCtasPerSm<T>) primal_step_kernel(PrimalArgs<T> a) {
-  __shared__ T rs_all[kBlock / 32][32];
-  __shared__ double red[kBlock];
-  __shared__ T wlane[kBlock];
-  __shared__ Tile tl[kTilesPerCtaMax];
-  const int b = a.plan.cta_map ? a.plan.cta_map[blockIdx.x] : (int)blockIdx.x;
+struct PrimalScalars {
+  bool pending;
+  T w;
+  T tto;
+  const T* yg;
+};
+
+// Column j's epilogue inputs.
+template <class T>
+__device__ __forceinline__ void primal_load(const PrimalArgs<T>& a, bool pending, bool commit_only, int j,
+                                            PrimalIn<T>& e) {
+  if (!commit_only) {
+    e.c = lds(a.c + j);
+    e.l = lds(a.l + j);
+    e.u = lds(a.u + j);
+  }
+  if (pending) {
+    e.dx = lds(a.dx + j);
+    if (!a.direct) e.x = lds(a.x + j);
+    e.sx = lds(a.sx + j);
+  } else {
+    e.x = lds(a.x + j);
+    e.dx = lds(a.kty + j);
+  }
+}
+// x^ = proj(x - (tau/omega)(c - K'y)) and dx (:177-197), which is returned; out is what the dual
+// pass gathers.
+template <class T>
+__device__ __forceinline__ T primal_candidate(const PrimalArgs<T>& a, T tto, int j, T xv, T ktyv, const PrimalIn<T>& e,
+                                              T& out) {
+  T v = xv - tto * (e.c - ktyv);
+  v = imin(e.u, imax(e.l, v));   // min(u, max(l, .)) (:192)
+  const T d = v - xv;
+  out = a.direct ? v : d;
+  a.dx[j] = out;                 // gathered by the dual kernel next: a normal (L2-resident) store
+  return d;
+}
+// The accepted step applied to column j with K'y = ktyv; returns the new x.
+template <class T>
+__device__ __forceinline__ T primal_commit(const PrimalArgs<T>& a, T w, int j, T ktyv, const PrimalIn<T>& e) {
+  const T xv = a.direct ? e.dx : e.x + e.dx;   // x += dx (:303)
+  sts(a.x + j, xv);
+  sts(a.kty + j, ktyv);                         // K'y = A'y (:307)
+  sts(a.sx + j, e.sx + xv * w);                 // weighted sum (src/saddle_point_gpu.jl:137)
+  return xv;
+}
+
+// Shared memory of a CTA's primal work.
+template <class T>
+struct PrimalShared {
+  T rs_all[kBlock / 32][32];
+  T wlane[kBlock];
+  T lsum[kDenseEpilogue<T> ? kTilesPerCtaMax : 1];   // sums of FP64 warp-streamed rows
+};
+
+// One CTA's primal work on its nt staged tiles: the pending commit and the next candidate of
+// every row (commit_only: the commit alone). acc takes the thread's share of ||dx||^2.
+template <class T>
+__device__ __forceinline__ void primal_work(const PrimalArgs<T>& a, const PrimalScalars<T>& sc, PrimalShared<T>& sm,
+                                            const Tile* tl, int nt, bool commit_only, T& acc) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // programmatic dependent launch: stage the constant tile descriptors, wait for the previous
-  // kernel, and only then let the next (dual) kernel's CTAs launch: once all of ours have
-  // passed this point, the state the previous dual kernel wrote is complete, so the dual
-  // kernel may read it before its own wait (this kernel never writes it)
-  const int nt = stage_tiles(a.plan.tiles, a.plan.cta_tile_begin[b], a.plan.cta_tile_begin[b + 1], tl);
-  pdl_wait();
-  pdl_launch_dependents();
-  const StepState* st = a.st + a.plan.cta_inst[b];
-  if (st->done) return;
-  const int pending = st->pending_commit;
-  const bool commit_only = a.mode == kStepCommitOnly;
-  if (commit_only && !pending) return;
-  const bool direct = a.direct != 0;
-  // step_size / primal_weight: one FP64 division per CTA (GB300's FP64 pipe is narrow)
-  __shared__ double s_tto;
-  if (threadIdx.x == 0) s_tto = st->tau / st->omega;
-  __syncthreads();
-  const T w = (T)st->commit_weight;
-  const T tto = (T)s_tto;
-  const T* yg = st->parity ? a.y1 : a.y0;
-  T* rs = rs_all[warp];
-  T acc = T(0);
+  const bool pending = sc.pending;
+  const T w = sc.w, tto = sc.tto;
+  const T* yg = sc.yg;
+  T* rs = sm.rs_all[warp];
   auto load_in = [&](const Tile& t, PrimalIn<T>& e) {
     e = PrimalIn<T>{};
-    if (lane >= t.rows) return;
-    const int j = t.row_begin + lane;
-    if (!commit_only) {
-      e.c = lds(a.c + j);
-      e.l = lds(a.l + j);
-      e.u = lds(a.u + j);
-    }
-    if (pending) {
-      e.dx = lds(a.dx + j);
-      if (!direct) e.x = lds(a.x + j);
-      e.sx = lds(a.sx + j);
-    } else {
-      e.x = lds(a.x + j);
-      e.dx = lds(a.kty + j);
-    }
+    if (lane < t.rows) primal_load(a, pending, commit_only, t.row_begin + lane, e);
   };
-  // x^ = proj(x - (tau/omega)(c - K'y)) and dx (:177-197); its ||dx||^2 term goes into the
-  // CTA's sum with one FMA, or into the split row's own slot
+  // the candidate; its ||dx||^2 term goes into the CTA's sum with one FMA, or into the split
+  // row's own slot
   auto candidate = [&](int j, T xv, T ktyv, const PrimalIn<T>& e, const Tile& t, bool split) {
-    T v = xv - tto * (e.c - ktyv);
-    v = imin(e.u, imax(e.l, v));   // min(u, max(l, .)) (:192)
-    const T d = v - xv;
-    a.dx[j] = direct ? v : d;      // gathered by the dual kernel next: a normal (L2-resident) store
+    T out;
+    const T d = primal_candidate(a, tto, j, xv, ktyv, e, out);
     if (split) {
       a.part_p_split[t.split] = (double)(d * d);
       __threadfence();
@@ -232,10 +256,7 @@ __global__ void __launch_bounds__(kBlock, kPrimalCtasPerSm<T>) primal_step_kerne
       if (split) rows = split_finish(t, a.plan, rs) ? 1 : 0;
       if (lane < rows) {
         const T ktyv = rs[lane];
-        const T xv = direct ? e.dx : e.x + e.dx;   // x += dx (:303)
-        sts(a.x + j, xv);
-        sts(a.kty + j, ktyv);                       // K'y = A'y (:307)
-        sts(a.sx + j, e.sx + xv * w);               // weighted sum (src/saddle_point_gpu.jl:137)
+        const T xv = primal_commit(a, w, j, ktyv, e);
         if (!commit_only) candidate(j, xv, ktyv, e, t, split);
       }
       __syncwarp();
@@ -255,41 +276,28 @@ __global__ void __launch_bounds__(kBlock, kPrimalCtasPerSm<T>) primal_step_kerne
     Tile t{};
     if (has) t = tl[q];
     if (has && sub == 0) load_in(t, E0);
-    if (pending) group_row_sum(a.At.col, a.At.val, yg, t, has, W, sub, wlane, rs);
+    if (pending) group_row_sum(a.At.col, a.At.val, yg, t, has, W, sub, sm.wlane, rs);
     if (has && sub == 0) finish(t, E0);
   } else if (kDenseEpilogue<T> && nt > 0 && tl[0].e_log2 == kWarpLong) {
     // FP64 CTAs of warp-streamed rows (one row per tile): the warps stream their rows' sums
     // into shared memory, then thread q runs the epilogue of tile q's row, so the FP64
     // instructions of the epilogue run on full warps instead of on each warp's lane 0
-    __shared__ T lsum[kDenseEpilogue<T> ? kTilesPerCtaMax : 1];
     if (pending)
       for (int q = warp; q < nt; q += kBlock / 32) {
         const T sum = long_row_sum(a.At.col, a.At.val, yg, tl[q]);
-        if (lane == 0) lsum[q] = sum;
+        if (lane == 0) sm.lsum[q] = sum;
       }
     __syncthreads();
     for (int q = threadIdx.x; q < nt; q += kBlock) {
       const Tile& t = tl[q];
       const int j = t.row_begin;
       PrimalIn<T> e{};
-      if (!commit_only) {
-        e.c = lds(a.c + j);
-        e.l = lds(a.l + j);
-        e.u = lds(a.u + j);
-      }
+      primal_load(a, pending, commit_only, j, e);
       if (pending) {
-        e.dx = lds(a.dx + j);
-        if (!direct) e.x = lds(a.x + j);
-        e.sx = lds(a.sx + j);
-        const T ktyv = lsum[q];
-        const T xv = direct ? e.dx : e.x + e.dx;   // x += dx (:303)
-        sts(a.x + j, xv);
-        sts(a.kty + j, ktyv);                       // K'y = A'y (:307)
-        sts(a.sx + j, e.sx + xv * w);               // weighted sum (src/saddle_point_gpu.jl:137)
+        const T ktyv = sm.lsum[q];
+        const T xv = primal_commit(a, w, j, ktyv, e);
         if (!commit_only) candidate(j, xv, ktyv, e, t, false);
       } else {
-        e.x = lds(a.x + j);
-        e.dx = lds(a.kty + j);
         candidate(j, e.x, e.dx, e, t, false);
       }
     }
@@ -306,57 +314,77 @@ __global__ void __launch_bounds__(kBlock, kPrimalCtasPerSm<T>) primal_step_kerne
       finish(t, E0);
     }
   }
+}
+
+template <class T>
+__global__ void __launch_bounds__(kBlock, kPrimalCtasPerSm<T>) primal_step_kernel(PrimalArgs<T> a) {
+  __shared__ PrimalShared<T> sm;
+  __shared__ union {   // the tiles are done with when the sums begin (cta_sums' first barrier)
+    Tile tl[kTilesPerCtaMax];
+    double red[kBlock];
+  } ph;
+  Tile* const tl = ph.tl;
+  double* const red = ph.red;
+  const int b = a.plan.cta_map ? a.plan.cta_map[blockIdx.x] : (int)blockIdx.x;
+  // programmatic dependent launch: stage the constant tile descriptors, wait for the previous
+  // kernel, and only then let the next (dual) kernel's CTAs launch: once all of ours have
+  // passed this point, the state the previous dual kernel wrote is complete, so the dual
+  // kernel may read it before its own wait (this kernel never writes it)
+  const int nt = stage_tiles(a.plan.tiles, a.plan.cta_tile_begin[b], a.plan.cta_tile_begin[b + 1], tl);
+  pdl_wait();
+  pdl_launch_dependents();
+  const StepState* st = a.st + a.plan.cta_inst[b];
+  if (st->done) return;
+  const int pending = st->pending_commit;
+  const bool commit_only = a.mode == kStepCommitOnly;
+  if (commit_only && !pending) return;
+  const PrimalScalars<T> sc{pending != 0, (T)st->commit_weight, (T)st->tto, st->parity ? a.y1 : a.y0};
+  T acc = T(0);
+  primal_work(a, sc, sm, tl, nt, commit_only, acc);
   if (commit_only) return;
   const T v[1] = {acc};
-  double o[1];
+  __shared__ double o[1];
   cta_sums<1>(v, o, red);
   if (threadIdx.x == 0) a.part_p[b] = o[0];
 }
 
-// Primal part of take_step!'s movement (:324-333), 0.5 * omega * ||dx||^2 evaluated as the
-// reference does (the norm squared again).
-__device__ __forceinline__ double half_w_dx2(double omega, double dx2) {
-  const double ndx = sqrt(dx2);
-  return 0.5 * omega * ndx * ndx;
-}
-
-// Decision of take_step! for one attempt, on a copy of the instance's state (the caller
-// writes it back). f1 / f2 are the step-size factors (1 - (k+1)^-r), (1 + (k+1)^-g)
-// for the attempt counter after this attempt, hw_dx2 = half_w_dx2(omega, ||dx||^2) and
-// hoo = 0.5 / omega, all prepared by the instance's first dual CTA while the others still run.
-__device__ __forceinline__ void step_decision(StepState& s, double f1, double f2, double inter_signed, double hw_dx2,
-                                              double hoo, double dy2) {
+// Decision of take_step! for one attempt on the instance's state, by one thread: its chain of
+// dependent FP64 operations, the division above all, is the attempt's serial tail, so comparisons
+// run on the integer pipe. f1 / f2 are the step-size factors
+// (1 - (k+1)^-r), (1 + (k+1)^-g) for the attempt counter after this attempt; movement is
+// 0.5 omega ||dx||^2 + 0.5 / omega ||dy||^2. Returns false on the numerical error of
+// :384-390 (terminate at the next evaluation; the step size is left as it is).
+__device__ __forceinline__ bool step_decision(StepState& s, double f1, double f2, double inter_signed, double movement) {
+  const long long bi = __double_as_longlong(inter_signed) & 0x7fffffffffffffffLL;
+  const bool interacts = !s.constant_step && bi > 0 && bi <= 0x7ff0000000000000LL;   // |inter| > 0, not NaN
+  const double tau = s.tau;
+  double limit = __longlong_as_double(0x7ff0000000000000LL);
+  if (interacts) limit = movement / __longlong_as_double(bi);
   s.total_iters += s.constant_step ? 0 : 1;
   s.kkt_passes += 1.0;
   s.attempts_in_chunk += 1;
-  const double tau = s.tau;
-  const double inter = fabs(inter_signed);
-  const double ndy = sqrt(dy2);
-  const double movement = hw_dx2 + hoo * ndy * ndy;
-  double limit;
-  bool accept;
-  if (s.constant_step) {
-    limit = __longlong_as_double(0x7ff0000000000000LL);
-    accept = true;
-  } else {
-    if (inter > 0.0) {
-      limit = movement / inter;
-      if (movement == 0.0) {
-        // :384-390: terminate at the next evaluation; tau is left as it is
-        s.numerical_error = 1;
-        s.done = 1;
-        s.pending_commit = 0;
-        return;
-      }
-    } else {
-      limit = __longlong_as_double(0x7ff0000000000000LL);
-    }
-    accept = tau <= limit;
+  if (interacts && (__double_as_longlong(movement) << 1) == 0) {
+    s.numerical_error = 1;
+    s.done = 1;
+    s.pending_commit = 0;
+    return false;
   }
+  // positive operands and no NaN: order of the bits; else the comparisons as written
+  const long long bl = __double_as_longlong(limit), bt = __double_as_longlong(tau);
+  const bool plain = bl >= 0 && bl <= 0x7ff0000000000000LL && bt >= 0 && bt <= 0x7ff0000000000000LL;
+  const bool accept = s.constant_step || (plain ? bt <= bl : tau <= limit);
+  double next = tau;
+  if (!s.constant_step) {
+    const double first = f1 * limit, second = f2 * tau;
+    const long long b1 = __double_as_longlong(first), b2 = __double_as_longlong(second);
+    const bool both = b1 >= 0 && b1 <= 0x7ff0000000000000LL && b2 >= 0 && b2 <= 0x7ff0000000000000LL;
+    next = both ? __longlong_as_double(b1 < b2 ? b1 : b2) : jmin(first, second);
+  }
+  s.tau = next;
   s.last_limit = limit;
+  s.pending_commit = accept ? 1 : 0;
   if (accept) {
     s.parity ^= 1;
-    s.pending_commit = 1;
     s.commit_weight = s.iter_start_tau;
     s.count_primal += 1;
     s.count_dual += 1;
@@ -364,29 +392,25 @@ __device__ __forceinline__ void step_decision(StepState& s, double f1, double f2
     s.sum_w_dual += s.iter_start_tau;
     s.accepted += 1;
     s.accepted_in_chunk += 1;
+    s.iter_start_tau = next;
   } else {
-    s.pending_commit = 0;
     s.rejected += 1;
   }
-  if (!s.constant_step) {
-    const double first = f1 * limit;
-    const double second = f2 * tau;
-    s.tau = jmin(first, second);
-  }
-  if (accept) s.iter_start_tau = s.tau;
   if (s.accepted_in_chunk >= s.target_in_chunk || s.attempts_in_chunk >= s.max_attempts_in_chunk) s.done = 1;
+  return true;
 }
 
-// Step-size factors for attempt counter k (take_step!, :405-407): the host table while it
-// lasts, else the same formula on the device.
-__device__ __forceinline__ void step_factors(const StepState& s, long long k, double& f1, double& f2) {
-  if (s.pow_table && k < s.pow_table_len) {
-    f1 = __ldcg(s.pow_table + 2 * k);
-    f2 = __ldcg(s.pow_table + 2 * k + 1);
+// Step-size factors of the attempt that the state (in L2 or shared memory) stands before (take_step!,
+// :405-407): the host table while it lasts, else the same formula on the device.
+__device__ __forceinline__ void step_factors(const StepState* st, double (&f)[2]) {
+  const long long k = *(volatile const long long*)&st->total_iters + (*(volatile const int*)&st->constant_step ? 0 : 1);
+  if (st->pow_table && k < st->pow_table_len) {
+    f[0] = __ldcg(st->pow_table + 2 * k);
+    f[1] = __ldcg(st->pow_table + 2 * k + 1);
   } else {
     const double k1 = (double)(k + 1);
-    f1 = 1.0 - 1.0 / pow(k1, s.reduction_exponent);
-    f2 = 1.0 + 1.0 / pow(k1, s.growth_exponent);
+    f[0] = 1.0 - 1.0 / pow(k1, st->reduction_exponent);
+    f[1] = 1.0 + 1.0 / pow(k1, st->growth_exponent);
   }
 }
 
@@ -405,78 +429,77 @@ struct DualIn {
 template <class T>
 constexpr bool kSpanScan = sizeof(T) == 8;
 
+// What a dual pass takes from its instance's state.
 template <class T>
-__global__ void __launch_bounds__(kBlock, kDualCtasPerSm) dual_step_kernel(DualArgs<T> a) {
-  __shared__ T rs_all[kBlock / 32][32];
-  __shared__ T wlane[kBlock];
-  __shared__ T ipart[kBlock / 32][kBlock / 32];
-  __shared__ Tile tl[kTilesPerCtaMax];
-  __shared__ double red[2 * kBlock];
-  __shared__ int is_last;
-  const int b = a.plan.cta_map ? a.plan.cta_map[blockIdx.x] : (int)blockIdx.x;
+struct DualScalars {
+  bool pending;
+  T w;
+  T od;            // primal_weight * step_size
+  const T* ycur;
+  T* ynew;
+  const T* kxcur;
+  T* kxnew;
+};
+
+// Row i's epilogue inputs.
+template <class T>
+__device__ __forceinline__ void dual_load(const DualArgs<T>& a, const DualScalars<T>& sc, int i, DualIn<T>& e) {
+  e.y = lds(sc.ycur + i);
+  e.kx = lds(sc.kxcur + i);
+  e.b = lds(a.b + i);
+  if (sc.pending) {
+    e.sy = lds(a.sy + i);
+    e.sk = lds(a.skx + i);
+  }
+}
+// Row i's pending sums and its candidate y^ (returned) from the row sum rsum, with kdx and d = dy.
+template <class T>
+__device__ __forceinline__ T dual_row(const DualArgs<T>& a, const DualScalars<T>& sc, int i, bool ineq, T rsum,
+                                         const DualIn<T>& e, T& kdx, T& d) {
+  const T y = e.y, kx = e.kx;
+  if (sc.pending) {
+    sts(a.sy + i, e.sy + y * sc.w);
+    sts(a.skx + i, e.sk + kx * sc.w);
+  }
+  kdx = a.direct ? rsum - kx : rsum;
+  T v = y + sc.od * ((e.b - T(2) * kdx) - kx);   // (:247), extrapolation coefficient 1
+  if (ineq) v = imax(v, T(0));                   // (:254)
+  d = v - y;
+  const T out = y + d;                           // y += dy (:306)
+  sc.ynew[i] = out;                              // gathered by the next primal kernel
+  sts(sc.kxnew + i, a.direct ? rsum : kx + kdx); // Kx += K dx (:304)
+  return out;
+}
+
+// Shared memory of a CTA's dual work.
+template <class T>
+struct DualShared {
+  T rs_all[kBlock / 32][32];
+  T wlane[kBlock];
+  T ipart[kBlock / 32][kBlock / 32];
+  T csum[kDenseSlots<T>];                    // FP64 warp tiles: every row's sum,
+  int32_t slot_begin[kTilesPerCtaMax + 1];   // and each tile's first slot in it
+};
+
+// One CTA's dual work on its nt staged tiles: the pending commit's y and Kx sums and the next
+// candidate of every row. acc_i / acc_d take the thread's share of dy . K dx and ||dy||^2.
+template <class T>
+__device__ __forceinline__ void dual_work(const DualArgs<T>& a, const DualScalars<T>& sc, DualShared<T>& sm,
+                                          const Tile* tl, int nt, T& acc_i, T& acc_d) {
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  pdl_launch_dependents();  // the next primal kernel reads the state only after its wait
-  const int nt = stage_tiles(a.plan.tiles, a.plan.cta_tile_begin[b], a.plan.cta_tile_begin[b + 1], tl);
-  // The state this kernel reads was written by the previous dual kernel, which completed
-  // before the primal kernel let this one launch (see there): read it now, from L2 (a line in
-  // this SM's L1 may predate it), so the loads overlap the primal kernel's last CTAs.
-  const StepState* st = a.st_mut + a.plan.cta_inst[b];
-  const int done = __ldcg(&st->done);
-  const int pending = __ldcg(&st->pending_commit);
-  const int p = __ldcg(&st->parity);
-  const double commit_weight = __ldcg(&st->commit_weight);
-  const double od64 = __ldcg(&st->omega) * __ldcg(&st->tau);  // primal_weight * step_size
-  pdl_wait();
-  if (done) return;
-  const bool commit_only = a.mode == kStepCommitOnly;
-  if (commit_only && !pending) return;
-  const bool direct = a.direct != 0;
-  const T w = (T)commit_weight;
-  const T od = (T)od64;
-  const T* ycur = p ? a.y1 : a.y0;
-  T* ynew = p ? a.y0 : a.y1;
-  const T* kxcur = p ? a.kx1 : a.kx0;
-  T* kxnew = p ? a.kx0 : a.kx1;
-  T* rs = rs_all[warp];
-  T acc_i = T(0), acc_d = T(0);
+  T* rs = sm.rs_all[warp];
   auto load_in = [&](const Tile& t, DualIn<T>& e) {
     e = DualIn<T>{};
-    if (lane >= t.rows) return;
-    const int i = t.row_begin + lane;
-    e.y = lds(ycur + i);
-    e.kx = lds(kxcur + i);
-    if (!commit_only) e.b = lds(a.b + i);
-    if (pending) {
-      e.sy = lds(a.sy + i);
-      e.sk = lds(a.skx + i);
-    }
+    if (lane < t.rows) dual_load(a, sc, t.row_begin + lane, e);
   };
   auto finish = [&](const Tile& t, const DualIn<T>& e) {
     const bool split = t.split >= 0;
     const int i = t.row_begin + lane;
-    if (commit_only) {
-      const int rows = (split && t.piece != t.pieces - 1) ? 0 : t.rows;
-      if (lane < rows) {
-        sts(a.sy + i, e.sy + e.y * w);
-        sts(a.skx + i, e.sk + e.kx * w);
-      }
-      return;
-    }
     int rows = t.rows;
     if (split) rows = split_finish(t, a.plan, rs) ? 1 : 0;
     if (lane < rows) {
-      const T rsum = rs[lane];
-      const T y = e.y, kx = e.kx;
-      if (pending) {
-        sts(a.sy + i, e.sy + y * w);
-        sts(a.skx + i, e.sk + kx * w);
-      }
-      const T kdx = direct ? rsum - kx : rsum;
-      T v = y + od * ((e.b - T(2) * kdx) - kx);   // (:247), extrapolation coefficient 1
-      if (i >= t.aux) v = imax(v, T(0));          // (:254)
-      const T d = v - y;
-      ynew[i] = y + d;                            // y += dy (:306); gathered by the next primal kernel
-      sts(kxnew + i, direct ? rsum : kx + kdx);   // Kx += K dx (:304)
+      T kdx, d;
+      dual_row(a, sc, i, i >= t.aux, rs[lane], e, kdx, d);
       if (split) {
         a.part_d_split[2 * t.split] = (double)(kdx * d);
         a.part_d_split[2 * t.split + 1] = (double)(d * d);
@@ -496,7 +519,7 @@ __global__ void __launch_bounds__(kBlock, kDualCtasPerSm) dual_step_kernel(DualA
     // kBlock / 32 warp-streamed rows summed together (interleaved_rows_sum); warp w then
     // finishes row w as if it had streamed it
     load_in(tl[warp], E0);
-    if (!commit_only) interleaved_rows_sum(a.A.col, a.A.val, a.dx, tl, ipart, rs_all);
+    interleaved_rows_sum(a.A.col, a.A.val, a.dx, tl, sm.ipart, sm.rs_all);
     finish(tl[warp], E0);
   } else if (nt > 0 && tl[0].e_log2 <= group_code(1)) {
     const int W = 1 << group_log2(tl[0].e_log2);
@@ -505,13 +528,13 @@ __global__ void __launch_bounds__(kBlock, kDualCtasPerSm) dual_step_kernel(DualA
     Tile t{};
     if (has) t = tl[q];
     if (has && sub == 0) load_in(t, E0);
-    if (!commit_only) group_row_sum(a.A.col, a.A.val, a.dx, t, has, W, sub, wlane, rs);
+    group_row_sum(a.A.col, a.A.val, a.dx, t, has, W, sub, sm.wlane, rs);
     if (has && sub == 0) finish(t, E0);
   } else if (kDenseEpilogue<T>) {
     // warp tiles (never split): every row sum into the CTA's slot buffer, then the epilogue
     // with one row per thread, slot by slot (slot = the row's position among the tiles' rows)
-    __shared__ T csum[kDenseSlots<T>];
-    __shared__ int32_t slot_begin[kTilesPerCtaMax + 1];
+    T* csum = sm.csum;
+    int32_t* slot_begin = sm.slot_begin;
     if (threadIdx.x == 0) {
       int o = 0;
       for (int q = 0; q < nt; ++q) {
@@ -521,14 +544,12 @@ __global__ void __launch_bounds__(kBlock, kDualCtasPerSm) dual_step_kernel(DualA
       slot_begin[nt] = o;
     }
     __syncthreads();
-    if (!commit_only) {
-      for (int q = warp; q < nt; q += kBlock / 32) {
-        const Tile t = tl[q];
-        tile_load(a.A.row_ptr, a.plan.icol, a.plan.ival, t, L0);
-        tile_sums<T, kSpanScan<T>>(a.A.col, a.A.val, a.dx, t, L0, rs);
-        if (lane < t.rows) csum[slot_begin[q] + lane] = rs[lane];
-        __syncwarp();
-      }
+    for (int q = warp; q < nt; q += kBlock / 32) {
+      const Tile t = tl[q];
+      tile_load(a.A.row_ptr, a.plan.icol, a.plan.ival, t, L0);
+      tile_sums<T, kSpanScan<T>>(a.A.col, a.A.val, a.dx, t, L0, rs);
+      if (lane < t.rows) csum[slot_begin[q] + lane] = rs[lane];
+      __syncwarp();
     }
     __syncthreads();
     const int nslots = slot_begin[nt];
@@ -540,24 +561,10 @@ __global__ void __launch_bounds__(kBlock, kDualCtasPerSm) dual_step_kernel(DualA
         else hi = mid - 1;
       }
       const int i = tl[lo].row_begin + (sl - slot_begin[lo]);
-      const T y = lds(ycur + i), kx = lds(kxcur + i);
-      if (commit_only) {
-        sts(a.sy + i, lds(a.sy + i) + y * w);
-        sts(a.skx + i, lds(a.skx + i) + kx * w);
-        continue;
-      }
-      const T bi = lds(a.b + i);
-      if (pending) {
-        sts(a.sy + i, lds(a.sy + i) + y * w);
-        sts(a.skx + i, lds(a.skx + i) + kx * w);
-      }
-      const T rsum = csum[sl];
-      const T kdx = direct ? rsum - kx : rsum;
-      T v = y + od * ((bi - T(2) * kdx) - kx);   // (:247), extrapolation coefficient 1
-      if (i >= tl[lo].aux) v = imax(v, T(0));      // (:254)
-      const T d = v - y;
-      ynew[i] = y + d;                             // y += dy (:306)
-      sts(kxnew + i, direct ? rsum : kx + kdx);    // Kx += K dx (:304)
+      DualIn<T> e{};
+      dual_load(a, sc, i, e);
+      T kdx, d;
+      dual_row(a, sc, i, i >= tl[lo].aux, csum[sl], e, kdx, d);
       acc_i = fma(kdx, d, acc_i);
       acc_d = fma(d, d, acc_d);
     }
@@ -565,107 +572,130 @@ __global__ void __launch_bounds__(kBlock, kDualCtasPerSm) dual_step_kernel(DualA
     for (int q = warp; q < nt; q += kBlock / 32) {
       const Tile t = tl[q];
       load_in(t, E0);
-      if (!commit_only) {
-        tile_load(a.A.row_ptr, a.plan.icol, a.plan.ival, t, L0);
-        tile_sums<T, kSpanScan<T>>(a.A.col, a.A.val, a.dx, t, L0, rs);
-      }
+      tile_load(a.A.row_ptr, a.plan.icol, a.plan.ival, t, L0);
+      tile_sums<T, kSpanScan<T>>(a.A.col, a.A.val, a.dx, t, L0, rs);
       finish(t, E0);
     }
   }
-  const int inst = a.plan.cta_inst[b];
-  const int c0 = a.plan.inst_cta_begin[inst], c1 = a.plan.inst_cta_begin[inst + 1];
-  StepState* stw = a.st_mut + inst;
-  if (!commit_only) {
-    const T v[2] = {acc_i, acc_d};
-    double o[2];
-    cta_sums<2>(v, o, red);
-    if (threadIdx.x == 0) {
-      a.part_d[b] = o[0];
-      a.part_d[a.plan.num_ctas + b] = o[1];
-    }
-    if (b == c0) {
-      // the instance's primal ||dx||^2 in plan order (CTAs, then split rows), summed here
-      // once so that the deciding CTA reads one value instead of every primal partial
-      const int p0 = a.p_cta_begin[inst], p1 = a.p_cta_begin[inst + 1];
-      const int q0 = a.p_split_begin[inst], q1 = a.p_split_begin[inst + 1];
-      double sx[1] = {0.0};
-      for (int k0 = p0 + (int)threadIdx.x; k0 < p1; k0 += 4 * kBlock) {
-        double u[4];
-#pragma unroll
-        for (int j = 0; j < 4; ++j) u[j] = k0 + j * kBlock < p1 ? __ldcg(a.part_p + k0 + j * kBlock) : 0.0;
-#pragma unroll
-        for (int j = 0; j < 4; ++j) sx[0] += u[j];
-      }
-      for (int k = q0 + (int)threadIdx.x; k < q1; k += kBlock) sx[0] += __ldcg(a.part_p_split + k);
-      double ox[1];
-      cta_sums<1>(sx, ox, red);
-      if (threadIdx.x == 0) {
-        // and the decision's other inputs that need no dual partial
-        double f1, f2;
-        step_factors(*st, st->total_iters + (st->constant_step ? 0 : 1), f1, f2);
-        stw->half_w_dx2 = half_w_dx2(st->omega, ox[0]);
-        stw->half_over_omega = 0.5 / st->omega;
-        stw->f1 = f1;
-        stw->f2 = f2;
-      }
-    }
-  }
-  if (threadIdx.x == 0) {
-    __threadfence();
-    const unsigned prev = atomicAdd(&stw->arrive, 1u);
-    is_last = (prev == (unsigned)(c1 - c0 - 1)) ? 1 : 0;
-  }
-  __syncthreads();
-  if (!is_last) return;
-  if (commit_only) {
-    if (threadIdx.x == 0) {
-      stw->pending_commit = 0;
-      stw->arrive = 0;
-    }
-    return;
-  }
-  // the instance's last CTA: the first threads copy the state from L2 (the first CTA's
-  // fields are not in this SM's L1), one 8-byte word each, with the partials' loads; the
-  // barriers of cta_sums order the copy before thread 0 uses it. Partials in a fixed order.
-  __shared__ StepState s;
-  static_assert(sizeof(StepState) % 8 == 0 && sizeof(StepState) / 8 <= kBlock, "StepState copy");
-  if (threadIdx.x < sizeof(StepState) / 8)
+}
+
+constexpr int kStateWords = (int)(sizeof(StepState) / 8);
+static_assert(sizeof(StepState) % 8 == 0 && kStateWords <= kBlock, "StepState copies");
+// The state between L2 and shared memory, one 8-byte word per thread (the caller synchronises).
+__device__ __forceinline__ void load_state(const StepState* st, StepState& s) {
+  if (threadIdx.x < kStateWords)
     reinterpret_cast<unsigned long long*>(&s)[threadIdx.x] =
-        __ldcg(reinterpret_cast<const unsigned long long*>(stw) + threadIdx.x);
-  // one round of loads for both CTA ranges (interaction, ||dy||^2) up to 4 x kBlock CTAs,
-  // all issued before any is added; split-row slots (rare) follow
+        __ldcg(reinterpret_cast<const unsigned long long*>(st) + threadIdx.x);
+}
+__device__ __forceinline__ void store_state(const StepState& s, StepState* st) {
+  if (threadIdx.x < kStateWords)
+    reinterpret_cast<unsigned long long*>(st)[threadIdx.x] = reinterpret_cast<const unsigned long long*>(&s)[threadIdx.x];
+}
+
+// What the step decision needs of the instance's sums, in tot (shared): the interaction, ||dy|| and
+// 0.5 omega ||dx|| ||dx|| (the primal part of take_step!'s movement, :324-333, evaluated as the
+// reference does, the norm squared again). One round of loads for the CTAs' sums of both kernels
+// up to 4 x kBlock CTAs, all issued before any is added; split-row slots (rare) follow. The roots
+// (580 cycles each) are taken side by side, each by the warp that has its sum.
+template <class T>
+__device__ __forceinline__ void step_totals(const DualArgs<T>& a, int inst, const StepState& s, double* tot,
+                                            double* red) {
+  const int c0 = a.plan.inst_cta_begin[inst], c1 = a.plan.inst_cta_begin[inst + 1];
   const int s0 = a.plan.inst_split_begin[inst], s1 = a.plan.inst_split_begin[inst + 1];
-  double sd[2] = {0.0, 0.0};
-  for (int k0 = c0 + (int)threadIdx.x; k0 < c1; k0 += 4 * kBlock) {
-    double ui[4], ud[4];
+  const int p0 = a.p_cta_begin[inst], p1 = a.p_cta_begin[inst + 1];
+  const int q0 = a.p_split_begin[inst], q1 = a.p_split_begin[inst + 1];
+  double sd[3] = {0.0, 0.0, 0.0};
+  for (int k0 = (int)threadIdx.x; k0 < max(c1 - c0, p1 - p0); k0 += 4 * kBlock) {
+    double ui[4], ud[4], ux[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      const bool in = k0 + j * kBlock < c1;
-      ui[j] = in ? __ldcg(a.part_d + k0 + j * kBlock) : 0.0;
-      ud[j] = in ? __ldcg(a.part_d + a.plan.num_ctas + k0 + j * kBlock) : 0.0;
+      const int k = k0 + j * kBlock;
+      const bool in = k < c1 - c0;
+      ui[j] = in ? __ldcg(a.part_d + c0 + k) : 0.0;
+      ud[j] = in ? __ldcg(a.part_d + a.plan.num_ctas + c0 + k) : 0.0;
+      ux[j] = k < p1 - p0 ? __ldcg(a.part_p + p0 + k) : 0.0;
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
+      if (k0 + j * kBlock >= max(c1 - c0, p1 - p0)) break;
       sd[0] += ui[j];
       sd[1] += ud[j];
+      sd[2] += ux[j];
     }
   }
   for (int k = s0 + (int)threadIdx.x; k < s1; k += kBlock) {
     sd[0] += __ldcg(a.part_d_split + 2 * k);
     sd[1] += __ldcg(a.part_d_split + 2 * k + 1);
   }
-  double tot[2];
-  cta_sums<2>(sd, tot, red);
+  for (int k = q0 + (int)threadIdx.x; k < q1; k += kBlock) sd[2] += __ldcg(a.part_p_split + k);
+  cta_sums<3>(sd, tot, red, [&](int q, double sum) {
+    if (q == 0) return sum;
+    const double norm = sqrt(sum);
+    return q == 1 ? norm : __dmul_rn(__dmul_rn(0.5 * s.omega, norm), norm);
+  });
+}
+
+template <class T>
+__global__ void __launch_bounds__(kBlock, kDualCtasPerSm) dual_step_kernel(DualArgs<T> a) {
+  __shared__ DualShared<T> sm;
+  __shared__ union {   // the tiles are done with when the sums begin (cta_sums' first barrier)
+    Tile tl[kTilesPerCtaMax];
+    double red[3 * kBlock];
+  } ph;
+  Tile* const tl = ph.tl;
+  double* const red = ph.red;
+  __shared__ int is_last;
+  __shared__ double tot[3];
+  const int b = a.plan.cta_map ? a.plan.cta_map[blockIdx.x] : (int)blockIdx.x;
+  pdl_launch_dependents();  // the next primal kernel reads the state only after its wait
+  const int nt = stage_tiles(a.plan.tiles, a.plan.cta_tile_begin[b], a.plan.cta_tile_begin[b + 1], tl);
+  // The state this kernel reads was written by the previous dual kernel, which completed
+  // before the primal kernel let this one launch (see there): read it now, from L2 (a line in
+  // this SM's L1 may predate it), so the loads overlap the primal kernel's last CTAs.
+  const StepState* st = a.st_mut + a.plan.cta_inst[b];
+  const int done = __ldcg(&st->done);
+  const int pending = __ldcg(&st->pending_commit);
+  const int p = __ldcg(&st->parity);
+  const double commit_weight = __ldcg(&st->commit_weight);
+  const double od64 = __ldcg(&st->omega) * __ldcg(&st->tau);  // primal_weight * step_size
+  __shared__ double factors[2];   // the decision's, loaded while the primal kernel ends
+  if (threadIdx.x == 0) step_factors(st, factors);
+  pdl_wait();
+  if (done) return;
+  const DualScalars<T> sc{pending != 0, (T)commit_weight, (T)od64, p ? a.y1 : a.y0, p ? a.y0 : a.y1,
+                          p ? a.kx1 : a.kx0, p ? a.kx0 : a.kx1};
+  T acc_i = T(0), acc_d = T(0);
+  dual_work(a, sc, sm, tl, nt, acc_i, acc_d);
+  const int inst = a.plan.cta_inst[b];
+  const int c0 = a.plan.inst_cta_begin[inst], c1 = a.plan.inst_cta_begin[inst + 1];
+  StepState* stw = a.st_mut + inst;
+  const T v[2] = {acc_i, acc_d};
+  cta_sums<2>(v, tot, red);
+  if (threadIdx.x == 0) {
+    a.part_d[b] = tot[0];
+    a.part_d[a.plan.num_ctas + b] = tot[1];
+    __threadfence();
+    const unsigned prev = atomicAdd(&stw->arrive, 1u);
+    is_last = (prev == (unsigned)(c1 - c0 - 1)) ? 1 : 0;
+  }
+  __syncthreads();
+  if (!is_last) return;
+  // The instance's last CTA: the state into shared memory from L2, one 8-byte word per thread, and
+  // all CTAs' sums, in one round of loads (the barriers of cta_sums order the copy before its
+  // use); then thread 0 takes the decision. This tail is on every attempt's path: with the primal
+  // sum and the decision's inputs formed by the instance's first CTA after its own work (4,600
+  // cycles), sums by one warp (3,600) and the decision on the shared copy (2,600) it took twice as long.
+  __shared__ StepState s;
+  load_state(stw, s);
+  step_totals(a, inst, s, tot, red);
   if (threadIdx.x == 0) {
     s.arrive = 0;
     if (pending) s.primal_spmv += 1;
-    s.pending_commit = 0;
-    step_decision(s, s.f1, s.f2, tot[0], s.half_w_dx2, s.half_over_omega, tot[1]);
+    step_decision(s, factors[0], factors[1], tot[0], __fma_rn(__dmul_rn(s.half_over_omega, tot[1]), tot[1], tot[2]));
+    s.tto = s.tau / s.omega;
   }
   __syncthreads();
-  // the new state back to global memory, one 8-byte word per thread
-  if (threadIdx.x < sizeof(StepState) / 8)
-    reinterpret_cast<unsigned long long*>(stw)[threadIdx.x] = reinterpret_cast<const unsigned long long*>(&s)[threadIdx.x];
+  store_state(s, stw);
 }
 
 // Launches a step kernel with programmatic dependent launch enabled (see pdl_wait).
