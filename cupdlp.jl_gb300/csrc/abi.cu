@@ -140,7 +140,6 @@ gpdhg_status gpdhg_solve(gpdhg_problem* p, const gpdhg_params* params, gpdhg_res
     if (!p || !result) throw gpdhg::Error(GPDHG_ERR_INVALID_ARGUMENT, "problem or result is NULL");
     check_params(params);
     gpdhg::solve(p, *params, result, primal_out, dual_out);
-    gpdhg::to_caller_columns(p->col_perm, primal_out);
   });
 }
 

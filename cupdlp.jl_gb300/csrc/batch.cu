@@ -322,6 +322,11 @@ struct BatchWorkspace {
   PinnedBuf<uint8_t> flags_host;
   cudaGraphExec_t graphs[kBatchLevels] = {};
   long long launches = 0;
+  DBuf<double> caller;   // solutions in FP64, on their way to the host
+  double* caller_buffer() {
+    if (!caller.get()) caller.alloc((size_t)std::max(std::max(N, M), 1));
+    return caller.get();
+  }
   DBuf<double> pow_table;
   double pow_r = -1.0, pow_g = -1.0;
   const int direct = sizeof(T) == sizeof(float) ? 1 : 0;
@@ -544,6 +549,18 @@ static void run_batch(gpdhg_batch* B, BatchWorkspace<T>& W, const gpdhg_params& 
   const auto t0 = Clock::now();
   auto elapsed = [&]() { return std::chrono::duration<double>(Clock::now() - t0).count(); };
   uint8_t* fh = W.flags_host.p;
+  // entries [off, off + len) of a packed solution to the caller's array (FP32 widened on the device)
+  auto fetch_slice = [&](const T* dsrc, double* hdst, int off, int len) {
+    if (!hdst || len == 0) return;
+    const double* src = reinterpret_cast<const double*>(dsrc) + off;
+    if constexpr (sizeof(T) == 4) {
+      caller_values_kernel<T><<<W.grid(len), kBlock, 0, s>>>(len, dsrc + off, nullptr, W.caller_buffer() + off);
+      CK_LAUNCH();
+      ++W.launches;
+      src = W.caller_buffer() + off;
+    }
+    CK(cudaMemcpyAsync(hdst, src, sizeof(double) * len, cudaMemcpyDeviceToHost, s));
+  };
   int alive = K;
   long long rounds = 0;
   while (alive > 0) {
@@ -585,6 +602,7 @@ static void run_batch(gpdhg_batch* B, BatchWorkspace<T>& W, const gpdhg_params& 
       W.finish_reductions();
       bool any_restart = false;
       std::vector<uint8_t> ta(K, 0), rs(K, 0);
+      std::vector<int> ended;   // instances terminated in this round: their solutions are on their way to the caller
       for (int k = 0; k < K; ++k) {
         if (!fh[k]) continue;
         st[k].pending_commit = 0;
@@ -624,22 +642,14 @@ static void run_batch(gpdhg_batch* B, BatchWorkspace<T>& W, const gpdhg_params& 
           r.accepted_steps = st[k].accepted;
           r.rejected_steps = st[k].rejected;
           r.primal_spmv_launches = st[k].primal_spmv;
-          auto fetch_slice = [&](const T* dsrc, double* hdst, int off, int len) {
-            if (!hdst || len == 0) return;
-            std::vector<T> tmp(len);
-            CK(cudaMemcpyAsync(tmp.data(), dsrc + off, sizeof(T) * len, cudaMemcpyDeviceToHost, s));
-            CK(cudaStreamSynchronize(s));
-            for (int q = 0; q < len; ++q) hdst[q] = (double)tmp[q];
-          };
           fetch_slice(W.ax.get(), primal_out ? primal_out[k] : nullptr, B->col_off[k], B->col_off[k + 1] - B->col_off[k]);
-          if (primal_out) to_caller_columns(B->col_perm[k], primal_out[k]);
           fetch_slice(W.ay.get(), dual_out ? dual_out[k] : nullptr, B->row_off[k], B->row_off[k + 1] - B->row_off[k]);
           retired[k] = 1;
           fh[k] = 0;
           st[k].done = 1;
           --alive;
           r.kernels_launched = W.launches - launches0;
-          if (on_retire) (*on_retire)(k);
+          ended.push_back(k);
           continue;
         }
         // run_restart_scheme for the instances that have an average
@@ -654,6 +664,13 @@ static void run_batch(gpdhg_batch* B, BatchWorkspace<T>& W, const gpdhg_params& 
         st[k].sum_w_primal = st[k].sum_w_dual = 0.0;
         st[k].omega = dec.new_omega;
         any_restart = true;
+      }
+      if (!ended.empty()) {
+        CK(cudaStreamSynchronize(s));
+        for (int k : ended) {
+          if (primal_out) to_caller_columns(B->col_perm[k], primal_out[k]);
+          if (on_retire) (*on_retire)(k);
+        }
       }
       if (any_restart) {
         for (int k = 0; k < K; ++k) {

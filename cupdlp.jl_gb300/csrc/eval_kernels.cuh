@@ -414,4 +414,13 @@ __global__ void convert_kernel(long long len, const S* src, D* dst) {
     dst[i] = (D)src[i];
 }
 
+// A solution as the caller reads it: FP64, entry k at the caller's position perm[k] (NULL: k). On
+// the host, widening and permuting 2M columns took 3 ms of a solve's end.
+template <class T>
+__global__ void caller_values_kernel(int len, const T* __restrict__ src, const int32_t* __restrict__ perm,
+                                     double* __restrict__ dst) {
+  for (int k = blockIdx.x * blockDim.x + threadIdx.x; k < len; k += gridDim.x * blockDim.x)
+    dst[perm ? perm[k] : k] = (double)src[k];
+}
+
 }  // namespace gpdhg

@@ -647,6 +647,7 @@ void apply_column_order(gpdhg_problem* p) {
   p->norm2_c_scaled = norm2(hc.data(), n);
   p->l2_c = norm2(hoc.data(), n);
   p->col_perm.swap(perm);
+  p->col_perm_dev = std::move(dperm);
   tr.mark("  order: norms");
 }
 

@@ -160,6 +160,7 @@ struct gpdhg_problem {
   // column order inside the handle (column_order): handle column k is the caller's column
   // col_perm[k]; empty when the handle keeps the caller's order
   std::vector<int32_t> col_perm;
+  gpdhg::DBuf<int32_t> col_perm_dev;    // the same on the device
   ~gpdhg_problem();
 };
 
@@ -170,7 +171,7 @@ namespace gpdhg {
 void validate_lp_desc(const gpdhg_lp_desc* d, bool threads);
 // Builds the device problem from a descriptor (throws gpdhg::Error).
 void problem_init(gpdhg_problem* p, const gpdhg_lp_desc* d);
-// The solve loop (solver.cu); primal_out in the handle's column order.
+// The solve loop (solver.cu); primal_out in the caller's column order.
 void solve(gpdhg_problem* P, const gpdhg_params& prm, gpdhg_result* res, double* primal_out, double* dual_out);
 // The same from the matrix in compressed sparse columns (index base 0 or 1, int64 indices, as
 // Julia's SparseMatrixCSC): CSC(A) is uploaded as CSR(A') and A is built on the device.

@@ -96,6 +96,7 @@ double footprint_bytes(const gpdhg_lp_desc& d, const gpdhg_params& p) {
   bytes += plans * 2.0 * z * (t + 4.0) * 1.5;              // lane-interleaved tile copies
   bytes += 8.0 * (7.0 * n + 3.0 * m) + m + 4.0 * (n + m);  // FP64 vectors, flags, instance maps
   bytes += t * (13.0 * n + 11.0 * m);                      // workspace iterates
+  if (!fp64) bytes += 8.0 * (n + m);                       // the widened solution
   if (refine) bytes += 8.0 * (13.0 * n + 11.0 * m);        // the FP64 phase's workspace
   return 1.1 * bytes + (1 << 20);
 }
@@ -326,7 +327,6 @@ class Server {
         p = new gpdhg_problem();
         problem_init(p, &r.lp.d);
         gpdhg::solve(p, r.params, &result, r.x.data(), r.y.empty() ? nullptr : r.y.data());
-        to_caller_columns(p->col_perm, r.x.data());
       } catch (const Error& e) {
         status = e.status;
         error = e.what();

@@ -130,6 +130,11 @@ struct Workspace {
   cudaGraphExec_t graphs[kGraphLevels] = {};
   // profiled variants: an event between every pair of kernels
   std::vector<cudaEvent_t> pev;   // per-kernel timing events (params.profile_kernels)
+  DBuf<double> caller;   // a solution in FP64 and the caller's order, on its way to the host
+  double* caller_buffer() {
+    if (!caller.get()) caller.alloc((size_t)std::max(n, m));
+    return caller.get();
+  }
   DBuf<double> pow_table;
   double pow_r = -1.0, pow_g = -1.0;
   const int direct = sizeof(T) == sizeof(float) ? 1 : 0;
@@ -453,19 +458,19 @@ bool run_phase(gpdhg_problem* P, Workspace<T>& W, const gpdhg_params& prm, LoopS
       }
       if (reason != 0) {
         // copy the scaled average to the host (:713-720)
-        auto fetch = [&](const T* dsrc, double* hdst, int len) {
+        auto fetch = [&](const T* dsrc, const int32_t* perm, double* hdst, int len) {
           if (!hdst || len == 0) return;
-          if constexpr (sizeof(T) == sizeof(double)) {
-            CK(cudaMemcpyAsync(hdst, dsrc, sizeof(double) * len, cudaMemcpyDeviceToHost, s));
-          } else {
-            std::vector<float> tmp(len);
-            CK(cudaMemcpyAsync(tmp.data(), dsrc, sizeof(float) * len, cudaMemcpyDeviceToHost, s));
-            CK(cudaStreamSynchronize(s));
-            for (int k = 0; k < len; ++k) hdst[k] = tmp[k];
+          const double* src = reinterpret_cast<const double*>(dsrc);
+          if (sizeof(T) == 4 || perm) {
+            caller_values_kernel<T><<<W.grid_for(len), kBlock, 0, s>>>(len, dsrc, perm, W.caller_buffer());
+            CK_LAUNCH();
+            ++P->launches;
+            src = W.caller_buffer();
           }
+          CK(cudaMemcpyAsync(hdst, src, sizeof(double) * len, cudaMemcpyDeviceToHost, s));
         };
-        fetch(W.ax.get(), primal_out, n);
-        fetch(W.ay.get(), dual_out, m);
+        fetch(W.ax.get(), P->col_perm_dev.get(), primal_out, n);
+        fetch(W.ay.get(), nullptr, dual_out, m);
         CK(cudaStreamSynchronize(s));
         std::memset(res, 0, sizeof(*res));
         res->termination_reason = reason;
