@@ -318,9 +318,7 @@ struct BatchWorkspace {
   // launched CTAs: those of instances not yet retired (rebuilt when their count halves)
   DBuf<int32_t> map_p, map_d;
   int grid_p = 0, grid_d = 0;
-  DBuf<uint8_t> flags;             // 3 x count: evaluated, to_avg, restart
-  PinnedBuf<uint8_t> flags_host;
-  cudaGraphExec_t graphs[kBatchLevels] = {};
+  cudaGraphExec_t graphs[kBatchLevels] = {}, evaluation = nullptr;
   long long launches = 0;
   DBuf<double> caller;   // solutions in FP64, on their way to the host
   double* caller_buffer() {
@@ -343,8 +341,7 @@ struct BatchWorkspace {
   }
 
   explicit BatchWorkspace(gpdhg_batch* b_) : B(b_), count(b_->count), N(b_->N), M(b_->M),
-                                             st_host(b_->count), red_host((size_t)b_->count * kEvalStride),
-                                             flags_host(3 * (size_t)b_->count) {
+                                             st_host(b_->count), red_host((size_t)b_->count * kEvalStride) {
     PhaseTrace tr;
     cudaStream_t s = B->stream;
     if constexpr (sizeof(T) == sizeof(double)) {
@@ -387,13 +384,13 @@ struct BatchWorkspace {
     red_part_n.alloc((size_t)kPassNQ * B->nseg_n);
     red_part_m.alloc((size_t)kPassMQ * B->nseg_m);
     red_out.alloc((size_t)count * kEvalStride);
-    flags.alloc(3 * (size_t)count);
     compact(std::vector<char>(count, 0));
     tr.mark("batch ws: CTA maps, graphs");
   }
   ~BatchWorkspace() {
     for (cudaGraphExec_t g : graphs)
       if (g) cudaGraphExecDestroy(g);
+    if (evaluation) cudaGraphExecDestroy(evaluation);
   }
   TileView<T> view_p() const {
     TileView<T> v = plan_p.view();
@@ -443,6 +440,9 @@ struct BatchWorkspace {
       g = nullptr;
     }
     for (int lv = 0; lv < kBatchLevels; ++lv) graphs[lv] = capture(1 << lv);
+    if (evaluation) cudaGraphExecDestroy(evaluation);
+    evaluation = nullptr;
+    evaluation = capture_evaluation();
   }
   PrimalArgs<T> pargs(int mode) {
     return PrimalArgs<T>{B->At.view<T>(), view_p(), c, l, u, x.get(), dx.get(), kty.get(), sx.get(),
@@ -468,19 +468,10 @@ struct BatchWorkspace {
     cudaGraphDestroy(g);
     return ex;
   }
+  // the host edits the mirror only after synchronising with the work that follows
   void push_state() {
     CK(cudaMemcpyAsync(st_dev.get(), st_host.p, sizeof(StepState) * count, cudaMemcpyHostToDevice, B->stream));
-    CK(cudaStreamSynchronize(B->stream));
   }
-  void push_flags() {
-    CK(cudaMemcpyAsync(flags.get(), flags_host.p, 3 * (size_t)count, cudaMemcpyHostToDevice, B->stream));
-    CK(cudaStreamSynchronize(B->stream));
-  }
-  uint8_t* active() { return flags.get(); }
-  uint8_t* to_avg() { return flags.get() + count; }
-  uint8_t* restart() { return flags.get() + 2 * count; }
-  BatchVecArgs<T> vn(const uint8_t* flag) const { return BatchVecArgs<T>{B->col_inst.get(), flag, st_dev.get(), N}; }
-  BatchVecArgs<T> vm(const uint8_t* flag) const { return BatchVecArgs<T>{B->row_inst.get(), flag, st_dev.get(), M}; }
   int grid(int len) const { return std::max(1, std::min(ceil_div(len, kBlock), 4096)); }
 
   // one side's pass over the segments of the evaluated instances (StepState::eval_active)
@@ -490,17 +481,54 @@ struct BatchWorkspace {
     seg_reduce_kernel<Q, MAXMASK, F><<<nit, kBlock, 0, B->stream>>>(
         n_side ? B->seg_n.get() : B->seg_m.get(), st_dev.get(), f, n_side ? red_part_n.get() : red_part_m.get(), nit);
     CK_LAUNCH();
-    ++launches;
   }
-  void finish_reductions() {
-    const SegSide m{B->seg_m_begin.get(), red_part_m.get(), red_out.get(), B->nseg_m, kPassMQ, kEvalMMax};
-    const SegSide n{B->seg_n_begin.get(), red_part_n.get(), red_out.get() + kEvalOutN, B->nseg_n, kPassNQ, kEvalNMax};
-    seg_finalize_kernel<<<dim3(kPassMQ + kPassNQ, count), kBlock, 0, B->stream>>>(m, n, st_dev.get());
+  // One evaluation of the instances marked in the state, as the lone solve's graph: the state, the
+  // pending steps' column side beside the row pass and A' y-bar, the column pass, one read-back.
+  static constexpr int kEvaluationKernels = 5;
+  cudaGraphExec_t capture_evaluation() {
+    cudaStream_t s = B->stream;
+    cudaStream_t side_stream = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
+    CK(cudaStreamCreateWithFlags(&side_stream, cudaStreamNonBlocking));
+    CK(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
+    CK(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
+    CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+    CK(cudaMemcpyAsync(st_dev.get(), st_host.p, sizeof(StepState) * count, cudaMemcpyHostToDevice, s));
+    CK(cudaEventRecord(fork, s));
+    CK(cudaStreamWaitEvent(side_stream, fork, 0));
+    primal_step_kernel<T><<<grid_p, kBlock, 0, side_stream>>>(pargs(kStepCommitOnly));
+    CK(cudaEventRecord(join, side_stream));
+    seg_reduce<kPassMQ, kEvalMMax>(
+        false, EvalPassM<T>{B->con.get(), rcon.get(), B->ob.get(), b, y0.get(), y1.get(), kx0.get(), kx1.get(),
+                            ry.get(), rkx.get(), sy.get(), skx.get(), ay.get(), akx.get(), 0, B->ineq_flag.get()});
+    if (B->At.num_items > 0)
+      spmv_kernel<T><<<B->At.num_items, kBlock, 0, s>>>(B->At.view<T>(), ay.get(), aty.get(), B->col_inst.get(),
+                                                        st_dev.get());
+    CK(cudaStreamWaitEvent(s, join, 0));
+    seg_reduce<kPassNQ, kEvalNMax>(
+        true, EvalPassN<T>{B->var.get(), rvar.get(), B->ol.get(), B->ou.get(), B->oc.get(), l, u, c, x.get(), sx.get(),
+                           aty.get(), kty.get(), rx.get(), rgrad.get(), ax.get(), agrad.get(), grad.get()});
+    const SegSide sm{B->seg_m_begin.get(), red_part_m.get(), red_out.get(), B->nseg_m, kPassMQ, kEvalMMax};
+    const SegSide sn{B->seg_n_begin.get(), red_part_n.get(), red_out.get() + kEvalOutN, B->nseg_n, kPassNQ, kEvalNMax};
+    seg_finalize_kernel<<<dim3(kPassMQ + kPassNQ, count), kBlock, 0, s>>>(sm, sn, st_dev.get());
+    CK(cudaMemcpyAsync(red_host.p, red_out.get(), sizeof(double) * kEvalStride * count, cudaMemcpyDeviceToHost, s));
+    cudaGraph_t g = nullptr;
+    CK(cudaStreamEndCapture(s, &g));
+    cudaGraphExec_t ex = nullptr;
+    CK(cudaGraphInstantiate(&ex, g, 0));
+    cudaGraphDestroy(g);
+    cudaEventDestroy(fork);
+    cudaEventDestroy(join);
+    cudaStreamDestroy(side_stream);
+    return ex;
+  }
+  void launch_restart() {
+    const RestartArgs<T> a{st_dev.get(), B->col_inst.get(), B->row_inst.get(), N, M, c, ax.get(), agrad.get(),
+                           ay.get(), akx.get(), x.get(), kty.get(), grad.get(), sx.get(), rx.get(), rgrad.get(),
+                           y0.get(), y1.get(), kx0.get(), kx1.get(), sy.get(), skx.get(), ry.get(), rkx.get()};
+    restart_kernel<T><<<grid(std::max(N, M)), kBlock, 0, B->stream>>>(a);
     CK_LAUNCH();
     ++launches;
-    CK(cudaMemcpyAsync(red_host.p, red_out.get(), sizeof(double) * kEvalStride * count, cudaMemcpyDeviceToHost,
-                       B->stream));
-    CK(cudaStreamSynchronize(B->stream));
   }
 };
 
@@ -510,7 +538,7 @@ static void run_batch(gpdhg_batch* B, BatchWorkspace<T>& W, const gpdhg_params& 
                       const std::function<void(int)>* on_retire) {
   cudaStream_t s = B->stream;
   const int K = B->count;
-  const int N = B->N, M = B->M;
+  const int N = B->N;
   const long long freq = std::max(1, prm.termination_evaluation_frequency);
   const long long it_limit = prm.iteration_limit;
   const long long launches0 = W.launches;
@@ -545,10 +573,8 @@ static void run_batch(gpdhg_batch* B, BatchWorkspace<T>& W, const gpdhg_params& 
     q.iter_start_tau = q.tau;
     q.done = 1;
   }
-  W.push_state();
   const auto t0 = Clock::now();
   auto elapsed = [&]() { return std::chrono::duration<double>(Clock::now() - t0).count(); };
-  uint8_t* fh = W.flags_host.p;
   // entries [off, off + len) of a packed solution to the caller's array (FP32 widened on the device)
   auto fetch_slice = [&](const T* dsrc, double* hdst, int off, int len) {
     if (!hdst || len == 0) return;
@@ -565,14 +591,13 @@ static void run_batch(gpdhg_batch* B, BatchWorkspace<T>& W, const gpdhg_params& 
   long long rounds = 0;
   while (alive > 0) {
     // ---- evaluate every instance that reached its evaluation point ----
-    std::memset(fh, 0, 3 * (size_t)K);
-    bool any = false;
+    bool any = false, any_restart = false;
     for (int k = 0; k < K; ++k) {
       StepState& q = st[k];
+      q.restart = kNoRestart;
       q.eval_active = !retired[k] && due[k] ? 1 : 0;
       q.done = q.eval_active ? 0 : 1;  // not being evaluated: keep its kernels idle
       if (!q.eval_active) continue;
-      fh[k] = 1;
       q.eval_current = (q.numerical_error || q.count_primal == 0 || q.count_dual == 0) ? 1 : 0;
       q.eval_restart = restart_kkt[k].valid ? 0 : 1;
       q.rcp_w_primal = q.eval_current ? 0.0 : 1.0 / q.sum_w_primal;
@@ -581,30 +606,12 @@ static void run_batch(gpdhg_batch* B, BatchWorkspace<T>& W, const gpdhg_params& 
       any = true;
     }
     if (any) {
-      W.push_state();
-      W.push_flags();
-      // as the lone solve: the pending step's column side, the row pass, A' y-bar, the column pass
-      launch_step(primal_step_kernel<T>, W.grid_p, s, W.pargs(kStepCommitOnly));
-      W.template seg_reduce<kPassMQ, kEvalMMax>(
-          false, EvalPassM<T>{B->con.get(), W.rcon.get(), B->ob.get(), W.b, W.y0.get(), W.y1.get(), W.kx0.get(),
-                              W.kx1.get(), W.ry.get(), W.rkx.get(), W.sy.get(), W.skx.get(), W.ay.get(), W.akx.get(), 0,
-                              B->ineq_flag.get()});
-      if (B->At.num_items > 0) {
-        spmv_kernel<T><<<B->At.num_items, kBlock, 0, s>>>(B->At.view<T>(), W.ay.get(), W.aty.get(), B->col_inst.get(),
-                                                          W.active());
-        CK_LAUNCH();
-      }
-      W.launches += 2;
-      W.template seg_reduce<kPassNQ, kEvalNMax>(
-          true, EvalPassN<T>{B->var.get(), W.rvar.get(), B->ol.get(), B->ou.get(), B->oc.get(), W.l, W.u, W.c,
-                             W.x.get(), W.sx.get(), W.aty.get(), W.kty.get(), W.rx.get(), W.rgrad.get(), W.ax.get(),
-                             W.agrad.get(), W.grad.get()});
-      W.finish_reductions();
-      bool any_restart = false;
-      std::vector<uint8_t> ta(K, 0), rs(K, 0);
+      CK(cudaGraphLaunch(W.evaluation, s));
+      W.launches += W.kEvaluationKernels;
+      CK(cudaStreamSynchronize(s));
       std::vector<int> ended;   // instances terminated in this round: their solutions are on their way to the caller
       for (int k = 0; k < K; ++k) {
-        if (!fh[k]) continue;
+        if (!st[k].eval_active) continue;
         st[k].pending_commit = 0;
         const double* em = W.red_host.p + (size_t)kEvalStride * k;
         const double* en = em + kEvalOutN;
@@ -645,7 +652,6 @@ static void run_batch(gpdhg_batch* B, BatchWorkspace<T>& W, const gpdhg_params& 
           fetch_slice(W.ax.get(), primal_out ? primal_out[k] : nullptr, B->col_off[k], B->col_off[k + 1] - B->col_off[k]);
           fetch_slice(W.ay.get(), dual_out ? dual_out[k] : nullptr, B->row_off[k], B->row_off[k + 1] - B->row_off[k]);
           retired[k] = 1;
-          fh[k] = 0;
           st[k].done = 1;
           --alive;
           r.kernels_launched = W.launches - launches0;
@@ -657,8 +663,7 @@ static void run_batch(gpdhg_batch* B, BatchWorkspace<T>& W, const gpdhg_params& 
         const RestartDecision dec =
             decide_restart(prm, B->info[k], st[k].count_primal, st[k].tau, st[k].omega, iteration[k] - 1, kn, km, mem[k]);
         if (dec.restart_used == GPDHG_RESTART_CHOICE_NO_RESTART) continue;
-        rs[k] = 1;
-        ta[k] = dec.reset_to_average ? 1 : 0;
+        st[k].restart = dec.reset_to_average ? kRestartToAverage : kRestartFromCurrent;
         restart_kkt[k].valid = false;
         st[k].count_primal = st[k].count_dual = 0;
         st[k].sum_w_primal = st[k].sum_w_dual = 0.0;
@@ -671,26 +676,6 @@ static void run_batch(gpdhg_batch* B, BatchWorkspace<T>& W, const gpdhg_params& 
           if (primal_out) to_caller_columns(B->col_perm[k], primal_out[k]);
           if (on_retire) (*on_retire)(k);
         }
-      }
-      if (any_restart) {
-        for (int k = 0; k < K; ++k) {
-          fh[k] = rs[k];
-          fh[K + k] = ta[k];
-        }
-        W.push_flags();
-        W.push_state();  // restart kernels read each instance's parity
-        batch_restart_n_kernel<T><<<W.grid(N), kBlock, 0, s>>>(W.vn(W.active()), W.to_avg(), W.ax.get(),
-                                                               W.agrad.get(), W.c, W.x.get(), W.kty.get(),
-                                                               W.grad.get(), W.sx.get(), W.rx.get(), W.rgrad.get());
-        CK_LAUNCH();
-        if (M) {
-          batch_restart_m_kernel<T><<<W.grid(M), kBlock, 0, s>>>(W.vm(W.active()), W.to_avg(), W.ay.get(),
-                                                                 W.akx.get(), W.y0.get(), W.y1.get(), W.kx0.get(),
-                                                                 W.kx1.get(), W.sy.get(), W.skx.get(), W.ry.get(),
-                                                                 W.rkx.get());
-          CK_LAUNCH();
-        }
-        W.launches += 2;
       }
       // re-arm: take_step! calls until each instance's next evaluation
       for (int k = 0; k < K; ++k) {
@@ -713,13 +698,17 @@ static void run_batch(gpdhg_batch* B, BatchWorkspace<T>& W, const gpdhg_params& 
     if (2 * W.active_ctas(retired) < W.grid_p) W.compact(retired);
     // ---- step graphs until every running instance reached its evaluation point ----
     W.push_state();
+    if (any_restart) W.launch_restart();
     const auto tb = Clock::now();
     long long graph_launches = 0;
     while (true) {
       int max_remaining = 0;
       for (int k = 0; k < K; ++k)
         if (!retired[k] && !st[k].done) max_remaining = std::max(max_remaining, st[k].target_in_chunk - st[k].accepted_in_chunk);
-      if (max_remaining == 0) break;
+      if (max_remaining == 0) {
+        CK(cudaStreamSynchronize(s));   // the state's copy has left the mirror
+        break;
+      }
       int lv = 0;
       while (lv + 1 < kBatchLevels && (1 << lv) < max_remaining) ++lv;
       CK(cudaGraphLaunch(W.graphs[lv], s));

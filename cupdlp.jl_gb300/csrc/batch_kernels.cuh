@@ -71,51 +71,56 @@ static __global__ void __launch_bounds__(kBlock) seg_finalize_kernel(SegSide a, 
   if (threadIdx.x == 0) s.out[(size_t)inst * kEvalStride + q] = r;
 }
 
-// Per-element helpers driven by per-instance flags / weights.
+// ---- restart ----------------------------------------------------------------------
+// Restart actions (src/saddle_point_gpu.jl:575-614) of the instances whose StepState::restart is set
+// (kRestartToAverage: the average becomes the current point): the averaging sums are cleared and
+// the restart point is stored. Elements [0, n) are columns, the rest rows; inst_of NULL: one
+// instance. (As up to eleven copies and fills, a restart was mostly launches.)
+enum RestartMode : int { kNoRestart = 0, kRestartFromCurrent = 1, kRestartToAverage = 2 };
 template <class T>
-struct BatchVecArgs {
-  const int32_t* inst_of;   // instance of each element
-  const uint8_t* flag;      // per-instance selector
+struct RestartArgs {
   const StepState* st;
-  int len;
+  const int32_t* col_inst;
+  const int32_t* row_inst;
+  int n, m;
+  const T *c, *ax, *agrad, *ay, *akx;
+  T *x, *kty, *grad, *sx, *rx, *rgrad;
+  T *y0, *y1, *kx0, *kx1, *sy, *skx, *ry, *rkx;
 };
-
-// Restart actions (src/saddle_point_gpu.jl:575-614) for the instances with flag set:
-// to_avg[k] selects reset-to-average; sums are cleared; the restart point is stored.
 template <class T>
-__global__ void batch_restart_n_kernel(BatchVecArgs<T> v, const uint8_t* to_avg, const T* ax, const T* agrad,
-                                       const T* c, T* x, T* kty, T* grad, T* sx, T* rx, T* rgrad) {
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < v.len; j += gridDim.x * blockDim.x) {
-    const int k = v.inst_of[j];
-    if (!v.flag[k]) continue;
-    if (to_avg[k]) {
-      x[j] = ax[j];
-      kty[j] = c[j] - agrad[j];
-      grad[j] = agrad[j];
+__global__ void __launch_bounds__(kBlock) restart_kernel(RestartArgs<T> a) {
+  const int stride = gridDim.x * blockDim.x;
+  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < a.n; j += stride) {
+    const int mode = a.st[a.col_inst ? a.col_inst[j] : 0].restart;
+    if (mode == kNoRestart) continue;
+    T x = a.x[j], g = a.grad[j];
+    if (mode == kRestartToAverage) {
+      x = a.ax[j];
+      g = a.agrad[j];
+      a.x[j] = x;
+      a.kty[j] = a.c[j] - g;
+      a.grad[j] = g;
     }
-    sx[j] = T(0);
-    rx[j] = x[j];
-    rgrad[j] = grad[j];
+    a.sx[j] = T(0);
+    a.rx[j] = x;
+    a.rgrad[j] = g;
   }
-}
-
-template <class T>
-__global__ void batch_restart_m_kernel(BatchVecArgs<T> v, const uint8_t* to_avg, const T* ay, const T* akx, T* y0,
-                                       T* y1, T* kx0, T* kx1, T* sy, T* skx, T* ry, T* rkx) {
-  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < v.len; i += gridDim.x * blockDim.x) {
-    const int k = v.inst_of[i];
-    if (!v.flag[k]) continue;
-    const int p = v.st[k].parity;
-    T* yc = p ? y1 : y0;
-    T* kc = p ? kx1 : kx0;
-    if (to_avg[k]) {
-      yc[i] = ay[i];
-      kc[i] = akx[i];
+  for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < a.m; i += stride) {
+    const StepState& q = a.st[a.row_inst ? a.row_inst[i] : 0];
+    if (q.restart == kNoRestart) continue;
+    T* yc = q.parity ? a.y1 : a.y0;
+    T* kc = q.parity ? a.kx1 : a.kx0;
+    T y = yc[i], k = kc[i];
+    if (q.restart == kRestartToAverage) {
+      y = a.ay[i];
+      k = a.akx[i];
+      yc[i] = y;
+      kc[i] = k;
     }
-    sy[i] = T(0);
-    skx[i] = T(0);
-    ry[i] = yc[i];
-    rkx[i] = kc[i];
+    a.sy[i] = T(0);
+    a.skx[i] = T(0);
+    a.ry[i] = y;
+    a.rkx[i] = k;
   }
 }
 

@@ -119,7 +119,8 @@ struct StepState {
   // instance is evaluated, whether it has no average yet (the current point stands in), and
   // whether the last restart point's KKT ingredients are needed
   double rcp_w_primal, rcp_w_dual;
-  int eval_active, eval_current, eval_restart, pad;
+  int eval_active, eval_current, eval_restart;
+  int restart;             // RestartMode of the restart kernel that follows
 };
 
 // ----------------------------------------------------------------------------------

@@ -398,16 +398,6 @@ __global__ void grad_kernel(int n, const T* c, const T* kty, T* grad) {
   for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) grad[j] = c[j] - kty[j];
 }
 
-// restart to average, src/saddle_point_gpu.jl:579-583
-template <class T>
-__global__ void restart_n_kernel(int n, const T* ax, const T* agrad, const T* c, T* x, T* kty, T* grad) {
-  for (int j = blockIdx.x * blockDim.x + threadIdx.x; j < n; j += gridDim.x * blockDim.x) {
-    x[j] = ax[j];
-    kty[j] = c[j] - agrad[j];
-    grad[j] = agrad[j];
-  }
-}
-
 template <class S, class D>
 __global__ void convert_kernel(long long len, const S* src, D* dst) {
   for (long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x; i < len; i += (long long)gridDim.x * blockDim.x)

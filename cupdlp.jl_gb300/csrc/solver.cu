@@ -127,7 +127,7 @@ struct Workspace {
   DBuf<SegItem> seg_n, seg_m;
   DBuf<int32_t> seg_n_begin, seg_m_begin;
   int nseg_n = 1, nseg_m = 1;
-  cudaGraphExec_t graphs[kGraphLevels] = {};
+  cudaGraphExec_t graphs[kGraphLevels] = {}, evaluation = nullptr;
   // profiled variants: an event between every pair of kernels
   std::vector<cudaEvent_t> pev;   // per-kernel timing events (params.profile_kernels)
   DBuf<double> caller;   // a solution in FP64 and the caller's order, on its way to the host
@@ -225,6 +225,7 @@ struct Workspace {
   ~Workspace() {
     for (cudaGraphExec_t g : graphs)
       if (g) cudaGraphExecDestroy(g);
+    if (evaluation) cudaGraphExecDestroy(evaluation);
     for (cudaEvent_t e : pev) cudaEventDestroy(e);
     if (ev0) cudaEventDestroy(ev0);
     if (ev1) cudaEventDestroy(ev1);
@@ -232,8 +233,6 @@ struct Workspace {
 
   const T* ycur(int parity) const { return parity ? y1.get() : y0.get(); }
   const T* kxcur(int parity) const { return parity ? kx1.get() : kx0.get(); }
-  T* ycur_mut(int parity) { return parity ? y1.get() : y0.get(); }
-  T* kxcur_mut(int parity) { return parity ? kx1.get() : kx0.get(); }
 
   PrimalArgs<T> primal_args(int mode) {
     return PrimalArgs<T>{P->At.view<T>(), plan_p.view(), c, l, u, x.get(), dx.get(), kty.get(), sx.get(),
@@ -265,6 +264,7 @@ struct Workspace {
   }
   void build_graphs() {
     for (int lv = 0; lv < kGraphLevels; ++lv) graphs[lv] = capture(1 << lv);
+    evaluation = capture_evaluation();
   }
   // The same pairs launched directly with an event between every two kernels, for
   // per-kernel CUDA-event timing (events recorded as graph nodes cannot be timed).
@@ -301,7 +301,6 @@ struct Workspace {
     if (M.num_items == 0) return;
     spmv_kernel<T><<<M.num_items, kBlock, 0, P->stream>>>(M.view<T>(), xin, yout, nullptr, nullptr);
     CK_LAUNCH();
-    ++P->launches;
   }
 
   // one side's pass over its segments into its partials
@@ -311,25 +310,74 @@ struct Workspace {
     seg_reduce_kernel<Q, MAXMASK, F><<<nit, kBlock, 0, P->stream>>>(n_side ? seg_n.get() : seg_m.get(), st, f,
                                                                      n_side ? red_part_n.get() : red_part_m.get(), nit);
     CK_LAUNCH();
-    ++P->launches;
   }
   SegSide side(bool n_side, int quantities, unsigned maxmask) {
     return SegSide{n_side ? seg_n_begin.get() : seg_m_begin.get(), n_side ? red_part_n.get() : red_part_m.get(),
                    red_out.get() + (n_side ? kEvalOutN : 0), n_side ? nseg_n : nseg_m, quantities, maxmask};
   }
-  // the partials of both sides reduced (a side without quantities is skipped) and read back
+  // the partials of both sides reduced (a side without quantities is skipped), on their way to red_host
   void finish_reductions(SegSide a, SegSide b, const StepState* st) {
     seg_finalize_kernel<<<dim3(a.quantities + b.quantities, 1), kBlock, 0, P->stream>>>(a, b, st);
     CK_LAUNCH();
-    ++P->launches;
     CK(cudaMemcpyAsync(red_host.p, red_out.get(), sizeof(double) * kEvalStride, cudaMemcpyDeviceToHost, P->stream));
-    CK(cudaStreamSynchronize(P->stream));
+  }
+  // One evaluation as a graph: the state to the device; the accepted step still to be applied (its
+  // K'y, x and Sigma x) beside the row pass (its Sigma y and Sigma Kx, the averages y-bar and Kx-bar
+  // with their unscaled statistics, src/iteration_stats_utils_gpu.jl:447-502, and restart-scheme
+  // ingredients) and A' y-bar (the reference sums the steps' K'y with the averaging weights instead,
+  // src/saddle_point_gpu.jl:176-189; the two agree in exact arithmetic); then the column pass and
+  // one read-back of all sums.
+  static constexpr int kEvaluationKernels = 5;
+  cudaGraphExec_t capture_evaluation() {
+    cudaStream_t s = P->stream;
+    cudaStream_t side_stream = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
+    CK(cudaStreamCreateWithFlags(&side_stream, cudaStreamNonBlocking));
+    CK(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
+    CK(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
+    CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+    CK(cudaMemcpyAsync(st_dev.get(), st_host.p, sizeof(StepState), cudaMemcpyHostToDevice, s));
+    CK(cudaEventRecord(fork, s));
+    CK(cudaStreamWaitEvent(side_stream, fork, 0));
+    primal_step_kernel<T><<<plan_p.num_ctas, kBlock, 0, side_stream>>>(primal_args(kStepCommitOnly));
+    CK(cudaEventRecord(join, side_stream));
+    reduce<kPassMQ, kEvalMMax>(
+        false,
+        EvalPassM<T>{P->con.get(), rcon.get(), P->ob.get(), b, y0.get(), y1.get(), kx0.get(), kx1.get(), ry.get(),
+                     rkx.get(), sy.get(), skx.get(), ay.get(), akx.get(), P->neq, nullptr},
+        st_dev.get());
+    spmv(P->At, ay.get(), tmp_n.get());
+    CK(cudaStreamWaitEvent(s, join, 0));
+    reduce<kPassNQ, kEvalNMax>(
+        true,
+        EvalPassN<T>{P->var.get(), rvar.get(), P->ol.get(), P->ou.get(), P->oc.get(), l, u, c, x.get(), sx.get(),
+                     tmp_n.get(), kty.get(), rx.get(), rgrad.get(), ax.get(), agrad.get(), grad.get()},
+        st_dev.get());
+    finish_reductions(side(false, kPassMQ, kEvalMMax), side(true, kPassNQ, kEvalNMax), st_dev.get());
+    cudaGraph_t g = nullptr;
+    CK(cudaStreamEndCapture(s, &g));
+    cudaGraphExec_t ex = nullptr;
+    CK(cudaGraphInstantiate(&ex, g, 0));
+    cudaGraphDestroy(g);
+    cudaEventDestroy(fork);
+    cudaEventDestroy(join);
+    cudaStreamDestroy(side_stream);
+    return ex;
+  }
+  void launch_restart(cudaStream_t s) {
+    const RestartArgs<T> a{st_dev.get(), nullptr, nullptr, n, m, c, ax.get(), agrad.get(), ay.get(), akx.get(),
+                           x.get(), kty.get(), grad.get(), sx.get(), rx.get(), rgrad.get(), y0.get(), y1.get(),
+                           kx0.get(), kx1.get(), sy.get(), skx.get(), ry.get(), rkx.get()};
+    restart_kernel<T><<<grid_for(std::max(n, m)), kBlock, 0, s>>>(a);
+    CK_LAUNCH();
+    ++P->launches;
   }
 
   double dot(const T* a, const T* b2, long long len) {
     const bool n_side = len == n;
     reduce<1, 0u>(n_side, DotF<T>{a, b2}, nullptr);
     finish_reductions(side(n_side, 1, 0u), SegSide{}, nullptr);
+    CK(cudaStreamSynchronize(P->stream));
     return red_host.p[n_side ? kEvalOutN : 0];
   }
 
@@ -380,7 +428,6 @@ bool run_phase(gpdhg_problem* P, Workspace<T>& W, const gpdhg_params& prm, LoopS
   const long long freq = std::max(1, prm.termination_evaluation_frequency);
   const long long it_limit = prm.iteration_limit;
   const int n = P->n, m = P->m;
-  const int gn = W.grid_for(n), gm = W.grid_for(std::max(m, 1));
   InstanceInfo qi;
   qi.obj_const = P->obj_const;
   qi.linf_c = P->linf_c; qi.linf_b = P->linf_b; qi.l2_c = P->l2_c; qi.l2_b = P->l2_b;
@@ -396,39 +443,16 @@ bool run_phase(gpdhg_problem* P, Workspace<T>& W, const gpdhg_params& prm, LoopS
     if (eval_due(it, freq, it_limit, st.numerical_error != 0)) {
       st.kkt_passes += 2.0;  // KKT_PASSES_PER_TERMINATION_EVALUATION
       st.done = 0;
+      st.restart = kNoRestart;
       // The average, or the current point (src/primal_dual_hybrid_gradient_gpu.jl:635-642)
       st.eval_active = 1;
       st.eval_current = (st.numerical_error || st.count_primal == 0 || st.count_dual == 0) ? 1 : 0;
       st.eval_restart = W.restart_kkt.valid ? 0 : 1;
       st.rcp_w_primal = st.eval_current ? 0.0 : 1.0 / st.sum_w_primal;
       st.rcp_w_dual = st.eval_current ? 0.0 : 1.0 / st.sum_w_dual;
-      push_state_async();
-      // the accepted step still to be applied: its K'y, x and Sigma x here, Sigma y and Sigma Kx
-      // in the row pass
-      if (st.pending_commit) {
-        W.launch_primal(kStepCommitOnly, s);
-        CK_LAUNCH();
-        ++P->launches;
-      }
-      const int p = st.parity;
-      // One pass per side: the row pass forms the averages y-bar and Kx-bar with their unscaled
-      // statistics (src/iteration_stats_utils_gpu.jl:447-502) and restart-scheme ingredients;
-      // then the average's K'y = A' y-bar (the reference sums the steps' K'y with the averaging
-      // weights instead, src/saddle_point_gpu.jl:176-189; the two agree in exact arithmetic)
-      // and the column pass. One read-back for all of them.
-      W.template reduce<kPassMQ, kEvalMMax>(
-          false,
-          EvalPassM<T>{P->con.get(), W.rcon.get(), P->ob.get(), W.b, W.y0.get(), W.y1.get(), W.kx0.get(), W.kx1.get(),
-                       W.ry.get(), W.rkx.get(), W.sy.get(), W.skx.get(), W.ay.get(), W.akx.get(), P->neq, nullptr},
-          W.st_dev.get());
-      if (!st.eval_current) W.spmv(P->At, W.ay.get(), W.tmp_n.get());
-      W.template reduce<kPassNQ, kEvalNMax>(
-          true,
-          EvalPassN<T>{P->var.get(), W.rvar.get(), P->ol.get(), P->ou.get(), P->oc.get(), W.l, W.u, W.c, W.x.get(),
-                       W.sx.get(), W.tmp_n.get(), W.kty.get(), W.rx.get(), W.rgrad.get(), W.ax.get(), W.agrad.get(),
-                       W.grad.get()},
-          W.st_dev.get());
-      W.finish_reductions(W.side(false, kPassMQ, kEvalMMax), W.side(true, kPassNQ, kEvalNMax), W.st_dev.get());
+      CK(cudaGraphLaunch(W.evaluation, s));
+      P->launches += W.kEvaluationKernels;
+      CK(cudaStreamSynchronize(s));
       st.pending_commit = 0;
       const double* em = W.red_host.p;               // kM_*, then the rows' KKT ingredients
       const double* en = W.red_host.p + kEvalOutN;   // kN_*, then the columns'
@@ -516,32 +540,11 @@ bool run_phase(gpdhg_problem* P, Workspace<T>& W, const gpdhg_params& prm, LoopS
         const RestartDecision dec =
             decide_restart(prm, qi, st.count_primal, st.tau, st.omega, it - 1, kn, km, L.restart);
         if (dec.restart_used != GPDHG_RESTART_CHOICE_NO_RESTART) {
-          if (dec.reset_to_average) {
-            restart_n_kernel<T><<<gn, kBlock, 0, s>>>(n, W.ax.get(), W.agrad.get(), W.c, W.x.get(), W.kty.get(),
-                                                      W.grad.get());
-            CK_LAUNCH();
-            ++P->launches;
-            if (m) {
-              CK(cudaMemcpyAsync(W.ycur_mut(p), W.ay.get(), sizeof(T) * m, cudaMemcpyDeviceToDevice, s));
-              CK(cudaMemcpyAsync(W.kxcur_mut(p), W.akx.get(), sizeof(T) * m, cudaMemcpyDeviceToDevice, s));
-            }
-          }
-          W.restart_kkt.valid = false;  // the restart point moves below
-          // reset_solution_weighted_average!
-          CK(cudaMemsetAsync(W.sx.get(), 0, sizeof(T) * n, s));
-          if (m) {
-            CK(cudaMemsetAsync(W.sy.get(), 0, sizeof(T) * m, s));
-            CK(cudaMemsetAsync(W.skx.get(), 0, sizeof(T) * m, s));
-          }
+          // the vectors follow in restart_kernel, after the state that it reads
+          st.restart = dec.reset_to_average ? kRestartToAverage : kRestartFromCurrent;
+          W.restart_kkt.valid = false;  // the restart point moves
           st.count_primal = st.count_dual = 0;
           st.sum_w_primal = st.sum_w_dual = 0.0;
-          // update_last_restart_info!: the restart point becomes the (new) current point
-          CK(cudaMemcpyAsync(W.rx.get(), W.x.get(), sizeof(T) * n, cudaMemcpyDeviceToDevice, s));
-          CK(cudaMemcpyAsync(W.rgrad.get(), W.grad.get(), sizeof(T) * n, cudaMemcpyDeviceToDevice, s));
-          if (m) {
-            CK(cudaMemcpyAsync(W.ry.get(), W.ycur(p), sizeof(T) * m, cudaMemcpyDeviceToDevice, s));
-            CK(cudaMemcpyAsync(W.rkx.get(), W.kxcur(p), sizeof(T) * m, cudaMemcpyDeviceToDevice, s));
-          }
           st.omega = dec.new_omega;
           restart_used = dec.restart_used;
         }
@@ -561,6 +564,7 @@ bool run_phase(gpdhg_problem* P, Workspace<T>& W, const gpdhg_params& prm, LoopS
     st.tto = st.tau / st.omega;
     st.arrive = 0;
     push_state_async();
+    if (st.restart != kNoRestart) W.launch_restart(s);
     const auto tb = Clock::now();
     long long launches = 0;
     const bool prof = prm.profile_kernels != 0;
