@@ -592,42 +592,44 @@ __device__ __forceinline__ void store_state(const StepState& s, StepState* st) {
     reinterpret_cast<unsigned long long*>(st)[threadIdx.x] = reinterpret_cast<const unsigned long long*>(&s)[threadIdx.x];
 }
 
+// Plan ranges of an instance: first and end CTA and split row of the dual plan, then of the primal plan.
+struct PlanRanges {
+  int c0, c1, s0, s1, p0, p1, q0, q1;
+};
+
 // What the step decision needs of the instance's sums, in tot (shared): the interaction, ||dy|| and
 // 0.5 omega ||dx|| ||dx|| (the primal part of take_step!'s movement, :324-333, evaluated as the
 // reference does, the norm squared again). One round of loads for the CTAs' sums of both kernels
 // up to 4 x kBlock CTAs, all issued before any is added; split-row slots (rare) follow. The roots
 // (580 cycles each) are taken side by side, each by the warp that has its sum.
 template <class T>
-__device__ __forceinline__ void step_totals(const DualArgs<T>& a, int inst, const StepState& s, double* tot,
+__device__ __forceinline__ void step_totals(const DualArgs<T>& a, const PlanRanges& g, const StepState& s, double* tot,
                                             double* red) {
-  const int c0 = a.plan.inst_cta_begin[inst], c1 = a.plan.inst_cta_begin[inst + 1];
-  const int s0 = a.plan.inst_split_begin[inst], s1 = a.plan.inst_split_begin[inst + 1];
-  const int p0 = a.p_cta_begin[inst], p1 = a.p_cta_begin[inst + 1];
-  const int q0 = a.p_split_begin[inst], q1 = a.p_split_begin[inst + 1];
   double sd[3] = {0.0, 0.0, 0.0};
-  for (int k0 = (int)threadIdx.x; k0 < max(c1 - c0, p1 - p0); k0 += 4 * kBlock) {
+  const int count = max(g.c1 - g.c0, g.p1 - g.p0);
+  for (int k0 = (int)threadIdx.x; k0 < count; k0 += 4 * kBlock) {
     double ui[4], ud[4], ux[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int k = k0 + j * kBlock;
-      const bool in = k < c1 - c0;
-      ui[j] = in ? __ldcg(a.part_d + c0 + k) : 0.0;
-      ud[j] = in ? __ldcg(a.part_d + a.plan.num_ctas + c0 + k) : 0.0;
-      ux[j] = k < p1 - p0 ? __ldcg(a.part_p + p0 + k) : 0.0;
+      const bool in = k < g.c1 - g.c0;
+      ui[j] = in ? __ldcg(a.part_d + g.c0 + k) : 0.0;
+      ud[j] = in ? __ldcg(a.part_d + a.plan.num_ctas + g.c0 + k) : 0.0;
+      ux[j] = k < g.p1 - g.p0 ? __ldcg(a.part_p + g.p0 + k) : 0.0;
     }
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      if (k0 + j * kBlock >= max(c1 - c0, p1 - p0)) break;
+      if (k0 + j * kBlock >= count) break;
       sd[0] += ui[j];
       sd[1] += ud[j];
       sd[2] += ux[j];
     }
   }
-  for (int k = s0 + (int)threadIdx.x; k < s1; k += kBlock) {
+  for (int k = g.s0 + (int)threadIdx.x; k < g.s1; k += kBlock) {
     sd[0] += __ldcg(a.part_d_split + 2 * k);
     sd[1] += __ldcg(a.part_d_split + 2 * k + 1);
   }
-  for (int k = q0 + (int)threadIdx.x; k < q1; k += kBlock) sd[2] += __ldcg(a.part_p_split + k);
+  for (int k = g.q0 + (int)threadIdx.x; k < g.q1; k += kBlock) sd[2] += __ldcg(a.part_p_split + k);
   cta_sums<3>(sd, tot, red, [&](int q, double sum) {
     if (q == 0) return sum;
     const double norm = sqrt(sum);
@@ -648,27 +650,31 @@ __global__ void __launch_bounds__(kBlock, kDualCtasPerSm) dual_step_kernel(DualA
   __shared__ double tot[3];
   const int b = a.plan.cta_map ? a.plan.cta_map[blockIdx.x] : (int)blockIdx.x;
   pdl_launch_dependents();  // the next primal kernel reads the state only after its wait
+  // The state this kernel reads was written by the previous dual kernel, which completed before
+  // the primal kernel let this one launch (see there): read it now, from L2 (a line in this SM's
+  // L1 may predate it), so the loads overlap the primal kernel's last CTAs. The last CTA of the
+  // instance takes the decision on this copy, with the plan ranges read here too: loads of either
+  // after the last arrival would be on every attempt's path (FP64, 20,011 x 40,022: 24.8 us an
+  // attempt with them there, 22.4 with them here; FP32, 90,007 x 180,014: 35.9 and 30.8).
+  __shared__ StepState s;
+  __shared__ PlanRanges range;
+  const int inst = a.plan.cta_inst[b];
+  StepState* stw = a.st_mut + inst;
+  load_state(stw, s);
+  if (threadIdx.x >= 64 && threadIdx.x < 72) {
+    const int k = (int)threadIdx.x - 64, end = k & 1;
+    const int32_t* v[4] = {a.plan.inst_cta_begin, a.plan.inst_split_begin, a.p_cta_begin, a.p_split_begin};
+    reinterpret_cast<int*>(&range)[k] = v[k >> 1][inst + end];
+  }
   const int nt = stage_tiles(a.plan.tiles, a.plan.cta_tile_begin[b], a.plan.cta_tile_begin[b + 1], tl);
-  // The state this kernel reads was written by the previous dual kernel, which completed
-  // before the primal kernel let this one launch (see there): read it now, from L2 (a line in
-  // this SM's L1 may predate it), so the loads overlap the primal kernel's last CTAs.
-  const StepState* st = a.st_mut + a.plan.cta_inst[b];
-  const int done = __ldcg(&st->done);
-  const int pending = __ldcg(&st->pending_commit);
-  const int p = __ldcg(&st->parity);
-  const double commit_weight = __ldcg(&st->commit_weight);
-  const double od64 = __ldcg(&st->omega) * __ldcg(&st->tau);  // primal_weight * step_size
-  __shared__ double factors[2];   // the decision's, loaded while the primal kernel ends
-  if (threadIdx.x == 0) step_factors(st, factors);
   pdl_wait();
-  if (done) return;
-  const DualScalars<T> sc{pending != 0, (T)commit_weight, (T)od64, p ? a.y1 : a.y0, p ? a.y0 : a.y1,
+  if (s.done) return;
+  const int p = s.parity;
+  const bool pending = s.pending_commit != 0;
+  const DualScalars<T> sc{pending, (T)s.commit_weight, (T)(s.omega * s.tau), p ? a.y1 : a.y0, p ? a.y0 : a.y1,
                           p ? a.kx1 : a.kx0, p ? a.kx0 : a.kx1};
   T acc_i = T(0), acc_d = T(0);
   dual_work(a, sc, sm, tl, nt, acc_i, acc_d);
-  const int inst = a.plan.cta_inst[b];
-  const int c0 = a.plan.inst_cta_begin[inst], c1 = a.plan.inst_cta_begin[inst + 1];
-  StepState* stw = a.st_mut + inst;
   const T v[2] = {acc_i, acc_d};
   cta_sums<2>(v, tot, red);
   if (threadIdx.x == 0) {
@@ -676,18 +682,18 @@ __global__ void __launch_bounds__(kBlock, kDualCtasPerSm) dual_step_kernel(DualA
     a.part_d[a.plan.num_ctas + b] = tot[1];
     __threadfence();
     const unsigned prev = atomicAdd(&stw->arrive, 1u);
-    is_last = (prev == (unsigned)(c1 - c0 - 1)) ? 1 : 0;
+    is_last = (prev == (unsigned)(range.c1 - range.c0 - 1)) ? 1 : 0;
   }
   __syncthreads();
   if (!is_last) return;
-  // The instance's last CTA: the state into shared memory from L2, one 8-byte word per thread, and
-  // all CTAs' sums, in one round of loads (the barriers of cta_sums order the copy before its
-  // use); then thread 0 takes the decision. This tail is on every attempt's path: with the primal
-  // sum and the decision's inputs formed by the instance's first CTA after its own work (4,600
-  // cycles), sums by one warp (3,600) and the decision on the shared copy (2,600) it took twice as long.
-  __shared__ StepState s;
-  load_state(stw, s);
-  step_totals(a, inst, s, tot, red);
+  // The instance's last CTA: all CTAs' sums in one round of loads, the step-size factors by a warp
+  // that adds none, then thread 0 takes the decision. This tail is on every attempt's path (3-4 us
+  // of a 13 us attempt of a small LP): with the primal sum and the decision's inputs formed by the
+  // instance's first CTA after its own work, sums by one warp and the state and ranges loaded here
+  // it took more than twice as long.
+  __shared__ double factors[2];
+  if (threadIdx.x == 32 * (kBlock / 32 - 1)) step_factors(&s, factors);
+  step_totals(a, range, s, tot, red);
   if (threadIdx.x == 0) {
     s.arrive = 0;
     if (pending) s.primal_spmv += 1;
