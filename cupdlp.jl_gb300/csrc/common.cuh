@@ -121,6 +121,7 @@ struct StepState {
   double rcp_w_primal, rcp_w_dual;
   int eval_active, eval_current, eval_restart;
   int restart;             // RestartMode of the restart kernel that follows
+  long long chunk_ns;      // device time of cluster_kernel in this chunk
 };
 
 // ----------------------------------------------------------------------------------

@@ -32,7 +32,7 @@
 #include "host_logic.h"
 #include "problem.h"
 #include "spmv.cuh"
-#include "step_kernels.cuh"
+#include "cluster_solve.cuh"
 
 namespace gpdhg {
 
@@ -127,6 +127,7 @@ struct Workspace {
   DBuf<SegItem> seg_n, seg_m;
   DBuf<int32_t> seg_n_begin, seg_m_begin;
   int nseg_n = 1, nseg_m = 1;
+  ClusterPlan<T> cluster;   // a small LP's intervals run on one cluster instead of as step graphs
   cudaGraphExec_t graphs[kGraphLevels] = {}, evaluation = nullptr;
   // profiled variants: an event between every pair of kernels
   std::vector<cudaEvent_t> pev;   // per-kernel timing events (params.profile_kernels)
@@ -263,7 +264,9 @@ struct Workspace {
     return ex;
   }
   void build_graphs() {
-    for (int lv = 0; lv < kGraphLevels; ++lv) graphs[lv] = capture(1 << lv);
+    plan_cluster(cluster, plan_p, plan_d, n, m, P->stream);
+    if (!cluster.size)
+      for (int lv = 0; lv < kGraphLevels; ++lv) graphs[lv] = capture(1 << lv);
     evaluation = capture_evaluation();
   }
   // The same pairs launched directly with an event between every two kernels, for
@@ -572,17 +575,26 @@ bool run_phase(gpdhg_problem* P, Workspace<T>& W, const gpdhg_params& prm, LoopS
       const int remaining = st.target_in_chunk - st.accepted_in_chunk;
       const int attempts_before = st.attempts_in_chunk;
       const int lv = graph_level(remaining);
-      CK(cudaEventRecord(W.ev0, s));
-      if (prof)
-        W.launch_profiled(1 << lv);
-      else
-        CK(cudaGraphLaunch(W.graphs[lv], s));
-      P->launches += 2 * (1 << lv);
-      CK(cudaEventRecord(W.ev1, s));
-      CK(cudaStreamSynchronize(s));
-      float ms = 0.f;
-      CK(cudaEventElapsedTime(&ms, W.ev0, W.ev1));
-      L.step_loop_sec += 1e-3 * ms;
+      if (W.cluster.size && !prof) {
+        if (launches) push_state_async();   // the kernel leaves its state in the mirror
+        launch_cluster(W.cluster, s, W.primal_args(kStepNormal), W.dual_args(), W.st_host.p);
+        ++P->launches;
+        CK(cudaStreamSynchronize(s));
+        L.step_loop_sec += 1e-9 * (double)st.chunk_ns;
+        st.chunk_ns = 0;
+      } else {
+        CK(cudaEventRecord(W.ev0, s));
+        if (prof)
+          W.launch_profiled(1 << lv);
+        else
+          CK(cudaGraphLaunch(W.graphs[lv], s));
+        P->launches += 2 * (1 << lv);
+        CK(cudaEventRecord(W.ev1, s));
+        CK(cudaStreamSynchronize(s));
+        float ms = 0.f;
+        CK(cudaEventElapsedTime(&ms, W.ev0, W.ev1));
+        L.step_loop_sec += 1e-3 * ms;
+      }
       if (prof) {
         const std::vector<cudaEvent_t>& ev = W.pev;
         const int did = st.attempts_in_chunk - attempts_before;

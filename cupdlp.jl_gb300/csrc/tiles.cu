@@ -278,8 +278,13 @@ void build_tile_plan(TilePlan<T>& plan, const DeviceMatrix& M, const std::vector
   cta_begin.push_back((int32_t)tiles.size());
   // slots of the lane-interleaved copy: 32 E per warp tile, in plan order
   long long slots = 0;
+  plan.tile_slot.clear();
+  plan.tile_slot.reserve(tiles.size() + 1);
+  plan.warp_tiles_only = true;
   for (Tile& t : tiles) {
+    plan.tile_slot.push_back((int32_t)slots);
     if (t.e_log2 < 0) {
+      plan.warp_tiles_only = false;
       t.data_begin = 0;
       continue;
     }
@@ -287,6 +292,7 @@ void build_tile_plan(TilePlan<T>& plan, const DeviceMatrix& M, const std::vector
     slots += 32LL << t.e_log2;
     if (slots > 0x7fffffffLL) throw Error(GPDHG_ERR_NOT_SUPPORTED, "tile plan exceeds 2^31 interleaved slots");
   }
+  plan.tile_slot.push_back((int32_t)slots);
   plan.num_tiles = (int32_t)tiles.size();
   plan.num_ctas = (int32_t)cta_inst.size();
   plan.num_splits = splits;
@@ -315,6 +321,7 @@ void build_tile_plan(TilePlan<T>& plan, const DeviceMatrix& M, const std::vector
         plan.tiles.get(), nt, mv.col, mv.val, plan.icol.get(), plan.ival.get());
     CK_LAUNCH();
   }
+  plan.cta_tile = cta_begin;
   // the host vectors die at return: wait for the copies before they do
   CK(cudaStreamSynchronize(s));
   tr.mark(side == kTileSideAt ? "    plan A': copies, interleave" : "    plan A: copies, interleave");

@@ -108,6 +108,10 @@ struct TilePlan {
   DBuf<T> ival;
   int32_t num_tiles = 0, num_ctas = 0, num_splits = 0;
   long long interleaved_slots = 0;
+  // on the host: first tile of each CTA (CTAs + 1), first slot of each tile in plan order (tiles + 1),
+  // and whether every tile is a warp tile
+  std::vector<int32_t> cta_tile, tile_slot;
+  bool warp_tiles_only = true;
   TileView<T> view() const {
     return TileView<T>{tiles.get(),      cta_tile_begin.get(), cta_inst.get(), inst_cta_begin.get(),
                        inst_split_begin.get(), carry.get(),     counter.get(),  nullptr,

@@ -201,7 +201,7 @@ typedef struct gpdhg_result {
   int32_t fp64_handoff_iteration;  /* iteration at which the FP64 phase began, -1 if none */
   gpdhg_iteration_stats last_iteration_stats;
   /* measurement (additions): device time of the step loop, attempts per phase */
-  double step_loop_device_sec;     /* CUDA-event time of all step launches */
+  double step_loop_device_sec;     /* device time of all step launches */
   int64_t accepted_steps;
   int64_t rejected_steps;
   /* with params.profile_kernels: summed CUDA-event durations of the step kernels that did
