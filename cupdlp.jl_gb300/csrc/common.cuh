@@ -51,8 +51,8 @@ constexpr int kReduceBlocks = 304;   // 2 x 152 SMs for grid-stride reductions
 
 // One CTA's share of a CSR matrix: rows [row_begin, row_end) and the schedule used for
 // them (see spmv.cuh): staged short rows reduced by groups of `group` lanes, warp-per-row
-// register accumulation, or one long row streamed by the whole CTA.
-enum ItemMode : int32_t { kItemStaged = 0, kItemWarps = 1, kItemLong = 2 };
+// register accumulation, one long row streamed by the whole CTA, or long rows by a warp each.
+enum ItemMode : int32_t { kItemStaged = 0, kItemWarps = 1, kItemLong = 2, kItemLongWarps = 3 };
 struct RowItem {
   int32_t row_begin;
   int32_t row_end;

@@ -18,12 +18,22 @@ std::vector<RowItem> build_row_items(const int32_t* rp, int32_t nrows) {
   // power-law matrix into thousands of tiny items); such an item of at most 8 rows averaging
   // >= 64 nonzeros runs warp-per-row, any other is staged, with the largest power-of-two lane
   // group (<= 32) that still gives every row its own group.
+  // Runs of rows of more than kCtaRow nonzeros that fit a stage share a CTA, a warp each, in runs of 4
+  // to 8: a shorter run would leave most of its CTA idle while a whole CTA per row has 8 warps on it.
   constexpr int64_t kCtaRow = 256, kWarpRow = 64;
+  constexpr int kLongRun = 4;
   std::vector<RowItem> items;
   auto len = [&](int32_t r) { return (int64_t)rp[r + 1] - rp[r]; };
   int32_t r = 0;
   while (r < nrows) {
     if (len(r) > kCtaRow) {
+      int run = 0;
+      while (run < kBlock / 32 && r + run < nrows && len(r + run) > kCtaRow && len(r + run) <= kStage) ++run;
+      if (run >= kLongRun) {
+        items.push_back({r, r + run, 32, kItemLongWarps, rp[r], (int32_t)(rp[r + run] - rp[r])});
+        r += run;
+        continue;
+      }
       items.push_back({r, r + 1, 0, kItemLong, rp[r], (int32_t)len(r)});
       ++r;
       continue;

@@ -90,7 +90,7 @@ struct PinnedBuf {
 };
 
 // Row-block schedule: consecutive rows packed while their nonzeros fit the SpMV stage
-// (kStage) and there are at most kBlock of them; a longer row gets an item of its own.
+// (kStage) and there are at most kBlock of them; rows of more than 256 nonzeros get items of their own.
 std::vector<RowItem> build_row_items(const int32_t* row_ptr, int32_t nrows);
 
 // CSR of A' built on the GPU from an uploaded A (ingest.cu: a stable radix sort of the

@@ -5,7 +5,9 @@
 //                one row per group of `group` lanes (1..32) — steps 1-3 below;
 //   kItemWarps   up to 8 rows of >= 64 nonzeros, one warp per row: register accumulation
 //                (one FMA per nonzero, four independent loads per lane in flight);
-//   kItemLong    one row longer than the stage, streamed by the whole CTA.
+//   kItemLong    one row of more than 256 nonzeros, streamed by the whole CTA;
+//   kItemLongWarps  up to 8 such rows of at most kStage nonzeros, one per warp, each summed in
+//                the order of kItemLong (long_row_dot).
 // Staged items:
 //   1. the row's own epilogue loads (`pre`) are issued first;
 //   2. every thread loads U (col, val) pairs of the item — fully unrolled, independent,
@@ -48,6 +50,57 @@ __device__ __forceinline__ T warp_row_dot(const CsrView<T>& M, const T* __restri
   return warp_sum((a0 + a1) + (a2 + a3));
 }
 
+// Row r of M (at most kStage nonzeros) times xg by one warp, in the order of a whole CTA's sum
+// (kItemLong): virtual warp w takes the nonzeros 256 q + 32 w + lane in order of q, the warps' sums
+// are shuffle trees, added in order of w. The eight trees share their levels' instructions (lanes
+// keep half of the quantities at each), 9 additions instead of 40 or, by a CTA, 8 x (8 + 7 + 5):
+// on the power-law LPs, whose rows of 257 to 2,048 nonzeros hold most of the matrix, those kept the
+// FP64 pipe 74% busy, and a CTA per row is short of loads in flight. A'y of the 500k x 1M LP in FP64
+// 209 -> 88 us, of the 1M x 2M LP in FP32 173 -> 101 us.
+template <class T>
+__device__ __forceinline__ T long_row_dot(const CsrView<T>& M, const T* __restrict__ xg, int r, int lane) {
+  constexpr int W = kBlock / 32;
+  static_assert(W == 8, "three levels of pairs");
+  const unsigned full = 0xffffffffu;
+  const int s = M.row_ptr[r], e = M.row_ptr[r + 1];
+  T a[W];
+#pragma unroll
+  for (int w = 0; w < W; ++w) a[w] = T(0);
+  for (int base = s; base < e; base += kBlock) {
+    int c[W];
+    T v[W];
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      const int k = base + 32 * w + lane;
+      c[w] = k < e ? lds(M.col + k) : -1;
+      v[w] = k < e ? lds(M.val + k) : T(0);
+    }
+    T x[W];
+#pragma unroll
+    for (int w = 0; w < W; ++w) x[w] = c[w] >= 0 ? xg[c[w]] : T(0);
+#pragma unroll
+    for (int w = 0; w < W; ++w) {
+      if (base + 32 * w >= e) break;   // uniform over the warp
+      a[w] = base == s ? fma(v[w], x[w], T(0)) : a[w] + fma(v[w], x[w], T(0));
+    }
+  }
+#pragma unroll
+  for (int h = W / 2, o = 16; h > 0; h >>= 1, o >>= 1) {
+    const bool up = (lane & o) != 0;
+#pragma unroll
+    for (int w = 0; w < h; ++w) {
+      const T give = up ? a[w] : a[w + h], keep = up ? a[w + h] : a[w];
+      a[w] = keep + __shfl_xor_sync(full, give, o);
+    }
+  }
+  a[0] += __shfl_xor_sync(full, a[0], 2);
+  a[0] += __shfl_xor_sync(full, a[0], 1);
+  T sum = T(0);
+#pragma unroll
+  for (int w = 0; w < W; ++w) sum += __shfl_sync(full, a[0], 4 * w);   // lanes 4 w.. hold warp w's
+  return sum;
+}
+
 // Runs the item's rows. Every thread of the CTA must call it. `stage` holds kStage T, and
 // so does `stage2` when T is double (unused otherwise).
 template <class T, class Pre, class Post>
@@ -56,6 +109,16 @@ __device__ __forceinline__ void spmv_item(const CsrView<T>& M, const T* __restri
   constexpr int U = kStageDepth;
   const RowItem it = M.items[item];
   const int tid = threadIdx.x;
+  if (it.mode == kItemLongWarps) {
+    const int lane = tid & 31, r = it.row_begin + (tid >> 5);
+    if (r < it.row_end) {
+      decltype(pre(r)) p{};
+      if (lane == 0) p = pre(r);
+      const T sum = long_row_dot(M, xg, r, lane);
+      if (lane == 0) post(r, sum, p);
+    }
+    return;
+  }
   if (it.mode == kItemWarps) {
     const int lane = tid & 31;
     for (int base = it.row_begin; base < it.row_end; base += kBlock / 32) {
@@ -88,10 +151,12 @@ __device__ __forceinline__ void spmv_item(const CsrView<T>& M, const T* __restri
         v[q] = k < e ? lds(M.val + k) : T(0);
       }
 #pragma unroll
-      for (int q = 0; q < U; ++q) acc[q] += v[q] * xg[c[q]];
+      for (int q = 0; q < U; ++q)
+        if (base + q * kBlock < e) acc[q] += v[q] * xg[c[q]];   // the same for the whole CTA
     }
 #pragma unroll
-    for (int q = 1; q < U; ++q) acc[0] += acc[q];
+    for (int q = 1; q < U; ++q)
+      if (s + q * kBlock < e) acc[0] += acc[q];
     const T a = warp_sum(acc[0]);
     __syncthreads();
     if ((tid & 31) == 0) wsum[tid >> 5] = a;
