@@ -476,11 +476,9 @@ struct BatchWorkspace {
 
   // one side's pass over the segments of the evaluated instances (StepState::eval_active)
   template <int Q, unsigned MAXMASK, class F>
-  void seg_reduce(bool n_side, F f) {
-    const int nit = n_side ? B->nseg_n : B->nseg_m;
-    seg_reduce_kernel<Q, MAXMASK, F><<<nit, kBlock, 0, B->stream>>>(
-        n_side ? B->seg_n.get() : B->seg_m.get(), st_dev.get(), f, n_side ? red_part_n.get() : red_part_m.get(), nit);
-    CK_LAUNCH();
+  void seg_reduce(bool n_side, const F& f) {
+    launch_reduce<Q, MAXMASK>(n_side ? B->seg_n.get() : B->seg_m.get(), st_dev.get(), f,
+                              n_side ? red_part_n.get() : red_part_m.get(), n_side ? B->nseg_n : B->nseg_m, B->stream);
   }
   // One evaluation of the instances marked in the state, as the lone solve's graph: the state, the
   // pending steps' column side beside the row pass and A' y-bar, the column pass, one read-back.

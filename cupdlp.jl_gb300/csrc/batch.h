@@ -12,7 +12,7 @@
 
 namespace gpdhg {
 
-constexpr int kSegLen = 1024;   // elements per segmented-reduction item (one CTA each)
+constexpr int kSegLen = 1024;   // elements per segmented-reduction item
 
 template <class T>
 struct BatchWorkspace;

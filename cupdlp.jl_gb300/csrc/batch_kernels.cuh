@@ -15,30 +15,150 @@
 namespace gpdhg {
 
 // ---- segmented FP64 reductions --------------------------------------------------
-// A segment item is a contiguous element range of one instance, reduced by one CTA into its
-// partials; then one CTA per instance and quantity reduces the instance's items in order. (One
-// CTA per instance for all quantities took 15-34 us on 1,000-2,000 items, its loads of 25
-// quantities one after the other; one CTA each takes 6 us.) st NULL: every instance is active.
-// The passes are bound by the FP64 pipe (62-81% busy) and the latency of a thread's dozen loads, so
-// 3 CTAs per SM (80 registers, some spilled in the column pass; 2 CTAs: 110 and 212 us for the two
-// column passes below). Cold-cache times, FP64 arithmetic plainly written -> as it is: column pass
-// of the transportation LP (1M columns, FP64) 194 -> 101 us, of the power-law LP (2M, FP32) 428 ->
-// 189 us, its row pass (1M rows) 127 -> 93 us. (Longer segments, in one wave of CTAs, take 70, 138
-// and 70 us, but add the restart scores in another order.)
+// A segment item is a contiguous range of at most kSegLen elements of one instance, reduced by a
+// cluster of two CTAs of 128 threads into its partials; then one CTA per instance and quantity reduces
+// the instance's items in order. (One CTA per instance for all quantities took 15-34 us on
+// 1,000-2,000 items, its loads of 25 quantities one after the other; one CTA each takes 6 us.) st
+// NULL: every instance is active.
+//
+// Thread t of the 256 takes the elements t, t + 256, ... of its item; a quantity's 256 sums are added
+// by one warp, lane l the entries l, l + 32, ... in order and then a shuffle tree (restart scores
+// need this very order: they decide where the solve restarts). The passes are bound by the FP64 pipe
+// (a third of their time is the least its arithmetic can take, a sixth the reduction) and by the 4,000
+// cycles that one element takes a warp, so:
+//   * a thread loads its next element's dozen operands before it works on one (128 registers);
+//   * the item's sums are spread over both CTAs (stored into the reducing warp's CTA over
+//     distributed shared memory), which on a small LP are two SMs' FP64 pipes instead of one, and on
+//     a large one halve the granularity of the last wave;
+//   * a warp's up to three sums share the instructions of their trees (6 additions, not 15).
+// Times of the column and the row pass, with one CTA of 256 threads per item -> as it is: FP64 20,011 x
+// 40,022 18.6 -> 13.4 and 13.6 -> 10.4 us; FP32 90,007 x 180,014 25 -> 20 and 30 -> 22 us;
+// transportation 1M columns FP64 90 -> 66 us; power-law FP32 (2M, 1M) 177 -> 150 and 94 -> 87 us. Clusters of
+// 4 CTAs of 64 take 67, 152 and 87 us on the last two, of 8 CTAs of 32 twice that; a warp per item 88,
+// 203 and 125 us, and 60-72 us on the small ones.
+constexpr int kPassCluster = 2;
+template <int N, int O>
+__device__ __forceinline__ void packed_tree(double* a) {   // N sums over 32 lanes; sum q ends at lane packed_lane
+  constexpr int H = (N + 1) / 2;
+  const bool up = (threadIdx.x & O) != 0;
+#pragma unroll
+  for (int w = 0; w < N - H; ++w) {
+    const double give = of_bits(up ? bits_of(a[w]) : bits_of(a[w + H]));
+    const double keep = of_bits(up ? bits_of(a[w + H]) : bits_of(a[w]));
+    a[w] = keep + __shfl_xor_sync(0xffffffffu, give, O);
+  }
+  if (N - H < H) a[H - 1] += __shfl_xor_sync(0xffffffffu, a[H - 1], O);
+  if constexpr (O > 1) packed_tree<H, O / 2>(a);
+}
+__host__ __device__ constexpr int packed_lane(int n, int q) {
+  int lane = 0;
+  for (int o = 16; o > 0; o >>= 1) {
+    const int h = (n + 1) / 2;
+    if (q >= h) {
+      lane |= o;
+      q -= h;
+    }
+    n = h;
+  }
+  return lane;
+}
+__host__ __device__ constexpr int count_bits(unsigned m) { return m ? (int)(m & 1u) + count_bits(m >> 1) : 0; }
+// The quantities in the order of their reduction, sums before maxima: warp g of the cluster's eight
+// takes the slots g, g + 8, ...
+template <int Q, unsigned MAXMASK>
+struct PassSlots {
+  static constexpr int kWarps = kBlock / 32;
+  static constexpr int kSums = Q - count_bits(MAXMASK);
+  static constexpr int kRounds = (Q + kWarps - 1) / kWarps, kSumRounds = (kSums + kWarps - 1) / kWarps;
+  __host__ __device__ static constexpr int slot(int q) {
+    const int maxima = count_bits(MAXMASK & ((1u << q) - 1u));
+    return MAXMASK >> q & 1u ? kSums + maxima : q - maxima;
+  }
+  __device__ static __forceinline__ int quantity(int s) {
+    int q = 0;
+#pragma unroll
+    for (int k = 0; k < Q; ++k)
+      if (slot(k) == s) q = k;
+    return q;
+  }
+};
+// F: Params(st, inst), In, load(params, i, in), apply(params, i, in, acc).
 template <int Q, unsigned MAXMASK, class F>
-__global__ void __launch_bounds__(kBlock, 3) seg_reduce_kernel(const SegItem* items, const StepState* st, F f,
-                                                            double* partials, int num_items) {
-  __shared__ double sh[(Q < kRedChunk ? Q : kRedChunk) * kBlock];
-  __shared__ double res[Q];
-  const SegItem it = items[blockIdx.x];
-  if (st && !st[it.inst].eval_active) return;
+__global__ void __launch_bounds__(kBlock / kPassCluster, 2 * kPassCluster)
+    seg_reduce_kernel(const SegItem* items, const StepState* st, F f, double* partials, int num_items) {
+  using S = PassSlots<Q, MAXMASK>;
+  constexpr int W = S::kWarps, V = W / kPassCluster;   // warps of the cluster and of a CTA
+  __shared__ double sh[V * S::kRounds][kBlock];
+  const int rank = blockIdx.x % kPassCluster, item = blockIdx.x / kPassCluster;
+  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5, t = rank * (kBlock / kPassCluster) + (int)threadIdx.x;
+  const SegItem it = items[item];
+  if (st && !st[it.inst].eval_active) return;   // the whole cluster
+  cluster_arrive();   // waited for before the first store into the other CTA
   const typename F::Params p(st, it.inst);
   double acc[Q];
 #pragma unroll
   for (int q = 0; q < Q; ++q) acc[q] = 0.0;
-  for (int i = it.begin + threadIdx.x; i < it.end; i += kBlock) f(p, i, acc);
-  const double r = block_reduce_q<Q, MAXMASK>(acc, sh, res);
-  if ((int)threadIdx.x < Q) partials[(size_t)threadIdx.x * num_items + blockIdx.x] = r;
+  typename F::In in, next;
+  int i = it.begin + t;
+  if (i < it.end) f.load(p, i, in);
+#pragma unroll 1
+  for (; i < it.end; i += kBlock) {
+    if (i + kBlock < it.end) f.load(p, i + kBlock, next);
+    f.apply(p, i, in, acc);
+    in = next;
+  }
+  __syncwarp();
+  cluster_wait();
+#pragma unroll
+  for (int q = 0; q < Q; ++q) {
+    constexpr S slots{};
+    const int s = slots.slot(q), owner = s % W;
+    remote_store(remote_address(&sh[owner % V + V * (s / W)][t], owner / V), acc[q]);
+  }
+  cluster_barrier();
+  const int g = rank * V + warp;
+  double sum[S::kSumRounds];
+#pragma unroll
+  for (int j = 0; j < S::kRounds; ++j) {
+    const int s = g + W * j;
+    if (j < S::kSumRounds) sum[j] = 0.0;
+    if (s >= Q) break;
+    const double* c = sh[warp + V * j] + lane;
+    double v = c[0];
+    if (s < S::kSums) {
+#pragma unroll
+      for (int w = 1; w < W; ++w) v += c[w * 32];
+      if (j < S::kSumRounds) sum[j] = v;
+    } else {
+#pragma unroll
+      for (int w = 1; w < W; ++w) v = nan_max(v, c[w * 32]);
+      v = warp_nan_max(v);
+      if (lane == 0) partials[(size_t)S::quantity(s) * num_items + item] = v;
+    }
+  }
+  __syncwarp();
+  packed_tree<S::kSumRounds, 16>(sum);
+#pragma unroll
+  for (int j = 0; j < S::kSumRounds; ++j) {
+    const int s = g + W * j;
+    if (s < S::kSums && lane == packed_lane(S::kSumRounds, j)) partials[(size_t)S::quantity(s) * num_items + item] = sum[0];
+  }
+}
+template <int Q, unsigned MAXMASK, class F>
+inline void launch_reduce(const SegItem* items, const StepState* st, const F& f, double* partials, int num_items,
+                          cudaStream_t s) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3((unsigned)(kPassCluster * num_items));
+  cfg.blockDim = dim3(kBlock / kPassCluster);
+  cfg.stream = s;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = kPassCluster;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  CK(cudaLaunchKernelEx(&cfg, seg_reduce_kernel<Q, MAXMASK, F>, items, st, f, partials, num_items));
 }
 
 // Where one side's partials lie and where its results go (quantity q of instance k at

@@ -44,22 +44,6 @@ __device__ __forceinline__ unsigned cluster_size() {
   asm volatile("mov.u32 %0, %cluster_nctarank;" : "=r"(n));
   return n;
 }
-// Every thread of every CTA: what was written before is visible to all after.
-__device__ __forceinline__ void cluster_barrier() {
-  asm volatile("barrier.cluster.arrive.release.aligned;\n\tbarrier.cluster.wait.acquire.aligned;" ::: "memory");
-}
-// The shared-memory address of p (this CTA's) in CTA `rank` of the cluster, and a store there.
-__device__ __forceinline__ unsigned remote_address(const void* p, unsigned rank) {
-  unsigned a;
-  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(a) : "r"((unsigned)__cvta_generic_to_shared(p)), "r"(rank));
-  return a;
-}
-__device__ __forceinline__ void remote_store(unsigned a, double v) {
-  asm volatile("st.shared::cluster.f64 [%0], %1;" ::"r"(a), "d"(v) : "memory");
-}
-__device__ __forceinline__ void remote_store(unsigned a, float v) {
-  asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
-}
 // A product kept from being fused with what uses it.
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }

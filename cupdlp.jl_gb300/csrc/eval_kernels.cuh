@@ -274,12 +274,33 @@ struct EvalPassM {
     add_square(dual_violation(y, ineq), a[1]);
     a[2] = fma(b, y, a[2]);
   }
-  __device__ __forceinline__ void operator()(const Params& s, int i, double* a) const {
-    const T yc = (s.parity ? y1 : y0)[i], kc = (s.parity ? kx1 : kx0)[i];
-    const bool ineq = ineq_flag ? ineq_flag[i] != 0 : i >= neq;
+  // A row's operands, loaded apart from their use so that a caller can load ahead.
+  struct In {
+    T yc, kc, sy, skx, b, ry, rkx;
+    double con, rcon, ob;
+    bool ineq;
+  };
+  __device__ __forceinline__ void load(const Params& s, int i, In& v) const {
+    v.yc = (s.parity ? y1 : y0)[i];
+    v.kc = (s.parity ? kx1 : kx0)[i];
+    v.ineq = ineq_flag ? ineq_flag[i] != 0 : i >= neq;
+    if (!s.current) {
+      v.sy = sy[i];
+      v.skx = skx[i];
+    }
+    v.con = con[i];
+    v.rcon = rcon[i];
+    v.ob = ob[i];
+    v.b = this->b[i];
+    v.ry = ry[i];
+    if (s.restart) v.rkx = rkx[i];
+  }
+  __device__ __forceinline__ void apply(const Params& s, int i, const In& v, double* a) const {
+    const T yc = v.yc, kc = v.kc;
+    const bool ineq = v.ineq;
     T ya = yc, ka = kc;
     if (!s.current) {
-      T vy = sy[i], vk = skx[i];
+      T vy = v.sy, vk = v.skx;
       if (s.pending) {
         vy = fma(yc, s.commit_weight, vy);
         vk = fma(kc, s.commit_weight, vk);
@@ -292,9 +313,9 @@ struct EvalPassM {
     ay[i] = ya;
     akx[i] = ka;
     {
-      const double y = div_rcp(widen(ya), con[i], rcon[i]);   // :474-475
-      const double kx = widen(ka) * con[i];                   // :476-477
-      const double b = ob[i];
+      const double y = div_rcp(widen(ya), v.con, v.rcon);   // :474-475
+      const double kx = widen(ka) * v.con;                  // :476-477
+      const double b = v.ob;
       const double cv = row_violation(b - kx, ineq);
       add_square(cv, a[kM_CvSq]);
       a[kM_CvMax] = nan_max(a[kM_CvMax], cv);
@@ -308,12 +329,11 @@ struct EvalPassM {
       a[kM_RayCvMax] = nan_max(a[kM_RayCvMax], row_violation(negate_bits(kx), ineq));
     }
     double* k = a + kEvalMQ;
-    const double b = widen(this->b[i]);
+    const double b = widen(v.b);
     point(yc, kc, b, ineq, k);
     point(ya, ka, b, ineq, k + 3);
-    const T yr = ry[i];
-    if (s.restart) point(yr, rkx[i], b, ineq, k + 6);
-    const double d = widen(ya) - widen(yr);
+    if (s.restart) point(v.ry, v.rkx, b, ineq, k + 6);
+    const double d = widen(ya) - widen(v.ry);
     k[9] = fma(d, d, k[9]);
   }
 };
@@ -342,23 +362,46 @@ struct EvalPassN {
     add_square(cost_residual(g, kept), a[2]);
     add_bound_term<false>(g, kept, l, u, a[3]);
   }
-  __device__ __forceinline__ void operator()(const Params& s, int j, double* a) const {
-    const T cs = c[j], xc = x[j];
-    T xa = xc, ga;
+  // A column's operands, loaded apart from their use so that a caller can load ahead.
+  struct In {
+    T c, x, sx, g, kty, l, u, rx, rgrad;   // g: A' y-bar, or the gradient as it stood
+    double var, rvar, ol, ou, oc;
+  };
+  __device__ __forceinline__ void load(const Params& s, int j, In& v) const {
+    v.c = c[j];
+    v.x = x[j];
     if (s.current) {
-      ga = grad[j];
+      v.g = grad[j];
     } else {
-      xa = (T)div_rcp(widen(sx[j]), s.wx, s.rwx);
-      ga = cs - aty[j];
+      v.sx = sx[j];
+      v.g = aty[j];
+    }
+    v.kty = kty[j];
+    v.var = var[j];
+    v.rvar = rvar[j];
+    v.ol = ol[j];
+    v.ou = ou[j];
+    v.oc = oc[j];
+    v.l = l[j];
+    v.u = u[j];
+    v.rx = rx[j];
+    if (s.restart) v.rgrad = rgrad[j];
+  }
+  __device__ __forceinline__ void apply(const Params& s, int j, const In& v, double* a) const {
+    const T cs = v.c, xc = v.x;
+    T xa = xc, ga = v.g;
+    if (!s.current) {
+      xa = (T)div_rcp(widen(v.sx), s.wx, s.rwx);
+      ga = cs - v.g;
     }
     ax[j] = xa;
     agrad[j] = ga;
-    const T gc = cs - kty[j];
+    const T gc = cs - v.kty;
     grad[j] = gc;
     {
-      const double x = div_rcp(widen(xa), var[j], rvar[j]);   // :470-471
-      const double g = widen(ga) * var[j];                    // :472-473
-      const double l = ol[j], u = ou[j], c = oc[j];
+      const double x = div_rcp(widen(xa), v.var, v.rvar);   // :470-471
+      const double g = widen(ga) * v.var;                   // :472-473
+      const double l = v.ol, u = v.ou, c = v.oc;
       const bool fl = bits_finite(l), fu = bits_finite(u);
       add_violation<true>(x, l, u, a[kN_LuSq], a[kN_LuMax]);
       a[kN_Cx] = fma(c, x, a[kN_Cx]);
@@ -380,13 +423,12 @@ struct EvalPassN {
       if (keptr) a[kN_RayRcMax] = nan_max(a[kN_RayRcMax], gr);
     }
     double* k = a + kEvalNQ;
-    const double l = widen(this->l[j]), u = widen(this->u[j]), c = widen(cs);
+    const double l = widen(v.l), u = widen(v.u), c = widen(cs);
     const bool fl = bits_finite(l), fu = bits_finite(u);
     point(xc, gc, l, u, c, fl, fu, k);
     point(xa, ga, l, u, c, fl, fu, k + 4);
-    const T xr = rx[j];
-    if (s.restart) point(xr, rgrad[j], l, u, c, fl, fu, k + 8);
-    const double d = widen(xa) - widen(xr);
+    if (s.restart) point(v.rx, v.rgrad, l, u, c, fl, fu, k + 8);
+    const double d = widen(xa) - widen(v.rx);
     k[12] = fma(d, d, k[12]);
   }
 };

@@ -61,8 +61,12 @@ struct DotF {
   struct Params {
     __device__ Params(const StepState*, int) {}
   };
-  __device__ __forceinline__ void operator()(const Params&, int i, double* acc) const {
-    acc[0] += (double)a[i] * (double)b[i];
+  struct In {
+    T a, b;
+  };
+  __device__ __forceinline__ void load(const Params&, int i, In& v) const { v = In{a[i], b[i]}; }
+  __device__ __forceinline__ void apply(const Params&, int, const In& v, double* acc) const {
+    acc[0] += (double)v.a * (double)v.b;
   }
 };
 
@@ -308,11 +312,9 @@ struct Workspace {
 
   // one side's pass over its segments into its partials
   template <int Q, unsigned MAXMASK, class F>
-  void reduce(bool n_side, F f, const StepState* st) {
-    const int nit = n_side ? nseg_n : nseg_m;
-    seg_reduce_kernel<Q, MAXMASK, F><<<nit, kBlock, 0, P->stream>>>(n_side ? seg_n.get() : seg_m.get(), st, f,
-                                                                     n_side ? red_part_n.get() : red_part_m.get(), nit);
-    CK_LAUNCH();
+  void reduce(bool n_side, const F& f, const StepState* st) {
+    launch_reduce<Q, MAXMASK>(n_side ? seg_n.get() : seg_m.get(), st, f, n_side ? red_part_n.get() : red_part_m.get(),
+                              n_side ? nseg_n : nseg_m, P->stream);
   }
   SegSide side(bool n_side, int quantities, unsigned maxmask) {
     return SegSide{n_side ? seg_n_begin.get() : seg_m_begin.get(), n_side ? red_part_n.get() : red_part_m.get(),
