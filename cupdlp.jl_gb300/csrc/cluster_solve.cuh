@@ -57,7 +57,8 @@ __device__ __forceinline__ unsigned long long global_ns() {
 template <class T>
 struct ClusterSide {
   T* val;
-  unsigned long long* rows;   // 32 per tile: the row (5 bits) of each of the lane's elements
+  unsigned long long* rows;   // 32 per tile: where the sum after each of the lane's elements goes (8
+                              // bits): the row that ends there, 33 + lane if it began in an earlier lane, else 32
   int32_t* col;               // local columns
   unsigned* info;             // 32 per tile: the lane's RunInfo
   Tile* tiles;
@@ -82,12 +83,12 @@ __device__ __forceinline__ ClusterSide<T> cluster_side(char* base, int tiles, in
 }
 
 // How a lane walks its elements of a tile: bits 0-7 the elements after which a row ends, then
-// whether its first row began in an earlier lane (that row's end completes it), whether its last
-// row goes on in the next lane, and whether that row began in this lane; the elements it holds; and
-// the tile's scan length (how many lanes back a completed row begins, at most).
+// whether the first of them ends a row that began in an earlier lane (and bits 24-28 that row), whether
+// its last row goes on in the next lane, and whether that row began in this lane; the elements it
+// holds; and the tile's scan length (how many lanes back a completed row begins, at most).
 struct RunInfo {
   static constexpr unsigned kHead = 1u << 8, kTail = 1u << 9, kTailStart = 1u << 10;
-  static constexpr int kCountShift = 12, kSpanShift = 16;
+  static constexpr int kCountShift = 12, kSpanShift = 16, kRowShift = 24;
 };
 
 // Copies a plan CTA's tiles from `tile` on, with columns counted from col0; the caller synchronises.
@@ -134,14 +135,18 @@ __device__ __forceinline__ void stage_cluster_side(const ClusterSide<T>& s, cons
     }
     const int begin = __shfl_sync(0xffffffffu, off, lo), end = __shfl_sync(0xffffffffu, off, lo + 1);
     if (j >= count) continue;
-    rows |= (unsigned long long)lo << (5 * j);
-    if (j == 0 && begin < kb) info |= RunInfo::kHead;
+    int to = 32;
     if (k + 1 == end) {
       info |= 1u << j;
-      if (begin < kb) head_back = lane - (begin >> t.e_log2);
-    } else if (j == count - 1) {
-      info |= RunInfo::kTail | (begin >= kb ? RunInfo::kTailStart : 0u);
+      to = lo;
+      if (begin < kb) {
+        head_back = lane - (begin >> t.e_log2);
+        info |= RunInfo::kHead | (unsigned)lo << RunInfo::kRowShift;
+        to = 33 + lane;
+      }
     }
+    rows |= (unsigned long long)to << (8 * j);
+    if (k + 1 < end && j == count - 1) info |= RunInfo::kTail | (begin >= kb ? RunInfo::kTailStart : 0u);
   }
   info |= (unsigned)__reduce_max_sync(0xffffffffu, head_back) << RunInfo::kSpanShift;
   s.rows[32 * q + lane] = rows;
@@ -169,7 +174,7 @@ __device__ __forceinline__ void staged_run(const U* base, int e_log2, U* d) {
 }
 
 // Row sums of the warp's tile q into rs, gathered from x (shared memory): the sums of tile_sums (same
-// elements per lane, order and scan), with the walk over rows read from the staged structure.
+// elements per lane, order and scan), with the walk over rows read from the staged structure and free of branches (rs: 65 entries).
 template <class T>
 __device__ __forceinline__ void staged_tile_sums(const ClusterSide<T>& s, const T* x, const Tile& t, int q, T* rs) {
   constexpr int kEMax = TileTraits<T>::kEMax;
@@ -183,6 +188,7 @@ __device__ __forceinline__ void staged_tile_sums(const ClusterSide<T>& s, const 
   const unsigned info = s.info[32 * q + lane];
   const unsigned long long rows = s.rows[32 * q + lane];
   const int count = (int)(info >> RunInfo::kCountShift) & 15;
+  const unsigned to[2] = {(unsigned)rows, (unsigned)(rows >> 32)};
 #pragma unroll
   for (int j = 0; j < kEMax; ++j) {
     if (j >= E) break;   // uniform over the warp
@@ -190,26 +196,17 @@ __device__ __forceinline__ void staged_tile_sums(const ClusterSide<T>& s, const 
   }
   rs[lane] = T(0);   // rows without elements
   __syncwarp();
-  T sum = T(0), head_sum = T(0);
-  int head_row = -1;
-  bool head = (info & RunInfo::kHead) != 0;
+  T sum = T(0);
 #pragma unroll
   for (int j = 0; j < kEMax; ++j) {
     if (j >= E) break;
-    if (j < count) sum = fma(v[j], xv[j], sum);
-    if (info >> j & 1u) {
-      const int row = (int)(rows >> (5 * j)) & 31;
-      if (head) {
-        head_row = row;
-        head_sum = sum;
-      } else {
-        rs[row] = sum;
-      }
-      head = false;
-      sum = T(0);
+    if (j < count) {
+      sum = fma(v[j], xv[j], sum);
+      rs[to[j >> 2] >> (8 * (j & 3)) & 0xffu] = sum;
     }
+    if (info >> j & 1u) sum = T(0);
   }
-  const int span = (int)(info >> RunInfo::kSpanShift);
+  const int span = (int)(info >> RunInfo::kSpanShift) & 31;
   if (span > 0) {
     T tail = info & RunInfo::kTail ? sum : T(0);
     int f = !(info & RunInfo::kTail) || (info & RunInfo::kTailStart) ? 1 : 0;
@@ -224,7 +221,7 @@ __device__ __forceinline__ void staged_tile_sums(const ClusterSide<T>& s, const 
       }
     }
     const T prev = __shfl_up_sync(full, tail, 1);
-    if (head_row >= 0) rs[head_row] = head_sum + prev;
+    if (info & RunInfo::kHead) rs[info >> RunInfo::kRowShift & 31] = rs[33 + lane] + prev;
   }
   __syncwarp();
 }
@@ -246,7 +243,7 @@ __global__ void __launch_bounds__(kBlock, 1)
     cluster_kernel(PrimalArgs<T> pa, DualArgs<T> da, const int32_t* p_slot, const int32_t* d_slot, const ClusterLp* lps,
                    StepState* mirror) {
   extern __shared__ __align__(16) char dynamic[];
-  __shared__ T rs_all[kBlock / 32][32];
+  __shared__ T rs_all[kBlock / 32][65];
   __shared__ double part[3][kClusterPlanCtas];   // every plan CTA's sums: dy . K dx, ||dy||^2, ||dx||^2
   __shared__ double total[3], factors[2];
   __shared__ int slot_begin[kClusterRounds][kClusterTiles];
@@ -312,6 +309,7 @@ __global__ void __launch_bounds__(kBlock, 1)
       const int j = t.row_begin + lane;
       PrimalIn<T> e{};
       if (lane < t.rows) primal_load(pa, pending, false, j, e);
+      rs[lane] = e.x;   // waits for the operands: left to their first use, behind the sums, an attempt takes 1.6 us more
       T d = T(0), xv = e.x, ktyv = e.dx;
       if (pending) {
         staged_tile_sums(P[k], ys, t, warp, rs);
