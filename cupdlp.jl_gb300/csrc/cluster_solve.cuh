@@ -240,8 +240,7 @@ __host__ __device__ constexpr size_t cluster_vector_bytes(int cols, int rows) {
 
 template <class T>
 __global__ void __launch_bounds__(kBlock, 1)
-    cluster_kernel(PrimalArgs<T> pa, DualArgs<T> da, const int32_t* p_slot, const int32_t* d_slot, const ClusterLp* lps,
-                   StepState* mirror) {
+    cluster_kernel(PrimalArgs<T> pa, DualArgs<T> da, const int32_t* p_slot, const int32_t* d_slot, const ClusterLp* lps) {
   extern __shared__ __align__(16) char dynamic[];
   __shared__ T rs_all[kBlock / 32][65];
   __shared__ double part[3][kClusterPlanCtas];   // every plan CTA's sums: dy . K dx, ||dy||^2, ||dx||^2
@@ -413,7 +412,7 @@ __global__ void __launch_bounds__(kBlock, 1)
   if (rank == 0) {
     if (threadIdx.x == 0) s.chunk_ns += (long long)(global_ns() - t0);
     __syncthreads();
-    store_state(s, mirror + lp.inst);
+    store_state(s, da.st_mut + lp.inst);
   }
 }
 
@@ -492,13 +491,12 @@ void plan_cluster(ClusterPlan<T>& plan, const TilePlan<T>& p, const TilePlan<T>&
 }
 
 template <class T>
-void launch_cluster(const ClusterPlan<T>& plan, cudaStream_t s, const PrimalArgs<T>& pa, const DualArgs<T>& da,
-                    StepState* mirror) {
+void launch_cluster(const ClusterPlan<T>& plan, cudaStream_t s, const PrimalArgs<T>& pa, const DualArgs<T>& da) {
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
   cluster_config(cfg, attr, plan.size, plan.size, plan.shared, s);
   CK(cudaLaunchKernelEx(&cfg, cluster_kernel<T>, pa, da, (const int32_t*)plan.p_slot.get(),
-                        (const int32_t*)plan.d_slot.get(), (const ClusterLp*)plan.lp.get(), mirror));
+                        (const int32_t*)plan.d_slot.get(), (const ClusterLp*)plan.lp.get()));
 }
 
 }  // namespace gpdhg

@@ -115,9 +115,9 @@ struct StepState {
   long long pow_table_len;
   double half_over_omega;  // 0.5 / omega, set by the host with omega
   double tto;              // tau / omega, kept by whoever changes tau or omega (the host, the step decision)
-  // set by the host before an evaluation: 1 / sum_w_primal and 1 / sum_w_dual, whether the
-  // instance is evaluated, whether it has no average yet (the current point stands in), and
-  // whether the last restart point's KKT ingredients are needed
+  // for an evaluation, set by the host or by the decision that ends a chunk: 1 / sum_w_primal and
+  // 1 / sum_w_dual, whether the instance is evaluated, whether it has no average yet (the current
+  // point stands in), and (by the host) whether the last restart point's KKT ingredients are needed
   double rcp_w_primal, rcp_w_dual;
   int eval_active, eval_current, eval_restart;
   int restart;             // RestartMode of the restart kernel that follows

@@ -259,7 +259,6 @@ struct Workspace {
       launch_primal(kStepNormal, s);
       launch_dual(s);
     }
-    cudaMemcpyAsync(st_host.p, st_dev.get(), sizeof(StepState), cudaMemcpyDeviceToHost, s);
     cudaError_t e = cudaStreamEndCapture(s, &g);
     CK(e);
     cudaGraphExec_t ex = nullptr;
@@ -290,7 +289,6 @@ struct Workspace {
       CK(cudaEventRecord(pev[2 * k + 2], s));
     }
     CK_LAUNCH();
-    CK(cudaMemcpyAsync(st_host.p, st_dev.get(), sizeof(StepState), cudaMemcpyDeviceToHost, s));
   }
   const double* ensure_pow_table(double r, double g) {
     if (pow_table.get() && r == pow_r && g == pow_g) return pow_table.get();
@@ -304,9 +302,9 @@ struct Workspace {
     return pow_table.get();
   }
 
-  void spmv(const DeviceMatrix& M, const T* xin, T* yout) {
+  void spmv(const DeviceMatrix& M, const T* xin, T* yout, const StepState* st = nullptr) {
     if (M.num_items == 0) return;
-    spmv_kernel<T><<<M.num_items, kBlock, 0, P->stream>>>(M.view<T>(), xin, yout, nullptr, nullptr);
+    spmv_kernel<T><<<M.num_items, kBlock, 0, P->stream>>>(M.view<T>(), xin, yout, nullptr, st);
     CK_LAUNCH();
   }
 
@@ -326,24 +324,31 @@ struct Workspace {
     CK_LAUNCH();
     CK(cudaMemcpyAsync(red_host.p, red_out.get(), sizeof(double) * kEvalStride, cudaMemcpyDeviceToHost, P->stream));
   }
-  // One evaluation as a graph: the state to the device; the accepted step still to be applied (its
-  // K'y, x and Sigma x) beside the row pass (its Sigma y and Sigma Kx, the averages y-bar and Kx-bar
+  // One evaluation as a graph, with the state's way to the host: the accepted step still to be applied
+  // (its K'y, x and Sigma x) beside the row pass (its Sigma y and Sigma Kx, the averages y-bar and Kx-bar
   // with their unscaled statistics, src/iteration_stats_utils_gpu.jl:447-502, and restart-scheme
   // ingredients) and A' y-bar (the reference sums the steps' K'y with the averaging weights instead,
   // src/saddle_point_gpu.jl:176-189; the two agree in exact arithmetic); then the column pass and
-  // one read-back of all sums.
+  // one read-back of all sums. It is queued right behind the steps of its interval, whose last decision
+  // sets what it needs (end_chunk); behind steps that end short of the interval's goal it does
+  // nothing. (Launched by the host after reading the state, an interval took 12 us more, two round
+  // trips instead of one.)
   static constexpr int kEvaluationKernels = 5;
   cudaGraphExec_t capture_evaluation() {
     cudaStream_t s = P->stream;
-    cudaStream_t side_stream = nullptr;
-    cudaEvent_t fork = nullptr, join = nullptr;
+    cudaStream_t side_stream = nullptr, copy_stream = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr, copied = nullptr;
     CK(cudaStreamCreateWithFlags(&side_stream, cudaStreamNonBlocking));
     CK(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
+    CK(cudaStreamCreateWithFlags(&copy_stream, cudaStreamNonBlocking));
+    CK(cudaEventCreateWithFlags(&copied, cudaEventDisableTiming));
     CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    CK(cudaMemcpyAsync(st_dev.get(), st_host.p, sizeof(StepState), cudaMemcpyHostToDevice, s));
     CK(cudaEventRecord(fork, s));
     CK(cudaStreamWaitEvent(side_stream, fork, 0));
+    CK(cudaStreamWaitEvent(copy_stream, fork, 0));
+    CK(cudaMemcpyAsync(st_host.p, st_dev.get(), sizeof(StepState), cudaMemcpyDeviceToHost, copy_stream));
+    CK(cudaEventRecord(copied, copy_stream));
     primal_step_kernel<T><<<plan_p.num_ctas, kBlock, 0, side_stream>>>(primal_args(kStepCommitOnly));
     CK(cudaEventRecord(join, side_stream));
     reduce<kPassMQ, kEvalMMax>(
@@ -351,7 +356,7 @@ struct Workspace {
         EvalPassM<T>{P->con.get(), rcon.get(), P->ob.get(), b, y0.get(), y1.get(), kx0.get(), kx1.get(), ry.get(),
                      rkx.get(), sy.get(), skx.get(), ay.get(), akx.get(), P->neq, nullptr},
         st_dev.get());
-    spmv(P->At, ay.get(), tmp_n.get());
+    spmv(P->At, ay.get(), tmp_n.get(), st_dev.get());
     CK(cudaStreamWaitEvent(s, join, 0));
     reduce<kPassNQ, kEvalNMax>(
         true,
@@ -359,6 +364,7 @@ struct Workspace {
                      tmp_n.get(), kty.get(), rx.get(), rgrad.get(), ax.get(), agrad.get(), grad.get()},
         st_dev.get());
     finish_reductions(side(false, kPassMQ, kEvalMMax), side(true, kPassNQ, kEvalNMax), st_dev.get());
+    CK(cudaStreamWaitEvent(s, copied, 0));
     cudaGraph_t g = nullptr;
     CK(cudaStreamEndCapture(s, &g));
     cudaGraphExec_t ex = nullptr;
@@ -366,7 +372,9 @@ struct Workspace {
     cudaGraphDestroy(g);
     cudaEventDestroy(fork);
     cudaEventDestroy(join);
+    cudaEventDestroy(copied);
     cudaStreamDestroy(side_stream);
+    cudaStreamDestroy(copy_stream);
     return ex;
   }
   void launch_restart(cudaStream_t s) {
@@ -443,21 +451,30 @@ bool run_phase(gpdhg_problem* P, Workspace<T>& W, const gpdhg_params& prm, LoopS
     CK(cudaMemcpyAsync(W.st_dev.get(), W.st_host.p, sizeof(StepState), cudaMemcpyHostToDevice, s));
   };
 
+  auto launch_evaluation = [&]() {
+    CK(cudaGraphLaunch(W.evaluation, s));
+    P->launches += W.kEvaluationKernels;
+  };
+  bool evaluated = false;   // an evaluation of this iteration ran behind its steps
+
   while (true) {
     const long long it = L.iteration;
     if (eval_due(it, freq, it_limit, st.numerical_error != 0)) {
+      if (!evaluated) {   // not behind steps: at the start, and again in FP64 after a hand-off
+        // the average, or the current point (src/primal_dual_hybrid_gradient_gpu.jl:635-642)
+        st.eval_active = 1;
+        st.eval_current = (st.numerical_error || st.count_primal == 0 || st.count_dual == 0) ? 1 : 0;
+        st.eval_restart = W.restart_kkt.valid ? 0 : 1;
+        st.rcp_w_primal = st.eval_current ? 0.0 : 1.0 / st.sum_w_primal;
+        st.rcp_w_dual = st.eval_current ? 0.0 : 1.0 / st.sum_w_dual;
+        push_state_async();
+        launch_evaluation();
+        CK(cudaStreamSynchronize(s));
+      }
+      evaluated = false;
       st.kkt_passes += 2.0;  // KKT_PASSES_PER_TERMINATION_EVALUATION
       st.done = 0;
       st.restart = kNoRestart;
-      // The average, or the current point (src/primal_dual_hybrid_gradient_gpu.jl:635-642)
-      st.eval_active = 1;
-      st.eval_current = (st.numerical_error || st.count_primal == 0 || st.count_dual == 0) ? 1 : 0;
-      st.eval_restart = W.restart_kkt.valid ? 0 : 1;
-      st.rcp_w_primal = st.eval_current ? 0.0 : 1.0 / st.sum_w_primal;
-      st.rcp_w_dual = st.eval_current ? 0.0 : 1.0 / st.sum_w_dual;
-      CK(cudaGraphLaunch(W.evaluation, s));
-      P->launches += W.kEvaluationKernels;
-      CK(cudaStreamSynchronize(s));
       st.pending_commit = 0;
       const double* em = W.red_host.p;               // kM_*, then the rows' KKT ingredients
       const double* en = W.red_host.p + kEvalOutN;   // kN_*, then the columns'
@@ -568,22 +585,24 @@ bool run_phase(gpdhg_problem* P, Workspace<T>& W, const gpdhg_params& prm, LoopS
     st.half_over_omega = 0.5 / st.omega;
     st.tto = st.tau / st.omega;
     st.arrive = 0;
+    st.chunk_ns = 0;
+    st.eval_active = 0;
+    st.eval_restart = W.restart_kkt.valid ? 0 : 1;
     push_state_async();
     if (st.restart != kNoRestart) W.launch_restart(s);
-    const auto tb = Clock::now();
     long long launches = 0;
     const bool prof = prm.profile_kernels != 0;
+    const double loop_before = L.step_loop_sec;
     while (true) {
       const int remaining = st.target_in_chunk - st.accepted_in_chunk;
       const int attempts_before = st.attempts_in_chunk;
       const int lv = graph_level(remaining);
       if (W.cluster.size && !prof) {
-        if (launches) push_state_async();   // the kernel leaves its state in the mirror
-        launch_cluster(W.cluster, s, W.primal_args(kStepNormal), W.dual_args(), W.st_host.p);
+        launch_cluster(W.cluster, s, W.primal_args(kStepNormal), W.dual_args());
         ++P->launches;
+        launch_evaluation();
         CK(cudaStreamSynchronize(s));
-        L.step_loop_sec += 1e-9 * (double)st.chunk_ns;
-        st.chunk_ns = 0;
+        if (st.done) L.step_loop_sec += 1e-9 * (double)st.chunk_ns;
       } else {
         CK(cudaEventRecord(W.ev0, s));
         if (prof)
@@ -592,6 +611,7 @@ bool run_phase(gpdhg_problem* P, Workspace<T>& W, const gpdhg_params& prm, LoopS
           CK(cudaGraphLaunch(W.graphs[lv], s));
         P->launches += 2 * (1 << lv);
         CK(cudaEventRecord(W.ev1, s));
+        launch_evaluation();
         CK(cudaStreamSynchronize(s));
         float ms = 0.f;
         CK(cudaEventElapsedTime(&ms, W.ev0, W.ev1));
@@ -614,7 +634,8 @@ bool run_phase(gpdhg_problem* P, Workspace<T>& W, const gpdhg_params& prm, LoopS
       // accepted steps means the step size never settles
       if (++launches > 1000000) throw Error(GPDHG_ERR_INTERNAL, "step chunk did not finish");
     }
-    L.basic_time += std::chrono::duration<double>(Clock::now() - tb).count();
+    evaluated = true;
+    L.basic_time += L.step_loop_sec - loop_before;
     L.iteration += st.accepted_in_chunk + (st.numerical_error ? 1 : 0);
   }
 }

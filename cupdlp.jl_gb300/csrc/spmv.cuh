@@ -212,9 +212,9 @@ __device__ __forceinline__ void spmv_item(const CsrView<T>& M, const T* __restri
   if (owner) post(r, sum, p);
 }
 
-// y = M x over the row-block items of M. With row_inst non-NULL only the items whose first
-// row belongs to an instance under evaluation (StepState::eval_active) run (the packed matrix of a
-// batch; an item never spans two instances).
+// y = M x over the row-block items of M. With st non-NULL only the items of instances under evaluation
+// (StepState::eval_active) run; row_inst gives the instance of an item's first row (the packed matrix
+// of a batch; an item never spans two instances), NULL: one instance.
 struct NoPre {};
 template <class T>
 __global__ void __launch_bounds__(kBlock) spmv_kernel(CsrView<T> M, const T* __restrict__ x, T* y,
@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(kBlock) spmv_kernel(CsrView<T> M, const T* __r
   __shared__ T stage2[sizeof(T) == 8 ? kStage : 1];
   __shared__ T wsum[kBlock / 32];
   if ((int)blockIdx.x >= M.num_items) return;
-  if (row_inst && !st[row_inst[M.items[blockIdx.x].row_begin]].eval_active) return;
+  if (st && !st[row_inst ? row_inst[M.items[blockIdx.x].row_begin] : 0].eval_active) return;
   auto pre = [](int) { return NoPre{}; };
   auto post = [&](int i, T s, const NoPre&) { y[i] = s; };
   spmv_item(M, x, blockIdx.x, stage, stage2, wsum, pre, post);

@@ -334,10 +334,9 @@ __global__ void __launch_bounds__(kBlock, kPrimalCtasPerSm<T>) primal_step_kerne
   pdl_wait();
   pdl_launch_dependents();
   const StepState* st = a.st + a.plan.cta_inst[b];
-  if (st->done) return;
   const int pending = st->pending_commit;
   const bool commit_only = a.mode == kStepCommitOnly;
-  if (commit_only && !pending) return;
+  if (commit_only ? !pending || !st->eval_active : st->done != 0) return;
   const PrimalScalars<T> sc{pending != 0, (T)st->commit_weight, (T)st->tto, st->parity ? a.y1 : a.y0};
   T acc = T(0);
   primal_work(a, sc, sm, tl, nt, commit_only, acc);
@@ -346,6 +345,18 @@ __global__ void __launch_bounds__(kBlock, kPrimalCtasPerSm<T>) primal_step_kerne
   __shared__ double o[1];
   cta_sums<1>(v, o, red);
   if (threadIdx.x == 0) a.part_p[b] = o[0];
+}
+
+// The chunk is finished: what its evaluation, already queued behind it, needs of the state.
+__device__ __forceinline__ void end_chunk(StepState& s) {
+  s.done = 1;
+  s.eval_active = 1;
+  // the average, or the current point (src/primal_dual_hybrid_gradient_gpu.jl:635-642)
+  s.eval_current = s.numerical_error || s.count_primal == 0 || s.count_dual == 0 ? 1 : 0;
+  if (!s.eval_current) {
+    s.rcp_w_primal = 1.0 / s.sum_w_primal;
+    s.rcp_w_dual = 1.0 / s.sum_w_dual;
+  }
 }
 
 // Decision of take_step! for one attempt on the instance's state, by one thread: its chain of
@@ -365,8 +376,8 @@ __device__ __forceinline__ bool step_decision(StepState& s, double f1, double f2
   s.attempts_in_chunk += 1;
   if (interacts && (__double_as_longlong(movement) << 1) == 0) {
     s.numerical_error = 1;
-    s.done = 1;
     s.pending_commit = 0;
+    end_chunk(s);
     return false;
   }
   // positive operands and no NaN: order of the bits; else the comparisons as written
@@ -396,7 +407,7 @@ __device__ __forceinline__ bool step_decision(StepState& s, double f1, double f2
   } else {
     s.rejected += 1;
   }
-  if (s.accepted_in_chunk >= s.target_in_chunk || s.attempts_in_chunk >= s.max_attempts_in_chunk) s.done = 1;
+  if (s.accepted_in_chunk >= s.target_in_chunk || s.attempts_in_chunk >= s.max_attempts_in_chunk) end_chunk(s);
   return true;
 }
 
