@@ -310,7 +310,7 @@ struct BatchWorkspace {
   DBuf<T> y0, y1, kx0, kx1, sy, skx, ay, akx, ry, rkx;
   DBuf<StepState> st_dev;
   PinnedBuf<StepState> st_host;
-  DBuf<double> part_p, part_d, red_part_n, red_part_m, red_out;
+  DBuf<double> part_p, part_d, red_part_n, red_part_m;
   DBuf<double> rvar, rcon;   // 1 / variable and 1 / constraint rescaling (evaluation divisions)
   PinnedBuf<double> red_host;
   TilePlan<T> plan_p, plan_d;   // tiles of the packed A' and A, instance by instance
@@ -383,7 +383,6 @@ struct BatchWorkspace {
     part_d_split.alloc(2 * (size_t)std::max(plan_d.num_splits, 1));
     red_part_n.alloc((size_t)kPassNQ * B->nseg_n);
     red_part_m.alloc((size_t)kPassMQ * B->nseg_m);
-    red_out.alloc((size_t)count * kEvalStride);
     compact(std::vector<char>(count, 0));
     tr.mark("batch ws: CTA maps, graphs");
   }
@@ -461,7 +460,7 @@ struct BatchWorkspace {
       launch_step(primal_step_kernel<T>, grid_p, s, pargs(kStepNormal));
       launch_step(dual_step_kernel<T>, grid_d, s, dargs());
     }
-    cudaMemcpyAsync(st_host.p, st_dev.get(), sizeof(StepState) * count, cudaMemcpyDeviceToHost, s);
+    copy_state(st_dev.get(), st_host.p, count, s);
     CK(cudaStreamEndCapture(s, &g));
     cudaGraphExec_t ex = nullptr;
     CK(cudaGraphInstantiate(&ex, g, 0));
@@ -470,7 +469,8 @@ struct BatchWorkspace {
   }
   // the host edits the mirror only after synchronising with the work that follows
   void push_state() {
-    CK(cudaMemcpyAsync(st_dev.get(), st_host.p, sizeof(StepState) * count, cudaMemcpyHostToDevice, B->stream));
+    copy_state(st_host.p, st_dev.get(), count, B->stream);
+    ++launches;
   }
   int grid(int len) const { return std::max(1, std::min(ceil_div(len, kBlock), 4096)); }
 
@@ -482,7 +482,7 @@ struct BatchWorkspace {
   }
   // One evaluation of the instances marked in the state, as the lone solve's graph: the state, the
   // pending steps' column side beside the row pass and A' y-bar, the column pass, one read-back.
-  static constexpr int kEvaluationKernels = 5;
+  static constexpr int kEvaluationKernels = 6;
   cudaGraphExec_t capture_evaluation() {
     cudaStream_t s = B->stream;
     cudaStream_t side_stream = nullptr;
@@ -491,14 +491,14 @@ struct BatchWorkspace {
     CK(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
     CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    CK(cudaMemcpyAsync(st_dev.get(), st_host.p, sizeof(StepState) * count, cudaMemcpyHostToDevice, s));
+    copy_state(st_host.p, st_dev.get(), count, s);
     CK(cudaEventRecord(fork, s));
-    CK(cudaStreamWaitEvent(side_stream, fork, 0));
-    primal_step_kernel<T><<<grid_p, kBlock, 0, side_stream>>>(pargs(kStepCommitOnly));
-    CK(cudaEventRecord(join, side_stream));
     seg_reduce<kPassMQ, kEvalMMax>(
         false, EvalPassM<T>{B->con.get(), rcon.get(), B->ob.get(), b, y0.get(), y1.get(), kx0.get(), kx1.get(),
                             ry.get(), rkx.get(), sy.get(), skx.get(), ay.get(), akx.get(), 0, B->ineq_flag.get()});
+    CK(cudaStreamWaitEvent(side_stream, fork, 0));
+    primal_step_kernel<T><<<grid_p, kBlock, 0, side_stream>>>(pargs(kStepCommitOnly));
+    CK(cudaEventRecord(join, side_stream));
     if (B->At.num_items > 0)
       spmv_kernel<T><<<B->At.num_items, kBlock, 0, s>>>(B->At.view<T>(), ay.get(), aty.get(), B->col_inst.get(),
                                                         st_dev.get());
@@ -506,10 +506,9 @@ struct BatchWorkspace {
     seg_reduce<kPassNQ, kEvalNMax>(
         true, EvalPassN<T>{B->var.get(), rvar.get(), B->ol.get(), B->ou.get(), B->oc.get(), l, u, c, x.get(), sx.get(),
                            aty.get(), kty.get(), rx.get(), rgrad.get(), ax.get(), agrad.get(), grad.get()});
-    const SegSide sm{B->seg_m_begin.get(), red_part_m.get(), red_out.get(), B->nseg_m, kPassMQ, kEvalMMax};
-    const SegSide sn{B->seg_n_begin.get(), red_part_n.get(), red_out.get() + kEvalOutN, B->nseg_n, kPassNQ, kEvalNMax};
-    seg_finalize_kernel<<<dim3(kPassMQ + kPassNQ, count), kBlock, 0, s>>>(sm, sn, st_dev.get());
-    CK(cudaMemcpyAsync(red_host.p, red_out.get(), sizeof(double) * kEvalStride * count, cudaMemcpyDeviceToHost, s));
+    const SegSide sm{B->seg_m_begin.get(), red_part_m.get(), red_host.p, B->nseg_m, kPassMQ, kEvalMMax};
+    const SegSide sn{B->seg_n_begin.get(), red_part_n.get(), red_host.p + kEvalOutN, B->nseg_n, kPassNQ, kEvalNMax};
+    seg_finalize_kernel<<<dim3(kPassMQ + kPassNQ, count), kBlock, 0, s>>>(sm, sn, st_dev.get(), nullptr);
     cudaGraph_t g = nullptr;
     CK(cudaStreamEndCapture(s, &g));
     cudaGraphExec_t ex = nullptr;
@@ -710,7 +709,7 @@ static void run_batch(gpdhg_batch* B, BatchWorkspace<T>& W, const gpdhg_params& 
       int lv = 0;
       while (lv + 1 < kBatchLevels && (1 << lv) < max_remaining) ++lv;
       CK(cudaGraphLaunch(W.graphs[lv], s));
-      W.launches += 2 * (1 << lv);
+      W.launches += 2 * (1 << lv) + 1;
       CK(cudaStreamSynchronize(s));
       bool all_done = true;
       for (int k = 0; k < K; ++k)

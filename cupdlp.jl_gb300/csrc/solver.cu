@@ -123,7 +123,7 @@ struct Workspace {
   DBuf<T> y0, y1, kx0, kx1, sy, skx, ay, akx, ry, rkx, tmp_m;
   DBuf<StepState> st_dev;
   PinnedBuf<StepState> st_host;
-  DBuf<double> part_p, part_d, red_part_n, red_part_m, red_out;
+  DBuf<double> part_p, part_d, red_part_n, red_part_m;
   DBuf<double> rvar, rcon;   // 1 / variable and 1 / constraint rescaling (evaluation divisions)
   PinnedBuf<double> red_host;
   RestartKkt restart_kkt;
@@ -203,7 +203,6 @@ struct Workspace {
     part_d.alloc(2 * (size_t)plan_d.num_ctas);
     part_p_split.alloc(std::max(plan_p.num_splits, 1));
     part_d_split.alloc(2 * (size_t)std::max(plan_d.num_splits, 1));
-    red_out.alloc(kEvalStride);
     {
       std::vector<SegItem> it;
       std::vector<int32_t> beg;
@@ -316,46 +315,40 @@ struct Workspace {
   }
   SegSide side(bool n_side, int quantities, unsigned maxmask) {
     return SegSide{n_side ? seg_n_begin.get() : seg_m_begin.get(), n_side ? red_part_n.get() : red_part_m.get(),
-                   red_out.get() + (n_side ? kEvalOutN : 0), n_side ? nseg_n : nseg_m, quantities, maxmask};
+                   red_host.p + (n_side ? kEvalOutN : 0), n_side ? nseg_n : nseg_m, quantities, maxmask};
   }
-  // the partials of both sides reduced (a side without quantities is skipped), on their way to red_host
+  // the partials of both sides reduced (a side without quantities is skipped), into red_host
   void finish_reductions(SegSide a, SegSide b, const StepState* st) {
-    seg_finalize_kernel<<<dim3(a.quantities + b.quantities, 1), kBlock, 0, P->stream>>>(a, b, st);
+    seg_finalize_kernel<<<dim3(a.quantities + b.quantities, 1), kBlock, 0, P->stream>>>(a, b, st, st ? st_host.p : nullptr);
     CK_LAUNCH();
-    CK(cudaMemcpyAsync(red_host.p, red_out.get(), sizeof(double) * kEvalStride, cudaMemcpyDeviceToHost, P->stream));
   }
-  // One evaluation as a graph, with the state's way to the host: the accepted step still to be applied
-  // (its K'y, x and Sigma x) beside the row pass (its Sigma y and Sigma Kx, the averages y-bar and Kx-bar
-  // with their unscaled statistics, src/iteration_stats_utils_gpu.jl:447-502, and restart-scheme
-  // ingredients) and A' y-bar (the reference sums the steps' K'y with the averaging weights instead,
-  // src/saddle_point_gpu.jl:176-189; the two agree in exact arithmetic); then the column pass and
-  // one read-back of all sums. It is queued right behind the steps of its interval, whose last decision
-  // sets what it needs (end_chunk); behind steps that end short of the interval's goal it does
-  // nothing. (Launched by the host after reading the state, an interval took 12 us more, two round
-  // trips instead of one.)
+  // One evaluation as a graph, which also returns the state: the row pass (the last accepted step's
+  // Sigma y and Sigma Kx, the averages y-bar and Kx-bar with their unscaled statistics,
+  // src/iteration_stats_utils_gpu.jl:447-502, and restart-scheme ingredients), launched first since it
+  // is on the path, and that step's K'y, x and Sigma x beside it; A' y-bar (the reference sums the
+  // steps' K'y with the averaging weights instead, src/saddle_point_gpu.jl:176-189; the two agree in
+  // exact arithmetic); then the column pass and all sums. It is queued right behind the steps of its
+  // interval, whose last decision sets what it needs (end_chunk); behind steps that end short of the
+  // interval's goal it does nothing. (Launched by the host after reading the state, an interval took 12
+  // us more, two round trips instead of one.)
   static constexpr int kEvaluationKernels = 5;
   cudaGraphExec_t capture_evaluation() {
     cudaStream_t s = P->stream;
-    cudaStream_t side_stream = nullptr, copy_stream = nullptr;
-    cudaEvent_t fork = nullptr, join = nullptr, copied = nullptr;
+    cudaStream_t side_stream = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
     CK(cudaStreamCreateWithFlags(&side_stream, cudaStreamNonBlocking));
     CK(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
     CK(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
-    CK(cudaStreamCreateWithFlags(&copy_stream, cudaStreamNonBlocking));
-    CK(cudaEventCreateWithFlags(&copied, cudaEventDisableTiming));
     CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     CK(cudaEventRecord(fork, s));
-    CK(cudaStreamWaitEvent(side_stream, fork, 0));
-    CK(cudaStreamWaitEvent(copy_stream, fork, 0));
-    CK(cudaMemcpyAsync(st_host.p, st_dev.get(), sizeof(StepState), cudaMemcpyDeviceToHost, copy_stream));
-    CK(cudaEventRecord(copied, copy_stream));
-    primal_step_kernel<T><<<plan_p.num_ctas, kBlock, 0, side_stream>>>(primal_args(kStepCommitOnly));
-    CK(cudaEventRecord(join, side_stream));
     reduce<kPassMQ, kEvalMMax>(
         false,
         EvalPassM<T>{P->con.get(), rcon.get(), P->ob.get(), b, y0.get(), y1.get(), kx0.get(), kx1.get(), ry.get(),
                      rkx.get(), sy.get(), skx.get(), ay.get(), akx.get(), P->neq, nullptr},
         st_dev.get());
+    CK(cudaStreamWaitEvent(side_stream, fork, 0));
+    primal_step_kernel<T><<<plan_p.num_ctas, kBlock, 0, side_stream>>>(primal_args(kStepCommitOnly));
+    CK(cudaEventRecord(join, side_stream));
     spmv(P->At, ay.get(), tmp_n.get(), st_dev.get());
     CK(cudaStreamWaitEvent(s, join, 0));
     reduce<kPassNQ, kEvalNMax>(
@@ -364,7 +357,6 @@ struct Workspace {
                      tmp_n.get(), kty.get(), rx.get(), rgrad.get(), ax.get(), agrad.get(), grad.get()},
         st_dev.get());
     finish_reductions(side(false, kPassMQ, kEvalMMax), side(true, kPassNQ, kEvalNMax), st_dev.get());
-    CK(cudaStreamWaitEvent(s, copied, 0));
     cudaGraph_t g = nullptr;
     CK(cudaStreamEndCapture(s, &g));
     cudaGraphExec_t ex = nullptr;
@@ -372,9 +364,7 @@ struct Workspace {
     cudaGraphDestroy(g);
     cudaEventDestroy(fork);
     cudaEventDestroy(join);
-    cudaEventDestroy(copied);
     cudaStreamDestroy(side_stream);
-    cudaStreamDestroy(copy_stream);
     return ex;
   }
   void launch_restart(cudaStream_t s) {
@@ -448,7 +438,8 @@ bool run_phase(gpdhg_problem* P, Workspace<T>& W, const gpdhg_params& prm, LoopS
   // The state to the device. The mirror stays untouched until the stream has passed the copy: the
   // host edits it only after synchronising with the work that follows.
   auto push_state_async = [&]() {
-    CK(cudaMemcpyAsync(W.st_dev.get(), W.st_host.p, sizeof(StepState), cudaMemcpyHostToDevice, s));
+    copy_state(W.st_host.p, W.st_dev.get(), 1, s);
+    ++P->launches;
   };
 
   auto launch_evaluation = [&]() {
