@@ -457,8 +457,8 @@ struct BatchWorkspace {
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     for (int k = 0; k < pairs; ++k) {
-      launch_step(primal_step_kernel<T>, grid_p, s, pargs(kStepNormal));
-      launch_step(dual_step_kernel<T>, grid_d, s, dargs());
+      launch_step(primal_kernel<T>(grid_p), grid_p, s, pargs(kStepNormal));
+      launch_step(dual_kernel<T>(grid_d), grid_d, s, dargs());
     }
     copy_state(st_dev.get(), st_host.p, count, s);
     CK(cudaStreamEndCapture(s, &g));
@@ -497,7 +497,7 @@ struct BatchWorkspace {
         false, EvalPassM<T>{B->con.get(), rcon.get(), B->ob.get(), b, y0.get(), y1.get(), kx0.get(), kx1.get(),
                             ry.get(), rkx.get(), sy.get(), skx.get(), ay.get(), akx.get(), 0, B->ineq_flag.get()});
     CK(cudaStreamWaitEvent(side_stream, fork, 0));
-    primal_step_kernel<T><<<grid_p, kBlock, 0, side_stream>>>(pargs(kStepCommitOnly));
+    primal_kernel<T>(grid_p)<<<grid_p, kBlock, 0, side_stream>>>(pargs(kStepCommitOnly));
     CK(cudaEventRecord(join, side_stream));
     if (B->At.num_items > 0)
       spmv_kernel<T><<<B->At.num_items, kBlock, 0, s>>>(B->At.view<T>(), ay.get(), aty.get(), B->col_inst.get(),

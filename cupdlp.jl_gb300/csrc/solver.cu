@@ -247,8 +247,8 @@ struct Workspace {
                        dx.get(), b, y0.get(), y1.get(), kx0.get(), kx1.get(), sy.get(), skx.get(), st_dev.get(),
                        part_p.get(), part_p_split.get(), part_d.get(), part_d_split.get(), direct};
   }
-  void launch_primal(int mode, cudaStream_t s) { launch_step(primal_step_kernel<T>, plan_p.num_ctas, s, primal_args(mode)); }
-  void launch_dual(cudaStream_t s) { launch_step(dual_step_kernel<T>, plan_d.num_ctas, s, dual_args()); }
+  void launch_primal(int mode, cudaStream_t s) { launch_step(primal_kernel<T>(plan_p.num_ctas), plan_p.num_ctas, s, primal_args(mode)); }
+  void launch_dual(cudaStream_t s) { launch_step(dual_kernel<T>(plan_d.num_ctas), plan_d.num_ctas, s, dual_args()); }
 
   cudaGraphExec_t capture(int pairs) {
     cudaStream_t s = P->stream;
@@ -347,7 +347,7 @@ struct Workspace {
                      rkx.get(), sy.get(), skx.get(), ay.get(), akx.get(), P->neq, nullptr},
         st_dev.get());
     CK(cudaStreamWaitEvent(side_stream, fork, 0));
-    primal_step_kernel<T><<<plan_p.num_ctas, kBlock, 0, side_stream>>>(primal_args(kStepCommitOnly));
+    primal_kernel<T>(plan_p.num_ctas)<<<plan_p.num_ctas, kBlock, 0, side_stream>>>(primal_args(kStepCommitOnly));
     CK(cudaEventRecord(join, side_stream));
     spmv(P->At, ay.get(), tmp_n.get(), st_dev.get());
     CK(cudaStreamWaitEvent(s, join, 0));

@@ -316,8 +316,8 @@ __device__ __forceinline__ void primal_work(const PrimalArgs<T>& a, const Primal
   }
 }
 
-template <class T>
-__global__ void __launch_bounds__(kBlock, kPrimalCtasPerSm<T>) primal_step_kernel(PrimalArgs<T> a) {
+template <class T, int kCtas>
+__global__ void __launch_bounds__(kBlock, kCtas) primal_step_kernel(PrimalArgs<T> a) {
   __shared__ PrimalShared<T> sm;
   __shared__ union {   // the tiles are done with when the sums begin (cta_sums' first barrier)
     Tile tl[kTilesPerCtaMax];
@@ -648,8 +648,8 @@ __device__ __forceinline__ void step_totals(const DualArgs<T>& a, const PlanRang
   });
 }
 
-template <class T>
-__global__ void __launch_bounds__(kBlock, kDualCtasPerSm) dual_step_kernel(DualArgs<T> a) {
+template <class T, int kCtas>
+__global__ void __launch_bounds__(kBlock, kCtas) dual_step_kernel(DualArgs<T> a) {
   __shared__ DualShared<T> sm;
   __shared__ union {   // the tiles are done with when the sums begin (cta_sums' first barrier)
     Tile tl[kTilesPerCtaMax];
@@ -713,6 +713,27 @@ __global__ void __launch_bounds__(kBlock, kDualCtasPerSm) dual_step_kernel(DualA
   }
   __syncthreads();
   store_state(s, stw);
+}
+
+// The step kernels are compiled for 2, 3 and 4 resident CTAs per SM, and a launch takes the first that
+// holds all of its CTAs at once: a lane's loads in flight and its sums then have up to 128 registers
+// instead of 64 (1 per SM, 255 registers, was no faster for 128 CTAs). Per attempt, all with 4 -> as chosen: FP64 6,000 x 12,000 (128 dual
+// CTAs) 17.7 -> 15.7 us, 10,000 x 20,000 (212) 18.8 -> 16.3, 20,011 x 40,022 (425) 22.1 -> 20.3; FP32 20,000 x
+// 40,000 (204) 16.1 -> 15.9, 40,000 x 80,000 (449) 20.6 -> 18.8. One more CTA than fits is a second wave: FP64
+// 22,000 x 44,000 (467) takes 22.3 with 4 and 25.3 with 3.
+template <class T>
+using PrimalKernel = void (*)(PrimalArgs<T>);
+template <class T>
+using DualKernel = void (*)(DualArgs<T>);
+template <class T>
+inline PrimalKernel<T> primal_kernel(int ctas) {
+  static_assert(kPrimalCtasPerSm<T> == 4);
+  return ctas <= 2 * kSms ? primal_step_kernel<T, 2> : ctas <= 3 * kSms ? primal_step_kernel<T, 3> : primal_step_kernel<T, 4>;
+}
+template <class T>
+inline DualKernel<T> dual_kernel(int ctas) {
+  static_assert(kDualCtasPerSm == 4);
+  return ctas <= 2 * kSms ? dual_step_kernel<T, 2> : ctas <= 3 * kSms ? dual_step_kernel<T, 3> : dual_step_kernel<T, 4>;
 }
 
 // Launches a step kernel with programmatic dependent launch enabled (see pdl_wait).

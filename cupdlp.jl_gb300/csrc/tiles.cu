@@ -202,7 +202,7 @@ void build_tile_plan(TilePlan<T>& plan, const DeviceMatrix& M, const std::vector
     // every resident CTA slot (152 SMs x ctas_per_sm), then as many as make the instance's
     // CTAs one wave, up to kTilesPerCtaMax
     const long long nt = (long long)P.tiles.size();
-    const long long slots = 152LL * ctas_per_sm;
+    const long long slots = (long long)kSms * ctas_per_sm;
     const long long tpc = std::min<long long>(cfg.tpc_max, std::max<long long>(kTilesPerCtaMin, (nt + slots - 1) / slots));
     long long open = 0;   // tiles in the CTA being filled
     int open_code = 0;    // its tiles' kind: 0 normal, kWarpLong, else the group code

@@ -45,11 +45,12 @@ constexpr int kCtaNnz = 16384;    // longest row (piece) one CTA sums
 constexpr int kLongRound = 8;     // (column, value) loads per lane and round of a long row
 constexpr int kTilesPerCtaMin = 8;   // tiles per CTA: one per warp for small instances,
 constexpr int kTilesPerCtaMax = 96;  // up to twelve per warp for large ones
-// Resident CTAs per SM of the step kernels (their __launch_bounds__ minimum): a large
-// instance gets one CTA per resident slot of the GPU's 152 SMs, so its CTAs run as one wave
-// with no partly filled last wave.
+constexpr int kSms = 152;
+// Resident CTAs per SM of the step kernels (their __launch_bounds__ minimum) for a large instance: it
+// gets one CTA per resident slot of the GPU's SMs, so its CTAs run as one wave with no partly filled
+// last wave.
 template <class T>
-constexpr int kPrimalCtasPerSm = sizeof(T) == 8 ? 4 : 4;
+constexpr int kPrimalCtasPerSm = 4;
 constexpr int kDualCtasPerSm = 4;
 
 // Slot of lane `lane`'s j-th element in a warp tile's interleaved copy of `bytes`-byte
