@@ -401,7 +401,7 @@ struct BatchWorkspace {
     v.cta_map = map_d.get();
     return v;
   }
-  // Launches only the CTAs of instances that are not retired; re-captures the step graphs.
+  // Launches only the CTAs of instances that are not retired; the graphs are captured anew.
   std::vector<int32_t> hbeg_p, hbeg_d;  // host copies of the plans' per-instance CTA ranges
   // CTAs the step kernels would launch with the given retirements (primal plan)
   int active_ctas(const std::vector<char>& retired) const {
@@ -438,7 +438,6 @@ struct BatchWorkspace {
       if (g) cudaGraphExecDestroy(g);
       g = nullptr;
     }
-    for (int lv = 0; lv < kBatchLevels; ++lv) graphs[lv] = capture(1 << lv);
     if (evaluation) cudaGraphExecDestroy(evaluation);
     evaluation = nullptr;
     evaluation = capture_evaluation();
@@ -466,6 +465,11 @@ struct BatchWorkspace {
     CK(cudaGraphInstantiate(&ex, g, 0));
     cudaGraphDestroy(g);
     return ex;
+  }
+  // The graph of 2^lv pairs, captured at its first use (after a compaction: anew).
+  cudaGraphExec_t step_graph(int lv) {
+    if (!graphs[lv]) graphs[lv] = capture(1 << lv);
+    return graphs[lv];
   }
   // the host edits the mirror only after synchronising with the work that follows
   void push_state() {
@@ -708,7 +712,7 @@ static void run_batch(gpdhg_batch* B, BatchWorkspace<T>& W, const gpdhg_params& 
       }
       int lv = 0;
       while (lv + 1 < kBatchLevels && (1 << lv) < max_remaining) ++lv;
-      CK(cudaGraphLaunch(W.graphs[lv], s));
+      CK(cudaGraphLaunch(W.step_graph(lv), s));
       W.launches += 2 * (1 << lv) + 1;
       CK(cudaStreamSynchronize(s));
       bool all_done = true;

@@ -267,9 +267,12 @@ struct Workspace {
   }
   void build_graphs() {
     plan_cluster(cluster, plan_p, plan_d, n, m, P->stream);
-    if (!cluster.size)
-      for (int lv = 0; lv < kGraphLevels; ++lv) graphs[lv] = capture(1 << lv);
     evaluation = capture_evaluation();
+  }
+  // The graph of 2^lv pairs, captured at its first use: a solve needs two or three of the levels.
+  cudaGraphExec_t step_graph(int lv) {
+    if (!graphs[lv]) graphs[lv] = capture(1 << lv);
+    return graphs[lv];
   }
   // The same pairs launched directly with an event between every two kernels, for
   // per-kernel CUDA-event timing (events recorded as graph nodes cannot be timed).
@@ -595,11 +598,12 @@ bool run_phase(gpdhg_problem* P, Workspace<T>& W, const gpdhg_params& prm, LoopS
         CK(cudaStreamSynchronize(s));
         if (st.done) L.step_loop_sec += 1e-9 * (double)st.chunk_ns;
       } else {
+        const cudaGraphExec_t step_graph = prof ? nullptr : W.step_graph(lv);
         CK(cudaEventRecord(W.ev0, s));
         if (prof)
           W.launch_profiled(1 << lv);
         else
-          CK(cudaGraphLaunch(W.graphs[lv], s));
+          CK(cudaGraphLaunch(step_graph, s));
         P->launches += 2 * (1 << lv);
         CK(cudaEventRecord(W.ev1, s));
         launch_evaluation();
