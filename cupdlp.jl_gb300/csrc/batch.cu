@@ -320,10 +320,58 @@ struct BatchWorkspace {
   int grid_p = 0, grid_d = 0;
   cudaGraphExec_t graphs[kBatchLevels] = {}, evaluation = nullptr;
   long long launches = 0;
-  DBuf<double> caller;   // solutions in FP64, on their way to the host
-  double* caller_buffer() {
-    if (!caller.get()) caller.alloc((size_t)std::max(std::max(N, M), 1));
-    return caller.get();
+  // solutions in FP64 and in the callers' orders (columns, then rows from N on), and on the host
+  DBuf<double> caller;
+  std::unique_ptr<double[]> caller_host;
+  DBuf<int32_t> caller_order;   // a packed column's place in its instance's own order
+  void ensure_caller() {
+    if (caller.get()) return;
+    caller.alloc((size_t)N + M + 1);
+    caller_host.reset(new double[(size_t)N + M + 1]);
+    std::vector<int32_t> order((size_t)std::max(N, 1));
+    for (int k = 0; k < count; ++k) {
+      const std::vector<int32_t>& perm = B->col_perm[k];
+      const int32_t c0 = B->col_off[k];
+      for (int32_t j = 0; j < B->col_off[k + 1] - c0; ++j) order[(size_t)(c0 + j)] = c0 + (perm.empty() ? j : perm[(size_t)j]);
+    }
+    caller_order.alloc(order.size());
+    CK(cudaMemcpyAsync(caller_order.get(), order.data(), sizeof(int32_t) * order.size(), cudaMemcpyHostToDevice, B->stream));
+    CK(cudaStreamSynchronize(B->stream));   // the host order dies here
+  }
+  // The averages of the instances [k0, k1) to their callers' arrays (NULL: not wanted). Widened and put
+  // in the callers' column orders on the device, and several instances cross in one copy: copied and
+  // permuted one by one on the host, the solutions of 48 LPs (13 MB) took 3.0 ms of a 8.7 ms solve; so 2.2.
+  void fetch(int k0, int k1, double* const* primal_out, double* const* dual_out) {
+    ensure_caller();
+    cudaStream_t s = B->stream;
+    const int c0 = B->col_off[k0], cols = B->col_off[k1] - c0, r0 = B->row_off[k0], rows = B->row_off[k1] - r0;
+    auto convert = [&](const T* src, const int32_t* order, int off, int len) {
+      if (len == 0) return;
+      caller_values_kernel<T><<<grid(len), kBlock, 0, s>>>(len, src + off, order ? order + off : nullptr,
+                                                         caller.get() + (order ? 0 : (size_t)N + off));
+      CK_LAUNCH();
+      ++launches;
+    };
+    if (primal_out) convert(ax.get(), caller_order.get(), c0, cols);
+    if (dual_out) convert(ay.get(), nullptr, r0, rows);
+    auto down = [&](double* const* out, const std::vector<int32_t>& off, size_t base) {
+      if (!out) return;
+      const bool lone = k1 - k0 == 1;
+      double* dst = lone ? out[k0] : caller_host.get() + base + off[k0];
+      const size_t len = (size_t)(off[k1] - off[k0]);
+      if (dst && len) CK(cudaMemcpyAsync(dst, caller.get() + base + off[k0], sizeof(double) * len, cudaMemcpyDeviceToHost, s));
+    };
+    down(primal_out, B->col_off, 0);
+    down(dual_out, B->row_off, (size_t)N);
+    CK(cudaStreamSynchronize(s));
+    for (int k = k0; k < k1 && k1 - k0 > 1; ++k) {
+      auto hand_out = [&](double* const* out, const std::vector<int32_t>& off, size_t base) {
+        const size_t len = (size_t)(off[k + 1] - off[k]);
+        if (out && out[k] && len) std::memcpy(out[k], caller_host.get() + base + off[k], sizeof(double) * len);
+      };
+      hand_out(primal_out, B->col_off, 0);
+      hand_out(dual_out, B->row_off, (size_t)N);
+    }
   }
   DBuf<double> pow_table;
   double pow_r = -1.0, pow_g = -1.0;
@@ -576,18 +624,6 @@ static void run_batch(gpdhg_batch* B, BatchWorkspace<T>& W, const gpdhg_params& 
   }
   const auto t0 = Clock::now();
   auto elapsed = [&]() { return std::chrono::duration<double>(Clock::now() - t0).count(); };
-  // entries [off, off + len) of a packed solution to the caller's array (FP32 widened on the device)
-  auto fetch_slice = [&](const T* dsrc, double* hdst, int off, int len) {
-    if (!hdst || len == 0) return;
-    const double* src = reinterpret_cast<const double*>(dsrc) + off;
-    if constexpr (sizeof(T) == 4) {
-      caller_values_kernel<T><<<W.grid(len), kBlock, 0, s>>>(len, dsrc + off, nullptr, W.caller_buffer() + off);
-      CK_LAUNCH();
-      ++W.launches;
-      src = W.caller_buffer() + off;
-    }
-    CK(cudaMemcpyAsync(hdst, src, sizeof(double) * len, cudaMemcpyDeviceToHost, s));
-  };
   int alive = K;
   long long rounds = 0;
   while (alive > 0) {
@@ -610,7 +646,7 @@ static void run_batch(gpdhg_batch* B, BatchWorkspace<T>& W, const gpdhg_params& 
       CK(cudaGraphLaunch(W.evaluation, s));
       W.launches += W.kEvaluationKernels;
       CK(cudaStreamSynchronize(s));
-      std::vector<int> ended;   // instances terminated in this round: their solutions are on their way to the caller
+      std::vector<int> ended;   // instances terminated in this round
       for (int k = 0; k < K; ++k) {
         if (!st[k].eval_active) continue;
         st[k].pending_commit = 0;
@@ -650,12 +686,9 @@ static void run_batch(gpdhg_batch* B, BatchWorkspace<T>& W, const gpdhg_params& 
           r.accepted_steps = st[k].accepted;
           r.rejected_steps = st[k].rejected;
           r.primal_spmv_launches = st[k].primal_spmv;
-          fetch_slice(W.ax.get(), primal_out ? primal_out[k] : nullptr, B->col_off[k], B->col_off[k + 1] - B->col_off[k]);
-          fetch_slice(W.ay.get(), dual_out ? dual_out[k] : nullptr, B->row_off[k], B->row_off[k + 1] - B->row_off[k]);
           retired[k] = 1;
           st[k].done = 1;
           --alive;
-          r.kernels_launched = W.launches - launches0;
           ended.push_back(k);
           continue;
         }
@@ -672,9 +705,12 @@ static void run_batch(gpdhg_batch* B, BatchWorkspace<T>& W, const gpdhg_params& 
         any_restart = true;
       }
       if (!ended.empty()) {
-        CK(cudaStreamSynchronize(s));
+        for (size_t q = 0, e; (primal_out || dual_out) && q < ended.size(); q = e) {   // runs of neighbours
+          for (e = q + 1; e < ended.size() && ended[e] == ended[e - 1] + 1;) ++e;
+          W.fetch(ended[q], ended[e - 1] + 1, primal_out, dual_out);
+        }
         for (int k : ended) {
-          if (primal_out) to_caller_columns(B->col_perm[k], primal_out[k]);
+          results[k].kernels_launched = W.launches - launches0;
           if (on_retire) (*on_retire)(k);
         }
       }
