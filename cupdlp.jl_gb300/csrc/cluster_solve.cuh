@@ -4,7 +4,7 @@
 // Launched one by one (step_kernels.cuh), an attempt of a small LP is latency: two launches, loads of
 // descriptors, state and matrix, and chains of dependent FP64 operations (64 cycles each on GB300),
 // around a microsecond of work: 13.4 us for a 203 x 406 and 13.1 for a 1,000 x 2,000 LP in FP64,
-// against 9.4 and 9.3 here (launch and staging, 5-6 us an interval, included). Here a cluster
+// against 7.6 and 8.0 here (launch and staging, 5-6 us an interval, included). Here a cluster
 // of up to 16 CTAs keeps the LP on chip for the interval: every CTA holds its share of both
 // matrices in shared memory (columns, values and the lanes' row structure, staged once per
 // launch) and the whole of the two gathered vectors, x^ / dx and y, into which the CTAs write their

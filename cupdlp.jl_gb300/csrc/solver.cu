@@ -1,14 +1,15 @@
 // solver.cu — the restarted PDHG loop of optimize() on one GPU.
 //
 // Host/device split (src/primal_dual_hybrid_gradient_gpu.jl:457-798):
-//   * step attempts run as CUDA graphs of [primal_step_kernel, dual_step_kernel] pairs;
-//     accept/reject and the step size live on the device (StepState), so a whole
-//     evaluation interval (64 accepted steps) needs one or two host synchronisations
-//     instead of ~5 per attempt;
+//   * step attempts run as CUDA graphs of [primal_step_kernel, dual_step_kernel] pairs, a
+//     small LP's as one cluster_kernel; accept/reject and the step size live on the device
+//     (StepState);
 //   * evaluations (every termination_evaluation_frequency iterations, the first 10,
-//     and on a numerical error) run FP64 reduction kernels and read back ~40 scalars;
-//     the termination test, restart scheme and primal-weight update are the reference's
-//     scalar logic on the host;
+//     and on a numerical error) are a graph of FP64 reduction kernels queued behind the
+//     steps, so a whole evaluation interval (64 accepted steps) needs one host
+//     synchronisation (again after rejected attempts) instead of ~5 per attempt; the host
+//     reads ~40 scalars, and the termination test, restart scheme and primal-weight update
+//     are the reference's scalar logic there;
 //   * with GPDHG_PRECISION_FP32_REFINE the loop runs on FP32 copies of the matrix and
 //     iterates until the relative KKT error reaches fp64_handoff_relative_kkt (or stalls),
 //     then converts the state to FP64, recomputes K x and K'y exactly, and continues.
