@@ -4,7 +4,7 @@
 // Launched one by one (step_kernels.cuh), an attempt of a small LP is latency: two launches, loads of
 // descriptors, state and matrix, and chains of dependent FP64 operations (64 cycles each on GB300),
 // around a microsecond of work: 13.4 us for a 203 x 406 and 13.1 for a 1,000 x 2,000 LP in FP64,
-// against 7.6 and 8.0 here (launch and staging, 5-6 us an interval, included). Here a cluster
+// against 7.4 and 7.7 here (launch and staging, 5-6 us an interval, included). Here a cluster
 // of up to 16 CTAs keeps the LP on chip for the interval: every CTA holds its share of both
 // matrices in shared memory (columns, values and the lanes' row structure, staged once per
 // launch) and the whole of the two gathered vectors, x^ / dx and y, into which the CTAs write their
@@ -26,6 +26,7 @@
 
 namespace gpdhg {
 
+constexpr int kClusterThreads = kBlock + 32;   // a warp per tile, and one that decides
 constexpr int kClusterMax = 16;       // CTAs per cluster (above 8: non-portable, GB300 takes 16)
 constexpr int kClusterRounds = 4;     // plan CTAs per CTA and side, at most
 constexpr int kClusterPlanCtas = kClusterMax * kClusterRounds;
@@ -238,8 +239,14 @@ __host__ __device__ constexpr size_t cluster_vector_bytes(int cols, int rows) {
   return ((size_t)cols * sizeof(T) + 15) / 16 * 16 + ((size_t)rows * sizeof(T) + 15) / 16 * 16;
 }
 
+// What the attempt under way takes of the state, which the ninth warp keeps up one attempt behind.
+struct ClusterStep {
+  double w, tto, od;   // commit weight, tau / omega, omega tau
+  int pending, parity, done;
+};
+
 template <class T>
-__global__ void __launch_bounds__(kBlock, 1)
+__global__ void __launch_bounds__(kClusterThreads, 1)
     cluster_kernel(PrimalArgs<T> pa, DualArgs<T> da, const int32_t* p_slot, const int32_t* d_slot, const ClusterLp* lps) {
   extern __shared__ __align__(16) char dynamic[];
   __shared__ T rs_all[kBlock / 32][65];
@@ -247,6 +254,7 @@ __global__ void __launch_bounds__(kBlock, 1)
   __shared__ double total[3], factors[2];
   __shared__ int slot_begin[kClusterRounds][kClusterTiles];
   __shared__ StepState s;
+  __shared__ ClusterStep now;
   const int size = (int)cluster_size(), rank = (int)cluster_rank();
   const ClusterLp lp = lps[blockIdx.x / size];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -294,23 +302,44 @@ __global__ void __launch_bounds__(kBlock, 1)
           at_row += D[k].tiles[q].rows;
         }
   }
-  T* rs = rs_all[warp];
+  T* rs = rs_all[warp % (kBlock / 32)];
+  // The ninth warp's first lane takes the decisions. Of one, the others wait for the verdict alone;
+  // the state's upkeep and the division for tau / omega run beside the next attempt's sums (7.7 -> 7.4
+  // and 7.9 -> 7.7 us an attempt of the LPs above).
+  const bool decides = threadIdx.x == kBlock;
+  StepVerdict verdict{};
+  if (decides) {
+    now = ClusterStep{s.commit_weight, s.tto, s.omega * s.tau, s.pending_commit, s.parity, 0};
+    step_factors(&s, factors);
+  }
+  auto account = [&](bool was_pending) {
+    if (was_pending) s.primal_spmv += 1;
+    step_account(s, verdict);
+    s.tto = s.tau / s.omega;
+  };
+  bool pending_before = false;
   cluster_barrier();   // every CTA runs and has staged: its shared memory may be written
   for (int attempt = 0; attempt < kClusterAttempts; ++attempt) {
-    if (threadIdx.x == 0) step_factors(&s, factors);   // used at the attempt's end
-    const bool pending = s.pending_commit != 0;
-    const int p = s.parity;
-    const T w = (T)s.commit_weight, tto = (T)s.tto;
+    const bool pending = now.pending != 0;
+    const int p = now.parity;
+    const T w = (T)now.w;
+    if (decides && attempt > 0) {
+      account(pending_before);
+      now.tto = s.tto;
+      now.od = s.omega * s.tau;
+      step_factors(&s, factors);   // used at the attempt's end
+    }
 #pragma unroll
     for (int k = 0; k < kClusterRounds; ++k) {
-      if (warp >= P[k].count) continue;
-      const Tile t = P[k].tiles[warp];
+      const bool has = warp < P[k].count;
+      Tile t{};
+      if (has) t = P[k].tiles[warp];
       const int j = t.row_begin + lane;
       PrimalIn<T> e{};
       if (lane < t.rows) primal_load(pa, pending, false, j, e);
-      rs[lane] = e.x;   // waits for the operands: left to their first use, behind the sums, an attempt takes 1.6 us more
+      if (has) rs[lane] = e.x;   // waits for the operands: left to their first use, behind the sums, an attempt takes 1.6 us more
       T d = T(0), xv = e.x, ktyv = e.dx;
-      if (pending) {
+      if (has && pending) {
         staged_tile_sums(P[k], ys, t, warp, rs);
         if (lane < t.rows) {
           ktyv = rs[lane];
@@ -318,6 +347,12 @@ __global__ void __launch_bounds__(kBlock, 1)
         }
         __syncwarp();
       }
+      if (k == 0) {   // tau / omega is there
+        __syncwarp();
+        asm volatile("bar.sync 1, %0;" ::"n"(kClusterThreads) : "memory");
+      }
+      if (!has) continue;
+      const T tto = (T)now.tto;
       if (lane < t.rows) {
         T out;
         d = primal_candidate(pa, tto, j, xv, ktyv, e, out);
@@ -333,7 +368,7 @@ __global__ void __launch_bounds__(kBlock, 1)
     }
     cluster_barrier();
     {
-      const DualScalars<T> sc{pending, w, (T)(s.omega * s.tau), p ? da.y1 : da.y0, p ? da.y0 : da.y1,
+      const DualScalars<T> sc{pending, w, (T)now.od, p ? da.y1 : da.y0, p ? da.y0 : da.y1,
                               p ? da.kx1 : da.kx0, p ? da.kx0 : da.kx1};
 #pragma unroll
       for (int k = 0; k < kClusterRounds; ++k) {
@@ -366,7 +401,7 @@ __global__ void __launch_bounds__(kBlock, 1)
     }
     __syncthreads();
     // the plan CTAs' sums, as cta_sums adds them, one per warp; each to every CTA
-    for (int task = warp; task < 3 * kClusterRounds; task += kBlock / 32) {
+    for (int task = warp; task < 3 * kClusterRounds && warp < kBlock / 32; task += kBlock / 32) {
       const int q = task % 3, b = rank + task / 3 * size;
       if (b >= (q == 2 ? np : nd)) continue;
       const double* term = terms + task * kTerms;
@@ -401,14 +436,22 @@ __global__ void __launch_bounds__(kBlock, 1)
       }
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
-      if (pending) s.primal_spmv += 1;
-      step_decision(s, factors[0], factors[1], total[0], __fma_rn(__dmul_rn(s.half_over_omega, total[1]), total[1], total[2]));
-      s.tto = s.tau / s.omega;
+    if (decides) {
+      verdict = step_verdict(s, factors[0], factors[1], total[0],
+                             __fma_rn(__dmul_rn(s.half_over_omega, total[1]), total[1], total[2]));
+      pending_before = pending;
+      now.pending = verdict.accept ? 1 : 0;
+      if (verdict.accept) {
+        now.parity = p ^ 1;
+        now.w = s.iter_start_tau;
+      }
+      now.done = verdict.error || s.accepted_in_chunk + now.pending >= s.target_in_chunk ||
+                 s.attempts_in_chunk + 1 >= s.max_attempts_in_chunk;
     }
     __syncthreads();
-    if (s.done) break;
+    if (now.done) break;
   }
+  if (decides) account(pending_before);
   if (rank == 0) {
     if (threadIdx.x == 0) s.chunk_ns += (long long)(global_ns() - t0);
     __syncthreads();
@@ -419,7 +462,7 @@ __global__ void __launch_bounds__(kBlock, 1)
 inline void cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, int ctas, int size, size_t shared,
                            cudaStream_t s) {
   cfg.gridDim = dim3((unsigned)ctas);
-  cfg.blockDim = dim3(kBlock);
+  cfg.blockDim = dim3(kClusterThreads);
   cfg.dynamicSmemBytes = shared;
   cfg.stream = s;
   attr[0].id = cudaLaunchAttributeClusterDimension;

@@ -362,38 +362,49 @@ __device__ __forceinline__ void end_chunk(StepState& s) {
 // dependent FP64 operations, the division above all, is the attempt's serial tail, so comparisons
 // run on the integer pipe. f1 / f2 are the step-size factors
 // (1 - (k+1)^-r), (1 + (k+1)^-g) for the attempt counter after this attempt; movement is
-// 0.5 omega ||dx||^2 + 0.5 / omega ||dy||^2. Returns false on the numerical error of
-// :384-390 (terminate at the next evaluation; the step size is left as it is).
-__device__ __forceinline__ bool step_decision(StepState& s, double f1, double f2, double inter_signed, double movement) {
+// 0.5 omega ||dx||^2 + 0.5 / omega ||dy||^2. error: the numerical error of :384-390
+// (terminate at the next evaluation; the step size is left as it is).
+struct StepVerdict {
+  double limit, next;   // the step-size limit and the next step size
+  bool accept, error;
+};
+__device__ __forceinline__ StepVerdict step_verdict(const StepState& s, double f1, double f2, double inter_signed,
+                                                    double movement) {
   const long long bi = __double_as_longlong(inter_signed) & 0x7fffffffffffffffLL;
   const bool interacts = !s.constant_step && bi > 0 && bi <= 0x7ff0000000000000LL;   // |inter| > 0, not NaN
   const double tau = s.tau;
-  double limit = __longlong_as_double(0x7ff0000000000000LL);
-  if (interacts) limit = movement / __longlong_as_double(bi);
+  StepVerdict v;
+  v.limit = __longlong_as_double(0x7ff0000000000000LL);
+  if (interacts) v.limit = movement / __longlong_as_double(bi);
+  v.error = interacts && (__double_as_longlong(movement) << 1) == 0;
+  // positive operands and no NaN: order of the bits; else the comparisons as written
+  const long long bl = __double_as_longlong(v.limit), bt = __double_as_longlong(tau);
+  const bool plain = bl >= 0 && bl <= 0x7ff0000000000000LL && bt >= 0 && bt <= 0x7ff0000000000000LL;
+  v.accept = !v.error && (s.constant_step || (plain ? bt <= bl : tau <= v.limit));
+  v.next = tau;
+  if (!s.constant_step) {
+    const double first = f1 * v.limit, second = f2 * tau;
+    const long long b1 = __double_as_longlong(first), b2 = __double_as_longlong(second);
+    const bool both = b1 >= 0 && b1 <= 0x7ff0000000000000LL && b2 >= 0 && b2 <= 0x7ff0000000000000LL;
+    v.next = both ? __longlong_as_double(b1 < b2 ? b1 : b2) : jmin(first, second);
+  }
+  return v;
+}
+// The verdict entered into the state.
+__device__ __forceinline__ void step_account(StepState& s, const StepVerdict& v) {
   s.total_iters += s.constant_step ? 0 : 1;
   s.kkt_passes += 1.0;
   s.attempts_in_chunk += 1;
-  if (interacts && (__double_as_longlong(movement) << 1) == 0) {
+  if (v.error) {
     s.numerical_error = 1;
     s.pending_commit = 0;
     end_chunk(s);
-    return false;
+    return;
   }
-  // positive operands and no NaN: order of the bits; else the comparisons as written
-  const long long bl = __double_as_longlong(limit), bt = __double_as_longlong(tau);
-  const bool plain = bl >= 0 && bl <= 0x7ff0000000000000LL && bt >= 0 && bt <= 0x7ff0000000000000LL;
-  const bool accept = s.constant_step || (plain ? bt <= bl : tau <= limit);
-  double next = tau;
-  if (!s.constant_step) {
-    const double first = f1 * limit, second = f2 * tau;
-    const long long b1 = __double_as_longlong(first), b2 = __double_as_longlong(second);
-    const bool both = b1 >= 0 && b1 <= 0x7ff0000000000000LL && b2 >= 0 && b2 <= 0x7ff0000000000000LL;
-    next = both ? __longlong_as_double(b1 < b2 ? b1 : b2) : jmin(first, second);
-  }
-  s.tau = next;
-  s.last_limit = limit;
-  s.pending_commit = accept ? 1 : 0;
-  if (accept) {
+  s.tau = v.next;
+  s.last_limit = v.limit;
+  s.pending_commit = v.accept ? 1 : 0;
+  if (v.accept) {
     s.parity ^= 1;
     s.commit_weight = s.iter_start_tau;
     s.count_primal += 1;
@@ -402,12 +413,11 @@ __device__ __forceinline__ bool step_decision(StepState& s, double f1, double f2
     s.sum_w_dual += s.iter_start_tau;
     s.accepted += 1;
     s.accepted_in_chunk += 1;
-    s.iter_start_tau = next;
+    s.iter_start_tau = v.next;
   } else {
     s.rejected += 1;
   }
   if (s.accepted_in_chunk >= s.target_in_chunk || s.attempts_in_chunk >= s.max_attempts_in_chunk) end_chunk(s);
-  return true;
 }
 
 // Step-size factors of the attempt that the state (in L2 or shared memory) stands before (take_step!,
@@ -707,7 +717,8 @@ __global__ void __launch_bounds__(kBlock, kCtas) dual_step_kernel(DualArgs<T> a)
   if (threadIdx.x == 0) {
     s.arrive = 0;
     if (pending) s.primal_spmv += 1;
-    step_decision(s, factors[0], factors[1], tot[0], __fma_rn(__dmul_rn(s.half_over_omega, tot[1]), tot[1], tot[2]));
+    step_account(s, step_verdict(s, factors[0], factors[1], tot[0],
+                                 __fma_rn(__dmul_rn(s.half_over_omega, tot[1]), tot[1], tot[2])));
     s.tto = s.tau / s.omega;
   }
   __syncthreads();
