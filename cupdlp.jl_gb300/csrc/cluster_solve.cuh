@@ -48,11 +48,6 @@ __device__ __forceinline__ unsigned cluster_size() {
 // A product kept from being fused with what uses it.
 __device__ __forceinline__ double mul_rn(double a, double b) { return __dmul_rn(a, b); }
 __device__ __forceinline__ float mul_rn(float a, float b) { return __fmul_rn(a, b); }
-__device__ __forceinline__ unsigned long long global_ns() {
-  unsigned long long t;
-  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
-  return t;
-}
 
 // One side's share of one round: the tiles of a plan CTA, one per warp.
 template <class T>
@@ -261,7 +256,6 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
   load_state(da.st_mut + lp.inst, s);
   __syncthreads();
   if (s.done) return;   // the whole cluster
-  const unsigned long long t0 = global_ns();
   const int p0 = da.p_cta_begin[lp.inst], np = da.p_cta_begin[lp.inst + 1] - p0;
   const int d0 = da.plan.inst_cta_begin[lp.inst], nd = da.plan.inst_cta_begin[lp.inst + 1] - d0;
   T* xs = reinterpret_cast<T*>(dynamic);
@@ -452,9 +446,8 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
     if (now.done) break;
   }
   if (decides) account(pending_before);
+  __syncthreads();
   if (rank == 0) {
-    if (threadIdx.x == 0) s.chunk_ns += (long long)(global_ns() - t0);
-    __syncthreads();
     store_state(s, da.st_mut + lp.inst);
   }
 }

@@ -121,7 +121,7 @@ struct StepState {
   double rcp_w_primal, rcp_w_dual;
   int eval_active, eval_current, eval_restart;
   int restart;             // RestartMode of the restart kernel that follows
-  long long chunk_ns;      // device time of cluster_kernel in this chunk
+  unsigned long long chunk_start_ns, chunk_ns;   // when the chunk's state arrived, and what it took from then on
 };
 
 // ----------------------------------------------------------------------------------
@@ -132,6 +132,11 @@ __device__ __forceinline__ T warp_sum(T v) {
 #pragma unroll
   for (int o = 16; o > 0; o >>= 1) v += __shfl_down_sync(0xffffffffu, v, o);
   return v;
+}
+__device__ __forceinline__ unsigned long long global_ns() {
+  unsigned long long t;
+  asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
+  return t;
 }
 // Barrier of a thread-block cluster, for every thread of every CTA: what was written before is visible to all after.
 __device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }

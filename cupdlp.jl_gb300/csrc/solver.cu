@@ -144,7 +144,6 @@ struct Workspace {
   DBuf<double> pow_table;
   double pow_r = -1.0, pow_g = -1.0;
   const int direct = sizeof(T) == sizeof(float) ? 1 : 0;
-  cudaEvent_t ev0 = nullptr, ev1 = nullptr;
   // tile plans of A' (primal kernel) and A (dual kernel); the lone LP is a batch of one
   TilePlan<T> plan_p, plan_d;
   DBuf<double> part_p_split, part_d_split;
@@ -221,8 +220,6 @@ struct Workspace {
       red_part_n.alloc((size_t)kPassNQ * nseg_n);
       red_part_m.alloc((size_t)kPassMQ * nseg_m);
     }
-    CK(cudaEventCreate(&ev0));
-    CK(cudaEventCreate(&ev1));
     tr.mark("segments, partials");
     build_graphs();
     tr.mark("step graphs");
@@ -232,8 +229,6 @@ struct Workspace {
       if (g) cudaGraphExecDestroy(g);
     if (evaluation) cudaGraphExecDestroy(evaluation);
     for (cudaEvent_t e : pev) cudaEventDestroy(e);
-    if (ev0) cudaEventDestroy(ev0);
-    if (ev1) cudaEventDestroy(ev1);
   }
 
   const T* ycur(int parity) const { return parity ? y1.get() : y0.get(); }
@@ -251,26 +246,42 @@ struct Workspace {
   void launch_primal(int mode, cudaStream_t s) { launch_step(primal_kernel<T>(plan_p.num_ctas), plan_p.num_ctas, s, primal_args(mode)); }
   void launch_dual(cudaStream_t s) { launch_step(dual_kernel<T>(plan_d.num_ctas), plan_d.num_ctas, s, dual_args()); }
 
+  // An interval as a graph: `pairs` step attempts (the cluster kernel's, if the LP runs on one: as
+  // many as the interval takes), then its evaluation. pairs 0: the evaluation alone. (The two as
+  // graphs of their own stand 4-5 us apart.)
   cudaGraphExec_t capture(int pairs) {
     cudaStream_t s = P->stream;
+    cudaStream_t side_stream = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
+    CK(cudaStreamCreateWithFlags(&side_stream, cudaStreamNonBlocking));
+    CK(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
+    CK(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    for (int k = 0; k < pairs; ++k) {
-      launch_primal(kStepNormal, s);
-      launch_dual(s);
+    if (pairs && cluster.size) {
+      launch_cluster(cluster, s, primal_args(kStepNormal), dual_args());
+    } else {
+      for (int k = 0; k < pairs; ++k) {
+        launch_primal(kStepNormal, s);
+        launch_dual(s);
+      }
     }
-    cudaError_t e = cudaStreamEndCapture(s, &g);
-    CK(e);
+    record_evaluation(side_stream, fork, join);
+    CK(cudaStreamEndCapture(s, &g));
     cudaGraphExec_t ex = nullptr;
     CK(cudaGraphInstantiate(&ex, g, 0));
     cudaGraphDestroy(g);
+    cudaEventDestroy(fork);
+    cudaEventDestroy(join);
+    cudaStreamDestroy(side_stream);
     return ex;
   }
   void build_graphs() {
     plan_cluster(cluster, plan_p, plan_d, n, m, P->stream);
-    evaluation = capture_evaluation();
+    evaluation = capture(0);
   }
-  // The graph of 2^lv pairs, captured at its first use: a solve needs two or three of the levels.
+  // The graph of 2^lv pairs, captured at its first use: a solve needs two or three of the levels (one
+  // if it runs on a cluster).
   cudaGraphExec_t step_graph(int lv) {
     if (!graphs[lv]) graphs[lv] = capture(1 << lv);
     return graphs[lv];
@@ -326,24 +337,18 @@ struct Workspace {
     seg_finalize_kernel<<<dim3(a.quantities + b.quantities, 1), kBlock, 0, P->stream>>>(a, b, st, st ? st_host.p : nullptr);
     CK_LAUNCH();
   }
-  // One evaluation as a graph, which also returns the state: the row pass (the last accepted step's
+  // One evaluation, recorded into a graph; it also returns the state: the row pass (the last accepted step's
   // Sigma y and Sigma Kx, the averages y-bar and Kx-bar with their unscaled statistics,
   // src/iteration_stats_utils_gpu.jl:447-502, and restart-scheme ingredients), launched first since it
   // is on the path, and that step's K'y, x and Sigma x beside it; A' y-bar (the reference sums the
   // steps' K'y with the averaging weights instead, src/saddle_point_gpu.jl:176-189; the two agree in
-  // exact arithmetic); then the column pass and all sums. It is queued right behind the steps of its
+  // exact arithmetic); then the column pass and all sums. It stands right behind the steps of its
   // interval, whose last decision sets what it needs (end_chunk); behind steps that end short of the
   // interval's goal it does nothing. (Launched by the host after reading the state, an interval took 12
   // us more, two round trips instead of one.)
   static constexpr int kEvaluationKernels = 5;
-  cudaGraphExec_t capture_evaluation() {
+  void record_evaluation(cudaStream_t side_stream, cudaEvent_t fork, cudaEvent_t join) {
     cudaStream_t s = P->stream;
-    cudaStream_t side_stream = nullptr;
-    cudaEvent_t fork = nullptr, join = nullptr;
-    CK(cudaStreamCreateWithFlags(&side_stream, cudaStreamNonBlocking));
-    CK(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
-    CK(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
-    CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
     CK(cudaEventRecord(fork, s));
     reduce<kPassMQ, kEvalMMax>(
         false,
@@ -361,15 +366,6 @@ struct Workspace {
                      tmp_n.get(), kty.get(), rx.get(), rgrad.get(), ax.get(), agrad.get(), grad.get()},
         st_dev.get());
     finish_reductions(side(false, kPassMQ, kEvalMMax), side(true, kPassNQ, kEvalNMax), st_dev.get());
-    cudaGraph_t g = nullptr;
-    CK(cudaStreamEndCapture(s, &g));
-    cudaGraphExec_t ex = nullptr;
-    CK(cudaGraphInstantiate(&ex, g, 0));
-    cudaGraphDestroy(g);
-    cudaEventDestroy(fork);
-    cudaEventDestroy(join);
-    cudaStreamDestroy(side_stream);
-    return ex;
   }
   void launch_restart(cudaStream_t s) {
     const RestartArgs<T> a{st_dev.get(), nullptr, nullptr, n, m, c, ax.get(), agrad.get(), ay.get(), akx.get(),
@@ -592,27 +588,16 @@ bool run_phase(gpdhg_problem* P, Workspace<T>& W, const gpdhg_params& prm, LoopS
       const int remaining = st.target_in_chunk - st.accepted_in_chunk;
       const int attempts_before = st.attempts_in_chunk;
       const int lv = graph_level(remaining);
-      if (W.cluster.size && !prof) {
-        launch_cluster(W.cluster, s, W.primal_args(kStepNormal), W.dual_args());
-        ++P->launches;
-        launch_evaluation();
-        CK(cudaStreamSynchronize(s));
-        if (st.done) L.step_loop_sec += 1e-9 * (double)st.chunk_ns;
-      } else {
-        const cudaGraphExec_t step_graph = prof ? nullptr : W.step_graph(lv);
-        CK(cudaEventRecord(W.ev0, s));
-        if (prof)
-          W.launch_profiled(1 << lv);
-        else
-          CK(cudaGraphLaunch(step_graph, s));
+      if (prof) {
+        W.launch_profiled(1 << lv);
         P->launches += 2 * (1 << lv);
-        CK(cudaEventRecord(W.ev1, s));
         launch_evaluation();
-        CK(cudaStreamSynchronize(s));
-        float ms = 0.f;
-        CK(cudaEventElapsedTime(&ms, W.ev0, W.ev1));
-        L.step_loop_sec += 1e-3 * ms;
+      } else {
+        CK(cudaGraphLaunch(W.step_graph(W.cluster.size ? 0 : lv), s));
+        P->launches += (W.cluster.size ? 1 : 2 * (1 << lv)) + W.kEvaluationKernels;
       }
+      CK(cudaStreamSynchronize(s));
+      if (st.done) L.step_loop_sec += 1e-9 * (double)st.chunk_ns;
       if (prof) {
         const std::vector<cudaEvent_t>& ev = W.pev;
         const int did = st.attempts_in_chunk - attempts_before;

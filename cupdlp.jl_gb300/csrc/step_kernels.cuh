@@ -349,6 +349,7 @@ __global__ void __launch_bounds__(kBlock, kCtas) primal_step_kernel(PrimalArgs<T
 // The chunk is finished: what its evaluation, already queued behind it, needs of the state.
 __device__ __forceinline__ void end_chunk(StepState& s) {
   s.done = 1;
+  s.chunk_ns = global_ns() - s.chunk_start_ns;
   s.eval_active = 1;
   // the average, or the current point (src/primal_dual_hybrid_gradient_gpu.jl:635-642)
   s.eval_current = s.numerical_error || s.count_primal == 0 || s.count_dual == 0 ? 1 : 0;
