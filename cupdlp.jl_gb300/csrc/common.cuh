@@ -47,7 +47,6 @@ inline void cuda_check(cudaError_t e, const char* what, const char* file, int li
 constexpr int kBlock = 256;          // threads per CTA of every row-block kernel
 constexpr int kStageDepth = 8;                // independent (col, val) loads per thread and item
 constexpr int kStage = kBlock * kStageDepth;  // nonzeros staged per item (2048)
-constexpr int kReduceBlocks = 304;   // 2 x 152 SMs for grid-stride reductions
 
 // One CTA's share of a CSR matrix: rows [row_begin, row_end) and the schedule used for
 // them (see spmv.cuh): staged short rows reduced by groups of `group` lanes, warp-per-row
@@ -157,12 +156,6 @@ __device__ __forceinline__ void remote_store(unsigned a, double v) {
 __device__ __forceinline__ void remote_store(unsigned a, float v) {
   asm volatile("st.shared::cluster.f32 [%0], %1;" ::"r"(a), "f"(v) : "memory");
 }
-template <class T>
-__device__ __forceinline__ T warp_max(T v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v = fmax(v, __shfl_down_sync(0xffffffffu, v, o));
-  return v;
-}
 
 // Sum over the CTA; the result is valid in thread 0. `sh` holds >= 32 entries.
 template <class T>
@@ -176,20 +169,6 @@ __device__ __forceinline__ T block_sum(T v, T* sh) {
   if (wid == 0) {
     r = (lane < (int)(blockDim.x >> 5)) ? sh[lane] : T(0);
     r = warp_sum(r);
-  }
-  return r;
-}
-template <class T>
-__device__ __forceinline__ T block_max(T v, T* sh) {
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-  v = warp_max(v);
-  __syncthreads();
-  if (lane == 0) sh[wid] = v;
-  __syncthreads();
-  T r = T(0);
-  if (wid == 0) {
-    r = (lane < (int)(blockDim.x >> 5)) ? sh[lane] : T(0);
-    r = warp_max(r);
   }
   return r;
 }

@@ -611,7 +611,7 @@ bool run_phase(gpdhg_problem* P, Workspace<T>& W, const gpdhg_params& prm, LoopS
         L.kernel_launches += did;
       }
       if (st.done) break;
-      // every launch runs >= kGraphSmall attempts; 10^6 launches without the chunk's
+      // every launch runs an attempt at least; 10^6 launches without the chunk's
       // accepted steps means the step size never settles
       if (++launches > 1000000) throw Error(GPDHG_ERR_INTERNAL, "step chunk did not finish");
     }
