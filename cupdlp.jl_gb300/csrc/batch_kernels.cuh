@@ -204,7 +204,7 @@ static __global__ void copy_state_kernel(const StepState* src, StepState* dst) {
     reinterpret_cast<long long*>(dst + blockIdx.x)[threadIdx.x] =
         reinterpret_cast<const volatile long long*>(src + blockIdx.x)[threadIdx.x];
   __syncthreads();
-  if (threadIdx.x == 0) dst[blockIdx.x].chunk_start_ns = global_ns();
+  if (threadIdx.x == 0 && dst[blockIdx.x].attempts_in_chunk == 0) dst[blockIdx.x].chunk_start_ns = global_ns();
 }
 inline void copy_state(const StepState* src, StepState* dst, int count, cudaStream_t s) {
   copy_state_kernel<<<count, (kStateWords + 31) / 32 * 32, 0, s>>>(src, dst);

@@ -246,9 +246,9 @@ struct Workspace {
   void launch_primal(int mode, cudaStream_t s) { launch_step(primal_kernel<T>(plan_p.num_ctas), plan_p.num_ctas, s, primal_args(mode)); }
   void launch_dual(cudaStream_t s) { launch_step(dual_kernel<T>(plan_d.num_ctas), plan_d.num_ctas, s, dual_args()); }
 
-  // An interval as a graph: `pairs` step attempts (the cluster kernel's, if the LP runs on one: as
-  // many as the interval takes), then its evaluation. pairs 0: the evaluation alone. (The two as
-  // graphs of their own stand 4-5 us apart.)
+  // An interval as a graph: the state to the device, `pairs` step attempts (the cluster kernel's, if the LP runs on one: as
+  // many as the interval takes), then its evaluation. pairs 0: the evaluation alone. (Launches
+  // of their own stand 4-5 us apart.)
   cudaGraphExec_t capture(int pairs) {
     cudaStream_t s = P->stream;
     cudaStream_t side_stream = nullptr;
@@ -258,6 +258,7 @@ struct Workspace {
     CK(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+    copy_state(st_host.p, st_dev.get(), 1, s);
     if (pairs && cluster.size) {
       launch_cluster(cluster, s, primal_args(kStepNormal), dual_args());
     } else {
@@ -444,7 +445,7 @@ bool run_phase(gpdhg_problem* P, Workspace<T>& W, const gpdhg_params& prm, LoopS
 
   auto launch_evaluation = [&]() {
     CK(cudaGraphLaunch(W.evaluation, s));
-    P->launches += W.kEvaluationKernels;
+    P->launches += 1 + W.kEvaluationKernels;
   };
   bool evaluated = false;   // an evaluation of this iteration ran behind its steps
 
@@ -458,7 +459,6 @@ bool run_phase(gpdhg_problem* P, Workspace<T>& W, const gpdhg_params& prm, LoopS
         st.eval_restart = W.restart_kkt.valid ? 0 : 1;
         st.rcp_w_primal = st.eval_current ? 0.0 : 1.0 / st.sum_w_primal;
         st.rcp_w_dual = st.eval_current ? 0.0 : 1.0 / st.sum_w_dual;
-        push_state_async();
         launch_evaluation();
         CK(cudaStreamSynchronize(s));
       }
@@ -579,8 +579,10 @@ bool run_phase(gpdhg_problem* P, Workspace<T>& W, const gpdhg_params& prm, LoopS
     st.chunk_ns = 0;
     st.eval_active = 0;
     st.eval_restart = W.restart_kkt.valid ? 0 : 1;
-    push_state_async();
-    if (st.restart != kNoRestart) W.launch_restart(s);
+    if (st.restart != kNoRestart) {   // it reads the state ahead of the interval's graph
+      push_state_async();
+      W.launch_restart(s);
+    }
     long long launches = 0;
     const bool prof = prm.profile_kernels != 0;
     const double loop_before = L.step_loop_sec;
@@ -589,12 +591,15 @@ bool run_phase(gpdhg_problem* P, Workspace<T>& W, const gpdhg_params& prm, LoopS
       const int attempts_before = st.attempts_in_chunk;
       const int lv = graph_level(remaining);
       if (prof) {
+        // the state's two extra crossings are not counted: kernels_launched is the unprofiled solve's
+        if (!launches) copy_state(W.st_host.p, W.st_dev.get(), 1, s);
         W.launch_profiled(1 << lv);
         P->launches += 2 * (1 << lv);
+        copy_state(W.st_dev.get(), W.st_host.p, 1, s);   // the evaluation's graph starts from the mirror
         launch_evaluation();
       } else {
         CK(cudaGraphLaunch(W.step_graph(W.cluster.size ? 0 : lv), s));
-        P->launches += (W.cluster.size ? 1 : 2 * (1 << lv)) + W.kEvaluationKernels;
+        P->launches += 1 + (W.cluster.size ? 1 : 2 * (1 << lv)) + W.kEvaluationKernels;
       }
       CK(cudaStreamSynchronize(s));
       if (st.done) L.step_loop_sec += 1e-9 * (double)st.chunk_ns;
