@@ -107,7 +107,6 @@ __global__ void __launch_bounds__(kBlock / kPassCluster, 2 * kPassCluster)
     f.apply(p, i, in, acc);
     in = next;
   }
-  __syncwarp();
   cluster_wait();
 #pragma unroll
   for (int q = 0; q < Q; ++q) {

@@ -341,10 +341,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
         }
         __syncwarp();
       }
-      if (k == 0) {   // tau / omega is there
-        __syncwarp();
-        asm volatile("bar.sync 1, %0;" ::"n"(kClusterThreads) : "memory");
-      }
+      if (k == 0) named_barrier<1, kClusterThreads>();   // tau / omega is there
       if (!has) continue;
       const T tto = (T)now.tto;
       if (lane < t.rows) {
@@ -413,7 +410,6 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
       sum = __shfl_sync(0xffffffffu, sum, 0);
       if (lane < size) remote_store(remote_address(&part[q][b], lane), sum);
     }
-    __syncwarp();
     cluster_barrier();
     // the totals, as step_totals adds them, and the decision: the same in every CTA
     if (warp < 3) {

@@ -137,9 +137,24 @@ __device__ __forceinline__ unsigned long long global_ns() {
   asm volatile("mov.u64 %0, %globaltimer;" : "=l"(t));
   return t;
 }
-// Barrier of a thread-block cluster, for every thread of every CTA: what was written before is visible to all after.
-__device__ __forceinline__ void cluster_arrive() { asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory"); }
-__device__ __forceinline__ void cluster_wait() { asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory"); }
+// Barrier of a thread-block cluster, for every thread of every CTA: what was written before is
+// visible to all after. The aligned forms want the whole warp at the instruction, and the code
+// before may have left it diverged (a lane's own branch, the epilogue of the lanes that own rows):
+// each brings the warp together first.
+__device__ __forceinline__ void cluster_arrive() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;" ::: "memory");
+}
+__device__ __forceinline__ void cluster_wait() {
+  __syncwarp();
+  asm volatile("barrier.cluster.wait.acquire.aligned;" ::: "memory");
+}
+// A barrier of the CTA's first `threads` threads (whole warps) under its own number, apart from __syncthreads.
+template <int kNumber, int kThreads>
+__device__ __forceinline__ void named_barrier() {
+  __syncwarp();
+  asm volatile("bar.sync %0, %1;" ::"n"(kNumber), "n"(kThreads) : "memory");
+}
 __device__ __forceinline__ void cluster_barrier() {
   cluster_arrive();
   cluster_wait();
