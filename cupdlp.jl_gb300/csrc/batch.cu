@@ -550,17 +550,20 @@ struct BatchWorkspace {
                             ry.get(), rkx.get(), sy.get(), skx.get(), ay.get(), akx.get(), 0, B->ineq_flag.get()});
     CK(cudaStreamWaitEvent(side_stream, fork, 0));
     primal_kernel<T>(grid_p)<<<grid_p, kBlock, 0, side_stream>>>(pargs(kStepCommitOnly));
+    CK_LAUNCH();
     CK(cudaEventRecord(join, side_stream));
     if (B->At.num_items > 0)
       spmv_kernel<T><<<B->At.num_items, kBlock, 0, s>>>(B->At.view<T>(), ay.get(), aty.get(), B->col_inst.get(),
                                                         st_dev.get());
+    CK_LAUNCH();
     CK(cudaStreamWaitEvent(s, join, 0));
     seg_reduce<kPassNQ, kEvalNMax>(
         true, EvalPassN<T>{B->var.get(), rvar.get(), B->ol.get(), B->ou.get(), B->oc.get(), l, u, c, x.get(), sx.get(),
                            aty.get(), kty.get(), rx.get(), rgrad.get(), ax.get(), agrad.get(), grad.get()});
     const SegSide sm{B->seg_m_begin.get(), red_part_m.get(), red_host.p, B->nseg_m, kPassMQ, kEvalMMax};
     const SegSide sn{B->seg_n_begin.get(), red_part_n.get(), red_host.p + kEvalOutN, B->nseg_n, kPassNQ, kEvalNMax};
-    seg_finalize_kernel<<<dim3(kPassMQ + kPassNQ, count), kBlock, 0, s>>>(sm, sn, st_dev.get(), nullptr);
+    seg_finalize_kernel<<<dim3(count, kPassMQ + kPassNQ), kBlock, 0, s>>>(sm, sn, st_dev.get(), nullptr);
+    CK_LAUNCH();
     cudaGraph_t g = nullptr;
     CK(cudaStreamEndCapture(s, &g));
     cudaGraphExec_t ex = nullptr;

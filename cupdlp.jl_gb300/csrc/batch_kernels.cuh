@@ -172,19 +172,20 @@ struct SegSide {
 };
 constexpr int kEvalStride = 64;   // results per instance: rows' at 0, columns' at kEvalOutN
 constexpr int kEvalOutN = 32;
-// Grid (quantities of both sides, instances). The results go straight into the host's pinned memory,
+// Grid (instances, quantities of both sides): a grid's first dimension takes any number of
+// instances, the others 65,535 at most. The results go straight into the host's pinned memory,
 // and so does the state if mirror is given (the first CTA copies it, whether evaluated or not): behind
 // the kernel, a copy node cost 4-11 us.
 static __global__ void __launch_bounds__(kBlock) seg_finalize_kernel(SegSide a, SegSide b, const StepState* st,
                                                                         StepState* mirror) {
   __shared__ double sh[kBlock], res[1];
-  const int inst = blockIdx.y;
-  if (mirror && blockIdx.x == 0 && threadIdx.x < kStateWords)
+  const int inst = blockIdx.x;
+  if (mirror && blockIdx.y == 0 && threadIdx.x < kStateWords)
     reinterpret_cast<long long*>(mirror + inst)[threadIdx.x] = reinterpret_cast<const long long*>(st + inst)[threadIdx.x];
   if (st && !st[inst].eval_active) return;
-  const bool second = (int)blockIdx.x >= a.quantities;
+  const bool second = (int)blockIdx.y >= a.quantities;
   const SegSide& s = second ? b : a;
-  const int q = (int)blockIdx.x - (second ? a.quantities : 0);
+  const int q = (int)blockIdx.y - (second ? a.quantities : 0);
   const bool is_max = (s.maxmask >> q) & 1u;
   const double* p = s.partials + (size_t)q * s.num_items;
   const int k1 = s.inst_item_begin[inst + 1];

@@ -335,7 +335,7 @@ struct Workspace {
   }
   // the partials of both sides reduced (a side without quantities is skipped), into red_host
   void finish_reductions(SegSide a, SegSide b, const StepState* st) {
-    seg_finalize_kernel<<<dim3(a.quantities + b.quantities, 1), kBlock, 0, P->stream>>>(a, b, st, st ? st_host.p : nullptr);
+    seg_finalize_kernel<<<dim3(1, a.quantities + b.quantities), kBlock, 0, P->stream>>>(a, b, st, st ? st_host.p : nullptr);
     CK_LAUNCH();
   }
   // One evaluation, recorded into a graph; it also returns the state: the row pass (the last accepted step's
@@ -358,6 +358,7 @@ struct Workspace {
         st_dev.get());
     CK(cudaStreamWaitEvent(side_stream, fork, 0));
     primal_kernel<T>(plan_p.num_ctas)<<<plan_p.num_ctas, kBlock, 0, side_stream>>>(primal_args(kStepCommitOnly));
+    CK_LAUNCH();
     CK(cudaEventRecord(join, side_stream));
     spmv(P->At, ay.get(), tmp_n.get(), st_dev.get());
     CK(cudaStreamWaitEvent(s, join, 0));
