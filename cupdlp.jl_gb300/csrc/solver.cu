@@ -134,8 +134,10 @@ struct Workspace {
   int nseg_n = 1, nseg_m = 1;
   ClusterPlan<T> cluster;   // a small LP's intervals run on one cluster instead of as step graphs
   cudaGraphExec_t graphs[kGraphLevels] = {}, evaluation = nullptr;
-  // profiled variants: an event between every pair of kernels
-  std::vector<cudaEvent_t> pev;   // per-kernel timing events (params.profile_kernels)
+  // profiled solves (params.profile_kernels): an event between every two step kernels, and the evaluation
+  // behind steps that were launched one by one
+  std::vector<cudaEvent_t> pev;
+  cudaGraphExec_t profiled_evaluation = nullptr;
   DBuf<double> caller;   // a solution in FP64 and the caller's order, on its way to the host
   double* caller_buffer() {
     if (!caller.get()) caller.alloc((size_t)std::max(n, m));
@@ -228,6 +230,7 @@ struct Workspace {
     for (cudaGraphExec_t g : graphs)
       if (g) cudaGraphExecDestroy(g);
     if (evaluation) cudaGraphExecDestroy(evaluation);
+    if (profiled_evaluation) cudaGraphExecDestroy(profiled_evaluation);
     for (cudaEvent_t e : pev) cudaEventDestroy(e);
   }
 
@@ -246,10 +249,10 @@ struct Workspace {
   void launch_primal(int mode, cudaStream_t s) { launch_step(primal_kernel<T>(plan_p.num_ctas), plan_p.num_ctas, s, primal_args(mode)); }
   void launch_dual(cudaStream_t s) { launch_step(dual_kernel<T>(plan_d.num_ctas), plan_d.num_ctas, s, dual_args()); }
 
-  // An interval as a graph: the state to the device, `pairs` step attempts (the cluster kernel's, if the LP runs on one: as
-  // many as the interval takes), then its evaluation. pairs 0: the evaluation alone. (Launches
-  // of their own stand 4-5 us apart.)
-  cudaGraphExec_t capture(int pairs) {
+  // An interval as a graph: the state to the device (unless it is there already), `pairs` step attempts
+  // (the cluster kernel's, if the LP runs on one: as many as the interval takes), then its
+  // evaluation. pairs 0: the evaluation alone. (Launches of their own stand 4-5 us apart.)
+  cudaGraphExec_t capture(int pairs, bool with_state = true) {
     cudaStream_t s = P->stream;
     cudaStream_t side_stream = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
@@ -258,7 +261,7 @@ struct Workspace {
     CK(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
     cudaGraph_t g = nullptr;
     CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
-    copy_state(st_host.p, st_dev.get(), 1, s);
+    if (with_state) copy_state(st_host.p, st_dev.get(), 1, s);
     if (pairs && cluster.size) {
       launch_cluster(cluster, s, primal_args(kStepNormal), dual_args());
     } else {
@@ -287,15 +290,17 @@ struct Workspace {
     if (!graphs[lv]) graphs[lv] = capture(1 << lv);
     return graphs[lv];
   }
-  // The same pairs launched directly with an event between every two kernels, for
+  // The same interval with its pairs launched one by one and an event between every two kernels, for
   // per-kernel CUDA-event timing (events recorded as graph nodes cannot be timed).
   void launch_profiled(int pairs) {
-    if ((int)pev.size() < 2 * pairs + 1) {
-      const size_t old = pev.size();
-      pev.resize(2 * pairs + 1);
-      for (size_t k = old; k < pev.size(); ++k) CK(cudaEventCreate(&pev[k]));
-    }
     cudaStream_t s = P->stream;
+    if (!profiled_evaluation) profiled_evaluation = capture(0, false);
+    while ((int)pev.size() < 2 * pairs + 1) {
+      cudaEvent_t e = nullptr;
+      CK(cudaEventCreate(&e));
+      pev.push_back(e);
+    }
+    copy_state(st_host.p, st_dev.get(), 1, s);
     CK(cudaEventRecord(pev[0], s));
     for (int k = 0; k < pairs; ++k) {
       launch_primal(kStepNormal, s);
@@ -304,6 +309,8 @@ struct Workspace {
       CK(cudaEventRecord(pev[2 * k + 2], s));
     }
     CK_LAUNCH();
+    CK(cudaGraphLaunch(profiled_evaluation, s));
+    P->launches += 1 + 2 * pairs + kEvaluationKernels;
   }
   const double* ensure_pow_table(double r, double g) {
     if (pow_table.get() && r == pow_r && g == pow_g) return pow_table.get();
@@ -317,10 +324,12 @@ struct Workspace {
     return pow_table.get();
   }
 
+  // st: as recorded into an evaluation's graph, whose launch counts its kernels (as for the reductions)
   void spmv(const DeviceMatrix& M, const T* xin, T* yout, const StepState* st = nullptr) {
     if (M.num_items == 0) return;
     spmv_kernel<T><<<M.num_items, kBlock, 0, P->stream>>>(M.view<T>(), xin, yout, nullptr, st);
     CK_LAUNCH();
+    if (!st) ++P->launches;
   }
 
   // one side's pass over its segments into its partials
@@ -382,6 +391,7 @@ struct Workspace {
     const bool n_side = len == n;
     reduce<1, 0u>(n_side, DotF<T>{a, b2}, nullptr);
     finish_reductions(side(n_side, 1, 0u), SegSide{}, nullptr);
+    P->launches += 2;
     CK(cudaStreamSynchronize(P->stream));
     return red_host.p[n_side ? kEvalOutN : 0];
   }
@@ -592,12 +602,7 @@ bool run_phase(gpdhg_problem* P, Workspace<T>& W, const gpdhg_params& prm, LoopS
       const int attempts_before = st.attempts_in_chunk;
       const int lv = graph_level(remaining);
       if (prof) {
-        // the state's two extra crossings are not counted: kernels_launched is the unprofiled solve's
-        if (!launches) copy_state(W.st_host.p, W.st_dev.get(), 1, s);
         W.launch_profiled(1 << lv);
-        P->launches += 2 * (1 << lv);
-        copy_state(W.st_dev.get(), W.st_host.p, 1, s);   // the evaluation's graph starts from the mirror
-        launch_evaluation();
       } else {
         CK(cudaGraphLaunch(W.step_graph(W.cluster.size ? 0 : lv), s));
         P->launches += 1 + (W.cluster.size ? 1 : 2 * (1 << lv)) + W.kEvaluationKernels;
