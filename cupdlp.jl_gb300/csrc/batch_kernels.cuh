@@ -172,6 +172,8 @@ struct SegSide {
 };
 constexpr int kEvalStride = 64;   // results per instance: rows' at 0, columns' at kEvalOutN
 constexpr int kEvalOutN = 32;
+constexpr int kEvalSpan = 63;     // behind steps: seconds from their last decision to the end of the evaluation
+static_assert(kPassMQ <= kEvalOutN && kEvalOutN + kPassNQ <= kEvalSpan && kEvalSpan < kEvalStride, "results do not overlap");
 // Grid (instances, quantities of both sides): a grid's first dimension takes any number of
 // instances, the others 65,535 at most. The results go straight into the host's pinned memory,
 // and so does the state if mirror is given (the first CTA copies it, whether evaluated or not): behind
@@ -193,7 +195,12 @@ static __global__ void __launch_bounds__(kBlock) seg_finalize_kernel(SegSide a, 
   for (int k = s.inst_item_begin[inst] + (int)threadIdx.x; k < k1; k += kBlock)
     acc[0] = is_max ? nan_max(acc[0], p[k]) : acc[0] + p[k];
   const double r = is_max ? block_reduce_q<1, 1u>(acc, sh, res) : block_reduce_q<1, 0u>(acc, sh, res);
-  if (threadIdx.x == 0) s.out[(size_t)inst * kEvalStride + q] = r;
+  if (threadIdx.x == 0) {
+    s.out[(size_t)inst * kEvalStride + q] = r;
+    if (mirror && blockIdx.y == 0)
+      a.out[(size_t)inst * kEvalStride + kEvalSpan] =
+          1e-9 * (double)(long long)(global_ns() - st[inst].launch_start_ns - st[inst].launch_ns);
+  }
 }
 
 // ---- state ------------------------------------------------------------------------
@@ -204,7 +211,7 @@ static __global__ void copy_state_kernel(const StepState* src, StepState* dst) {
     reinterpret_cast<long long*>(dst + blockIdx.x)[threadIdx.x] =
         reinterpret_cast<const volatile long long*>(src + blockIdx.x)[threadIdx.x];
   __syncthreads();
-  if (threadIdx.x == 0 && dst[blockIdx.x].attempts_in_chunk == 0) dst[blockIdx.x].chunk_start_ns = global_ns();
+  if (threadIdx.x == 0) dst[blockIdx.x].launch_start_ns = global_ns();
 }
 inline void copy_state(const StepState* src, StepState* dst, int count, cudaStream_t s) {
   copy_state_kernel<<<count, (kStateWords + 31) / 32 * 32, 0, s>>>(src, dst);

@@ -120,7 +120,9 @@ struct StepState {
   double rcp_w_primal, rcp_w_dual;
   int eval_active, eval_current, eval_restart;
   int restart;             // RestartMode of the restart kernel that follows
-  unsigned long long chunk_start_ns, chunk_ns;   // when the chunk's state arrived, and what it took from then on
+  int launch_attempts;     // attempts_in_chunk after which the launch under way has run all of its own
+  // when the launch's state arrived, and from then to the decision of its last attempt that did work
+  unsigned long long launch_start_ns, launch_ns;
 };
 
 // ----------------------------------------------------------------------------------

@@ -349,7 +349,6 @@ __global__ void __launch_bounds__(kBlock, kCtas) primal_step_kernel(PrimalArgs<T
 // The chunk is finished: what its evaluation, already queued behind it, needs of the state.
 __device__ __forceinline__ void end_chunk(StepState& s) {
   s.done = 1;
-  s.chunk_ns = global_ns() - s.chunk_start_ns;
   s.eval_active = 1;
   // the average, or the current point (src/primal_dual_hybrid_gradient_gpu.jl:635-642)
   s.eval_current = s.numerical_error || s.count_primal == 0 || s.count_dual == 0 ? 1 : 0;
@@ -396,6 +395,9 @@ __device__ __forceinline__ void step_account(StepState& s, const StepVerdict& v)
   s.total_iters += s.constant_step ? 0 : 1;
   s.kkt_passes += 1.0;
   s.attempts_in_chunk += 1;
+  const bool ends = v.error || s.accepted_in_chunk + (v.accept ? 1 : 0) >= s.target_in_chunk ||
+                    s.attempts_in_chunk >= s.max_attempts_in_chunk;
+  if (ends || s.attempts_in_chunk == s.launch_attempts) s.launch_ns = global_ns() - s.launch_start_ns;
   if (v.error) {
     s.numerical_error = 1;
     s.pending_commit = 0;
@@ -418,7 +420,7 @@ __device__ __forceinline__ void step_account(StepState& s, const StepVerdict& v)
   } else {
     s.rejected += 1;
   }
-  if (s.accepted_in_chunk >= s.target_in_chunk || s.attempts_in_chunk >= s.max_attempts_in_chunk) end_chunk(s);
+  if (ends) end_chunk(s);
 }
 
 // Step-size factors of the attempt that the state (in L2 or shared memory) stands before (take_step!,

@@ -188,7 +188,7 @@ typedef struct gpdhg_iteration_stats {
   double cumulative_time_sec;
   double step_size;
   double primal_weight;
-  double time_spent_doing_basic_algorithm; /* method_specific_stats entry */
+  double time_spent_doing_basic_algorithm; /* method_specific_stats entry: wall time of the step attempts */
 } gpdhg_iteration_stats;
 
 typedef struct gpdhg_result {
@@ -201,7 +201,8 @@ typedef struct gpdhg_result {
   int32_t fp64_handoff_iteration;  /* iteration at which the FP64 phase began, -1 if none */
   gpdhg_iteration_stats last_iteration_stats;
   /* measurement (additions): device time of the step loop, attempts per phase */
-  double step_loop_device_sec;     /* device time of all step launches */
+  double step_loop_device_sec;     /* device time of all step launches: each from the arrival of its
+                                    * state to the decision of its last attempt (lone solves) */
   int64_t accepted_steps;
   int64_t rejected_steps;
   /* with params.profile_kernels: summed CUDA-event durations of the step kernels that did
