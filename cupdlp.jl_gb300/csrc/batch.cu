@@ -320,14 +320,15 @@ struct BatchWorkspace {
   int grid_p = 0, grid_d = 0;
   cudaGraphExec_t graphs[kBatchLevels] = {}, evaluation = nullptr;
   long long launches = 0;
-  // solutions in FP64 and in the callers' orders (columns, then rows from N on), and on the host
+  // Solutions in FP64 and in the callers' orders on their way to the host: FP32 needs room of its own
+  // (columns, then rows from N on), laid out with the workspace; FP64 columns take aty, which nothing
+  // needs between two evaluations, and FP64 rows leave from ay.
   DBuf<double> caller;
-  std::unique_ptr<double[]> caller_host;
-  DBuf<int32_t> caller_order;   // a packed column's place in its instance's own order
-  void ensure_caller() {
-    if (caller.get()) return;
-    caller.alloc((size_t)N + M + 1);
-    caller_host.reset(new double[(size_t)N + M + 1]);
+  DBuf<int32_t> caller_order;   // a packed column's place in its instance's own order; empty: its own place in all
+  std::unique_ptr<double[]> caller_host;   // runs of several instances, from the first of them on
+  void lay_out_caller() {
+    if (sizeof(T) == sizeof(float)) caller.alloc((size_t)N + M);
+    if (std::all_of(B->col_perm.begin(), B->col_perm.end(), [](const auto& p) { return p.empty(); })) return;
     std::vector<int32_t> order((size_t)std::max(N, 1));
     for (int k = 0; k < count; ++k) {
       const std::vector<int32_t>& perm = B->col_perm[k];
@@ -342,29 +343,33 @@ struct BatchWorkspace {
   // in the callers' column orders on the device, and several instances cross in one copy: copied and
   // permuted one by one on the host, the solutions of 48 LPs (13 MB) took 3.0 ms of a 8.7 ms solve; so 2.2.
   void fetch(int k0, int k1, double* const* primal_out, double* const* dual_out) {
-    ensure_caller();
     cudaStream_t s = B->stream;
     const int c0 = B->col_off[k0], cols = B->col_off[k1] - c0, r0 = B->row_off[k0], rows = B->row_off[k1] - r0;
-    auto convert = [&](const T* src, const int32_t* order, int off, int len) {
-      if (len == 0) return;
+    const bool lone = k1 - k0 == 1;
+    if (!lone && !caller_host) caller_host.reset(new double[(size_t)N + M]);
+    // src as the caller's values: in place, or through dst; the packed place of an entry is kept
+    auto convert = [&](const T* src, const int32_t* order, double* dst, int off, int len) -> const double* {
+      if (sizeof(T) == sizeof(double) && !order) return reinterpret_cast<const double*>(src);
+      if (len == 0) return dst;
       caller_values_kernel<T><<<grid(len), kBlock, 0, s>>>(len, src + off, order ? order + off : nullptr,
-                                                         caller.get() + (order ? 0 : (size_t)N + off));
+                                                         order ? dst : dst + off);
       CK_LAUNCH();
       ++launches;
+      return dst;
     };
-    if (primal_out) convert(ax.get(), caller_order.get(), c0, cols);
-    if (dual_out) convert(ay.get(), nullptr, r0, rows);
-    auto down = [&](double* const* out, const std::vector<int32_t>& off, size_t base) {
-      if (!out) return;
-      const bool lone = k1 - k0 == 1;
+    auto down = [&](double* const* out, const double* src, const std::vector<int32_t>& off, size_t base) {
       double* dst = lone ? out[k0] : caller_host.get() + base + off[k0];
       const size_t len = (size_t)(off[k1] - off[k0]);
-      if (dst && len) CK(cudaMemcpyAsync(dst, caller.get() + base + off[k0], sizeof(double) * len, cudaMemcpyDeviceToHost, s));
+      if (dst && len) CK(cudaMemcpyAsync(dst, src + off[k0], sizeof(double) * len, cudaMemcpyDeviceToHost, s));
     };
-    down(primal_out, B->col_off, 0);
-    down(dual_out, B->row_off, (size_t)N);
+    constexpr bool kNarrow = sizeof(T) == sizeof(float);
+    if (primal_out)
+      down(primal_out, convert(ax.get(), caller_order.get(), kNarrow ? caller.get() : reinterpret_cast<double*>(aty.get()),
+                               c0, cols), B->col_off, 0);
+    if (dual_out)
+      down(dual_out, convert(ay.get(), nullptr, kNarrow ? caller.get() + N : nullptr, r0, rows), B->row_off, (size_t)N);
     CK(cudaStreamSynchronize(s));
-    for (int k = k0; k < k1 && k1 - k0 > 1; ++k) {
+    for (int k = k0; k < k1 && !lone; ++k) {
       auto hand_out = [&](double* const* out, const std::vector<int32_t>& off, size_t base) {
         const size_t len = (size_t)(off[k + 1] - off[k]);
         if (out && out[k] && len) std::memcpy(out[k], caller_host.get() + base + off[k], sizeof(double) * len);
@@ -431,6 +436,7 @@ struct BatchWorkspace {
     part_d_split.alloc(2 * (size_t)std::max(plan_d.num_splits, 1));
     red_part_n.alloc((size_t)kPassNQ * B->nseg_n);
     red_part_m.alloc((size_t)kPassMQ * B->nseg_m);
+    lay_out_caller();
     compact(std::vector<char>(count, 0));
     tr.mark("batch ws: CTA maps, graphs");
   }

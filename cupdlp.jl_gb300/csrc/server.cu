@@ -96,6 +96,7 @@ double footprint_bytes(const gpdhg_lp_desc& d, const gpdhg_params& p) {
   bytes += plans * 2.0 * z * (t + 4.0) * 1.5;              // lane-interleaved tile copies
   bytes += 8.0 * (7.0 * n + 3.0 * m) + m + 4.0 * (n + m);  // FP64 vectors, flags, instance maps
   bytes += t * (13.0 * n + 11.0 * m);                      // workspace iterates
+  bytes += 4.0 * n;                                        // column order
   if (!fp64) bytes += 8.0 * (n + m);                       // the widened solution
   if (refine) bytes += 8.0 * (13.0 * n + 11.0 * m);        // the FP64 phase's workspace
   return 1.1 * bytes + (1 << 20);

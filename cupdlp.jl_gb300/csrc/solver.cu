@@ -138,10 +138,12 @@ struct Workspace {
   // behind steps that were launched one by one
   std::vector<cudaEvent_t> pev;
   cudaGraphExec_t profiled_evaluation = nullptr;
-  DBuf<double> caller;   // a solution in FP64 and the caller's order, on its way to the host
+  // A solution in FP64 and the caller's order on its way to the host: FP32 needs room of its own, laid out
+  // with the workspace; FP64 columns take tmp_n, which nothing needs after an evaluation.
+  DBuf<double> caller;
   double* caller_buffer() {
-    if (!caller.get()) caller.alloc((size_t)std::max(n, m));
-    return caller.get();
+    if constexpr (sizeof(T) == sizeof(double)) return tmp_n.get();
+    else return caller.get();
   }
   DBuf<double> pow_table;
   double pow_r = -1.0, pow_g = -1.0;
@@ -222,6 +224,7 @@ struct Workspace {
       red_part_n.alloc((size_t)kPassNQ * nseg_n);
       red_part_m.alloc((size_t)kPassMQ * nseg_m);
     }
+    if (sizeof(T) == sizeof(float)) caller.alloc(std::max(N, M));
     tr.mark("segments, partials");
     build_graphs();
     tr.mark("step graphs");
