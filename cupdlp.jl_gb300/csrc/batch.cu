@@ -507,18 +507,13 @@ struct BatchWorkspace {
   }
   cudaGraphExec_t capture(int pairs) {
     cudaStream_t s = B->stream;
-    cudaGraph_t g = nullptr;
-    CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+    GraphCapture g(s, false);
     for (int k = 0; k < pairs; ++k) {
       launch_step(primal_kernel<T>(grid_p), grid_p, s, pargs(kStepNormal));
       launch_step(dual_kernel<T>(grid_d), grid_d, s, dargs());
     }
     copy_state(st_dev.get(), st_host.p, count, s);
-    CK(cudaStreamEndCapture(s, &g));
-    cudaGraphExec_t ex = nullptr;
-    CK(cudaGraphInstantiate(&ex, g, 0));
-    cudaGraphDestroy(g);
-    return ex;
+    return g.finish();
   }
   // The graph of 2^lv pairs, captured at its first use (after a compaction: anew).
   cudaGraphExec_t step_graph(int lv) {
@@ -543,26 +538,21 @@ struct BatchWorkspace {
   static constexpr int kEvaluationKernels = 6;
   cudaGraphExec_t capture_evaluation() {
     cudaStream_t s = B->stream;
-    cudaStream_t side_stream = nullptr;
-    cudaEvent_t fork = nullptr, join = nullptr;
-    CK(cudaStreamCreateWithFlags(&side_stream, cudaStreamNonBlocking));
-    CK(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
-    CK(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
-    CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+    GraphCapture g(s);
     copy_state(st_host.p, st_dev.get(), count, s);
-    CK(cudaEventRecord(fork, s));
+    CK(cudaEventRecord(g.fork, s));
     seg_reduce<kPassMQ, kEvalMMax>(
         false, EvalPassM<T>{B->con.get(), rcon.get(), B->ob.get(), b, y0.get(), y1.get(), kx0.get(), kx1.get(),
                             ry.get(), rkx.get(), sy.get(), skx.get(), ay.get(), akx.get(), 0, B->ineq_flag.get()});
-    CK(cudaStreamWaitEvent(side_stream, fork, 0));
-    primal_kernel<T>(grid_p)<<<grid_p, kBlock, 0, side_stream>>>(pargs(kStepCommitOnly));
+    CK(cudaStreamWaitEvent(g.side, g.fork, 0));
+    primal_kernel<T>(grid_p)<<<grid_p, kBlock, 0, g.side>>>(pargs(kStepCommitOnly));
     CK_LAUNCH();
-    CK(cudaEventRecord(join, side_stream));
+    CK(cudaEventRecord(g.join, g.side));
     if (B->At.num_items > 0)
       spmv_kernel<T><<<B->At.num_items, kBlock, 0, s>>>(B->At.view<T>(), ay.get(), aty.get(), B->col_inst.get(),
                                                         st_dev.get());
     CK_LAUNCH();
-    CK(cudaStreamWaitEvent(s, join, 0));
+    CK(cudaStreamWaitEvent(s, g.join, 0));
     seg_reduce<kPassNQ, kEvalNMax>(
         true, EvalPassN<T>{B->var.get(), rvar.get(), B->ol.get(), B->ou.get(), B->oc.get(), l, u, c, x.get(), sx.get(),
                            aty.get(), kty.get(), rx.get(), rgrad.get(), ax.get(), agrad.get(), grad.get()});
@@ -570,15 +560,7 @@ struct BatchWorkspace {
     const SegSide sn{B->seg_n_begin.get(), red_part_n.get(), red_host.p + kEvalOutN, B->nseg_n, kPassNQ, kEvalNMax};
     seg_finalize_kernel<<<dim3(count, kPassMQ + kPassNQ), kBlock, 0, s>>>(sm, sn, st_dev.get(), nullptr);
     CK_LAUNCH();
-    cudaGraph_t g = nullptr;
-    CK(cudaStreamEndCapture(s, &g));
-    cudaGraphExec_t ex = nullptr;
-    CK(cudaGraphInstantiate(&ex, g, 0));
-    cudaGraphDestroy(g);
-    cudaEventDestroy(fork);
-    cudaEventDestroy(join);
-    cudaStreamDestroy(side_stream);
-    return ex;
+    return g.finish();
   }
   void launch_restart() {
     const RestartArgs<T> a{st_dev.get(), B->col_inst.get(), B->row_inst.get(), N, M, c, ax.get(), agrad.get(),

@@ -37,12 +37,64 @@ struct Error : std::runtime_error {
 
 inline void cuda_check(cudaError_t e, const char* what, const char* file, int line) {
   if (e != cudaSuccess) {
+    cudaGetLastError();   // reported here: the launch check of a later call must not find it again
     gpdhg_status s = (e == cudaErrorMemoryAllocation) ? GPDHG_ERR_OUT_OF_MEMORY : GPDHG_ERR_CUDA;
     throw Error(s, std::string(what) + ": " + cudaGetErrorString(e) + " (" + file + ":" + std::to_string(line) + ")");
   }
 }
 #define CK(call) ::gpdhg::cuda_check((call), #call, __FILE__, __LINE__)
 #define CK_LAUNCH() ::gpdhg::cuda_check(cudaGetLastError(), "kernel launch", __FILE__, __LINE__)
+
+// Records what is launched on a stream (and on `side`, a stream for work beside it, which joins it
+// through the events) into a graph. Thrown out of, it takes the stream out of capture.
+class GraphCapture {
+ public:
+  cudaStream_t side = nullptr;
+  cudaEvent_t fork = nullptr, join = nullptr;
+  explicit GraphCapture(cudaStream_t stream, bool with_side = true) : stream_(stream) {
+    try {
+      if (with_side) {
+        CK(cudaStreamCreateWithFlags(&side, cudaStreamNonBlocking));
+        CK(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
+        CK(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
+      }
+      CK(cudaStreamBeginCapture(stream_, cudaStreamCaptureModeThreadLocal));
+    } catch (...) {
+      release();
+      throw;
+    }
+    open_ = true;
+  }
+  GraphCapture(const GraphCapture&) = delete;
+  GraphCapture& operator=(const GraphCapture&) = delete;
+  ~GraphCapture() {
+    if (open_) {
+      cudaGraph_t g = nullptr;
+      if (cudaStreamEndCapture(stream_, &g) == cudaSuccess && g) cudaGraphDestroy(g);
+      cudaGetLastError();
+    }
+    release();
+  }
+  cudaGraphExec_t finish() {
+    cudaGraph_t g = nullptr;
+    open_ = false;   // whether it succeeds or not
+    CK(cudaStreamEndCapture(stream_, &g));
+    cudaGraphExec_t ex = nullptr;
+    const cudaError_t e = cudaGraphInstantiate(&ex, g, 0);
+    cudaGraphDestroy(g);
+    cuda_check(e, "cudaGraphInstantiate", __FILE__, __LINE__);
+    return ex;
+  }
+
+ private:
+  cudaStream_t stream_;
+  bool open_ = false;
+  void release() {
+    if (join) cudaEventDestroy(join);
+    if (fork) cudaEventDestroy(fork);
+    if (side) cudaStreamDestroy(side);
+  }
+};
 
 constexpr int kBlock = 256;          // threads per CTA of every row-block kernel
 constexpr int kStageDepth = 8;                // independent (col, val) loads per thread and item

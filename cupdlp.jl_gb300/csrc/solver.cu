@@ -257,13 +257,7 @@ struct Workspace {
   // evaluation. pairs 0: the evaluation alone. (Launches of their own stand 4-5 us apart.)
   cudaGraphExec_t capture(int pairs, bool with_state = true) {
     cudaStream_t s = P->stream;
-    cudaStream_t side_stream = nullptr;
-    cudaEvent_t fork = nullptr, join = nullptr;
-    CK(cudaStreamCreateWithFlags(&side_stream, cudaStreamNonBlocking));
-    CK(cudaEventCreateWithFlags(&fork, cudaEventDisableTiming));
-    CK(cudaEventCreateWithFlags(&join, cudaEventDisableTiming));
-    cudaGraph_t g = nullptr;
-    CK(cudaStreamBeginCapture(s, cudaStreamCaptureModeThreadLocal));
+    GraphCapture g(s);
     if (with_state) copy_state(st_host.p, st_dev.get(), 1, s);
     if (pairs && cluster.size) {
       launch_cluster(cluster, s, primal_args(kStepNormal), dual_args());
@@ -273,15 +267,8 @@ struct Workspace {
         launch_dual(s);
       }
     }
-    record_evaluation(side_stream, fork, join);
-    CK(cudaStreamEndCapture(s, &g));
-    cudaGraphExec_t ex = nullptr;
-    CK(cudaGraphInstantiate(&ex, g, 0));
-    cudaGraphDestroy(g);
-    cudaEventDestroy(fork);
-    cudaEventDestroy(join);
-    cudaStreamDestroy(side_stream);
-    return ex;
+    record_evaluation(g);
+    return g.finish();
   }
   void build_graphs() {
     plan_cluster(cluster, plan_p, plan_d, n, m, P->stream);
@@ -360,20 +347,20 @@ struct Workspace {
   // interval's goal it does nothing. (Launched by the host after reading the state, an interval took 12
   // us more, two round trips instead of one.)
   static constexpr int kEvaluationKernels = 5;
-  void record_evaluation(cudaStream_t side_stream, cudaEvent_t fork, cudaEvent_t join) {
+  void record_evaluation(GraphCapture& g) {
     cudaStream_t s = P->stream;
-    CK(cudaEventRecord(fork, s));
+    CK(cudaEventRecord(g.fork, s));
     reduce<kPassMQ, kEvalMMax>(
         false,
         EvalPassM<T>{P->con.get(), rcon.get(), P->ob.get(), b, y0.get(), y1.get(), kx0.get(), kx1.get(), ry.get(),
                      rkx.get(), sy.get(), skx.get(), ay.get(), akx.get(), P->neq, nullptr},
         st_dev.get());
-    CK(cudaStreamWaitEvent(side_stream, fork, 0));
-    primal_kernel<T>(plan_p.num_ctas)<<<plan_p.num_ctas, kBlock, 0, side_stream>>>(primal_args(kStepCommitOnly));
+    CK(cudaStreamWaitEvent(g.side, g.fork, 0));
+    primal_kernel<T>(plan_p.num_ctas)<<<plan_p.num_ctas, kBlock, 0, g.side>>>(primal_args(kStepCommitOnly));
     CK_LAUNCH();
-    CK(cudaEventRecord(join, side_stream));
+    CK(cudaEventRecord(g.join, g.side));
     spmv(P->At, ay.get(), tmp_n.get(), st_dev.get());
-    CK(cudaStreamWaitEvent(s, join, 0));
+    CK(cudaStreamWaitEvent(s, g.join, 0));
     reduce<kPassNQ, kEvalNMax>(
         true,
         EvalPassN<T>{P->var.get(), rvar.get(), P->ol.get(), P->ou.get(), P->oc.get(), l, u, c, x.get(), sx.get(),
