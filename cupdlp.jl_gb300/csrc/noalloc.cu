@@ -13,7 +13,7 @@
 // call is refused with GPDHG_ERR_NOT_SUPPORTED before any other CUDA call, which leaves the
 // caller's capture intact.
 //
-// Scratch: one file-scope device array (kScratchDoubles doubles, 608.3 KiB), which every GPU
+// Scratch: one file-scope device array (kScratchDoubles doubles, 89.3 KiB), which every GPU
 // that loads the library holds until the process exits. Its device address is looked up with
 // cudaGetSymbolAddress, with the device current, on the first call in each CUDA context (once
 // per device, again only if that device's context was destroyed and re-created, since the
@@ -32,14 +32,21 @@ namespace gpdhg {
 namespace {
 
 constexpr long long kNoallocMaxLength = 1LL << 24;                     // n and m at most
-constexpr int kNoallocMaxItems = 4096;                                 // CTAs per side at most
-// Elements per CTA: as few as one per thread, and one wave of 4 CTAs on each of 152 SMs for both
-// sides together on long vectors.
-int noalloc_item(long long n, long long m) {
-  return kBlock * (int)std::max<long long>(1, (n + m + kBlock * 600LL - 1) / (kBlock * 600LL));
+// Elements per CTA: as few as one per thread, and about one wave of 4 CTAs on each of 152 SMs for
+// both sides together on long vectors; either side then takes at most kNoallocCtas CTAs, for which the
+// scratch has room.
+constexpr int kNoallocCtas = 600;
+constexpr int noalloc_item(long long n, long long m) {
+  constexpr long long wave = (long long)kBlock * kNoallocCtas;
+  return kBlock * (int)std::max<long long>(1, (n + m + wave - 1) / wave);
 }
+constexpr int noalloc_items(long long len, int item) { return (int)((len + item - 1) / item); }
+static_assert(noalloc_items(kNoallocMaxLength, noalloc_item(kNoallocMaxLength, 0)) <= kNoallocCtas &&
+              noalloc_items(kNoallocMaxLength, noalloc_item(kNoallocMaxLength, 1)) <= kNoallocCtas &&
+              noalloc_items(kBlock * kNoallocCtas, noalloc_item(kBlock * kNoallocCtas, 0)) <= kNoallocCtas,
+              "the scratch holds every CTA's partials");
 constexpr int kQn = 10, kQm = 9;
-constexpr int kScratchDoubles = (kQn + kQm) * kNoallocMaxItems + 32;
+constexpr int kScratchDoubles = (kQn + kQm) * kNoallocCtas + 32;
 
 static __device__ __align__(256) double g_noalloc_scratch[kScratchDoubles];
 
@@ -127,8 +134,8 @@ __global__ void __launch_bounds__(kBlock, 4) noalloc_reduce_kernel(NoallocSide<C
   else noalloc_item_sums(m, (int)blockIdx.x - n.items, sh, res);
 }
 
-// 19 + 15 us as two CTAs over all quantities in turn, 5 us as one CTA per quantity.
-// One CTA per quantity (columns' then rows'), its items in order; rows' results from out + 16.
+// One CTA per quantity (columns' then rows'), its items in order; rows' results from out + 16. (5 us; two
+// CTAs over all quantities in turn took 19 + 15 us.)
 __global__ void __launch_bounds__(kBlock) noalloc_finalize_kernel(const double* part_n, int items_n,
                                                                   const double* part_m, int items_m, double* out) {
   __shared__ double sh[32];
@@ -217,10 +224,10 @@ void convergence_noalloc(int32_t n, int32_t m, int32_t neq, double obj_const, co
   }
   double* base = scratch_address();
   double* part_n = base;
-  double* part_m = base + (size_t)kQn * kNoallocMaxItems;
-  double* outs = base + (size_t)(kQn + kQm) * kNoallocMaxItems;
+  double* part_m = base + (size_t)kQn * kNoallocCtas;
+  double* outs = base + (size_t)(kQn + kQm) * kNoallocCtas;
   const int item = noalloc_item(n, m);
-  const int in = (n + item - 1) / item, im = (m + item - 1) / item;
+  const int in = noalloc_items(n, item), im = noalloc_items(m, item);
   noalloc_reduce_kernel<<<in + im, kBlock, 0, s>>>(
       NoallocSide<ColumnStats>{ColumnStats{l, u, c, x, aty}, n, item, in, part_n},
       NoallocSide<RowStats>{RowStats{b, y, ax, neq}, m, item, im, part_m});

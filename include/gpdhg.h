@@ -390,7 +390,7 @@ gpdhg_status gpdhg_batch_destroy(gpdhg_batch* b);
  * copies the statistics back and waits for `stream`), so a stream that is being captured into
  * a CUDA graph is refused with GPDHG_ERR_NOT_SUPPORTED before any other CUDA call, leaving the
  * capture valid. The library allocates nothing: its scratch is one fixed device array of
- * 608.3 KiB that every GPU loading the library holds until the process exits, so n and m are
+ * 89.3 KiB that every GPU loading the library holds until the process exits. n and m are
  * limited to 16,777,216 each (GPDHG_ERR_INVALID_ARGUMENT beyond). The first call in each CUDA
  * context looks the array's address up; calls that overlap on the GPU share the array and race.
  * ------------------------------------------------------------------------------- */
