@@ -27,6 +27,8 @@ problem resident in HBM. `--workload transportation` is the transportation LP (5
               by kernel with an event between every two (params.profile_kernels; events
               cannot split the kernels of a CUDA graph). traffic and
               fp64_pipe_active_pct_ncu come from the committed ncu capture (profiles/).
+              A small LP (plain), whose attempts run on one thread-block cluster: cluster_kernel,
+              from the timed solves themselves.
   cpu_baseline  the oracle (the CPU FP64 restatement of the reference loop) on the host
               cores: the same 1,000 iterations (power-law), the full solve (transportation).
   reference_gpu_equiv  the reference's loop in its own GPU form on the same GPU
@@ -332,6 +334,55 @@ def cpu_baseline(lp_problem, params, iters_cap, threads=None):
                       f"{r.solve_time_sec:.2f} s of loop, {wall:.1f} s wall)",
             "solve_sec": r.solve_time_sec, "iterations": r.iteration_count,
             "kkt_passes": r.cumulative_kkt_matrix_passes}
+
+
+def on_cluster(results):
+    """Whether the solves ran their step attempts on one thread-block cluster, an interval per launch:
+    as step kernels, every attempt launches two."""
+    return all(r.kernels_launched < 2 * (r.accepted_steps + r.rejected_steps) for r in results)
+
+
+def step_bytes(results, bm):
+    """Algorithmic bytes of the solves' attempts: (primal half, dual half)."""
+    attempts = sum(r.accepted_steps + r.rejected_steps for r in results)
+    spmv = sum(r.primal_spmv_launches for r in results)
+    return (spmv * bm["primal_commit"] + (attempts - spmv) * bm["primal_plain"],
+            attempts * bm["dual"] + spmv * bm["dual_commit_extra"])
+
+
+def cluster_roofline(results, bm, peak, peak_source):
+    """Of a small LP, from the timed solves themselves: the kernel that runs an evaluation interval
+    on one cluster, with matrix and gathered vectors in shared memory, is bound by latency."""
+    sec = sum(r.step_loop_device_sec for r in results)
+    attempts = sum(r.accepted_steps + r.rejected_steps for r in results)
+    achieved = sum(step_bytes(results, bm)) / sec / 1e9 if sec > 0 else None
+    return {"bound": "latency", "kernel": "cluster_kernel", "achieved": achieved, "peak": peak, "unit": "GB/s",
+            "frac": (achieved / peak) if achieved else None, "traffic": None, "peak_source": peak_source,
+            "us_per_attempt": sec / attempts * 1e6 if attempts else None,
+            "of": "algorithmic bytes of the timed solves' attempts / device time of their launches"}
+
+
+def step_roofline(prof, bm, peak, peak_source, workload, precision):
+    attempts = sum(r.primal_kernel_launches for r in prof)
+    spmv = sum(r.primal_spmv_launches for r in prof)
+    tp = sum(r.primal_kernel_sec for r in prof)
+    td = sum(r.dual_kernel_sec for r in prof)
+    bytes_p = spmv * bm["primal_commit"] + (attempts - spmv) * bm["primal_plain"]
+    bytes_d = attempts * bm["dual"] + spmv * bm["dual_commit_extra"]
+    dom = "primal_step_kernel" if tp >= td else "dual_step_kernel"
+    b_dom, t_dom = (bytes_p, tp) if tp >= td else (bytes_d, td)
+    achieved = (b_dom / t_dom / 1e9) if t_dom > 0 else None
+    return {"bound": "hbm", "kernel": dom, "achieved": achieved, "peak": peak, "unit": "GB/s",
+            "frac": (achieved / peak) if achieved else None, "traffic": profile_traffic(workload, dom),
+            "traffic_unit": "bytes per launch (ncu dram__bytes_read.sum + dram__bytes_write.sum, cold cache; "
+                            "profiles/" + PROFILE_FILES.get(workload, "-") + ")",
+            "peak_source": peak_source,
+            "share_of_step_time": {"primal_step_kernel": tp / max(tp + td, 1e-30),
+                                   "dual_step_kernel": td / max(tp + td, 1e-30)},
+            "bytes_per_launch": {"primal_with_commit": bm["primal_commit"], "dual": bm["dual"]},
+            "fp64_pipe_active_pct_ncu": profile_fp64_pipe(workload, dom),
+            "profiled_precision": precision,
+            "step_pair_GBps": ((bytes_p + bytes_d) / (tp + td) / 1e9) if tp + td > 0 else None}
 
 
 def reference_gpu_equiv(sq, params, repeats=2):
@@ -684,39 +735,23 @@ def run_ours(args):
     value = kkt_all / t_max
     launches = sum(r.kernels_launched for r in results)
 
-    # roofline of the dominant step kernel: the same solves again with a CUDA event between
-    # every two step kernels (launched one by one: events inside a CUDA graph cannot split
-    # its kernels), per-kernel durations summed over all attempts
-    prof, _ = timed_solves(profile=True)
     bm = bytes_model(m, n, nnz, 0 if prec == cupdlp.Precision.FP64 else 1)
-    attempts = sum(r.primal_kernel_launches for r in prof)
-    spmv = sum(r.primal_spmv_launches for r in prof)
-    tp = sum(r.primal_kernel_sec for r in prof)
-    td = sum(r.dual_kernel_sec for r in prof)
-    bytes_p = spmv * bm["primal_commit"] + (attempts - spmv) * bm["primal_plain"]
-    bytes_d = attempts * bm["dual"] + spmv * bm["dual_commit_extra"]
     peaks = {}
     try:
         peaks = json.load(open(os.path.join(REPO, "MEASURED_PEAKS.json")))
     except Exception:
         pass
     peak = float(peaks.get("hbm_gbs", 6800.0))
-    dom = "primal_step_kernel" if tp >= td else "dual_step_kernel"
-    b_dom, t_dom = (bytes_p, tp) if tp >= td else (bytes_d, td)
-    achieved = (b_dom / t_dom / 1e9) if t_dom > 0 else None
-    traffic = profile_traffic(args.workload, dom)
-    roofline = {"bound": "hbm", "kernel": dom, "achieved": achieved, "peak": peak, "unit": "GB/s",
-                "frac": (achieved / peak) if achieved else None, "traffic": traffic,
-                "traffic_unit": "bytes per launch (ncu dram__bytes_read.sum + dram__bytes_write.sum, cold cache; "
-                                "profiles/" + PROFILE_FILES.get(args.workload, "-") + ")",
-                "peak_source": "MEASURED_PEAKS.json hbm_gbs" if peaks else "fallback 6.8 TB/s",
-                "share_of_step_time": {"primal_step_kernel": tp / max(tp + td, 1e-30),
-                                       "dual_step_kernel": td / max(tp + td, 1e-30)},
-                "bytes_per_launch": {"primal_with_commit": bm["primal_commit"], "dual": bm["dual"]},
-                "fp64_pipe_active_pct_ncu": profile_fp64_pipe(args.workload, dom),
-                "profiled_precision": "FP32 (the bulk phase)" if prec == cupdlp.Precision.FP32_REFINE else
-                                      precision_name(prec),
-                "step_pair_GBps": ((bytes_p + bytes_d) / (tp + td) / 1e9) if tp + td > 0 else None}
+    peak_source = "MEASURED_PEAKS.json hbm_gbs" if peaks else "fallback 6.8 TB/s"
+    if on_cluster(results):
+        roofline = cluster_roofline(results, bm, peak, peak_source)
+    else:
+        # roofline of the dominant step kernel: the same solves again with a CUDA event between
+        # every two step kernels (launched one by one: events inside a CUDA graph cannot split
+        # its kernels), per-kernel durations summed over all attempts
+        prof, _ = timed_solves(profile=True)
+        roofline = step_roofline(prof, bm, peak, peak_source, args.workload,
+                                 "FP32 (the bulk phase)" if prec == cupdlp.Precision.FP32_REFINE else precision_name(prec))
 
     # e2e through the C ABI with host buffers (create -> solve -> copy back), every step; the
     # inputs sit in pinned host memory

@@ -139,7 +139,10 @@ typedef struct gpdhg_params {
   /* additions */
   double fp64_handoff_relative_kkt; /* FP32_REFINE: switch to FP64 below this relative KKT error */
   int32_t fp64_handoff_stall_evaluations; /* FP32_REFINE: or after this many evaluations without progress */
-  int32_t profile_kernels;         /* time every step kernel with CUDA events (result.*_kernel_sec) */
+  int32_t profile_kernels;         /* time every step kernel with CUDA events (result.*_kernel_sec). The
+                                    * steps are launched one by one then, also those of a small LP,
+                                    * which otherwise take one kernel per evaluation interval
+                                    * (cluster_kernel): the same bits, other times */
   double reserved[6];
 } gpdhg_params;
 
@@ -206,7 +209,8 @@ typedef struct gpdhg_result {
   int64_t accepted_steps;
   int64_t rejected_steps;
   /* with params.profile_kernels: summed CUDA-event durations of the step kernels that did
-   * work, and how many primal launches also ran the A'y product of a commit */
+   * work (0 without it), how many of each there were, and (always) how many attempts also ran
+   * the A'y product of a commit */
   double primal_kernel_sec;
   double dual_kernel_sec;
   int64_t primal_kernel_launches;
