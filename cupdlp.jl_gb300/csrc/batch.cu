@@ -270,8 +270,6 @@ void batch_init(gpdhg_batch* B, int32_t count, const gpdhg_lp_desc* descs) {
   B->At.items.alloc(std::max<size_t>(t_items.size(), 1));
   if (!t_items.empty())
     CK(cudaMemcpyAsync(B->At.items.get(), t_items.data(), sizeof(RowItem) * t_items.size(), cudaMemcpyHostToDevice, s));
-  up_i(B->row_off_d, B->row_off);
-  up_i(B->neq_d, B->neq);
   up_d(B->l, l); up_d(B->u, u); up_d(B->c, c); up_d(B->b, b);
   up_d(B->ol, ol); up_d(B->ou, ou); up_d(B->oc, oc); up_d(B->ob, ob);
   up_d(B->con, con); up_d(B->var, var);

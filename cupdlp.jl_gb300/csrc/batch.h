@@ -34,7 +34,6 @@ struct gpdhg_batch {
   std::vector<double> amax, norm_b, norm_c;
   std::vector<std::vector<int32_t>> col_perm;  // per instance: choose_column_order's order
   gpdhg::DeviceMatrix A, At;                   // block-diagonal CSR of A and A'
-  gpdhg::DBuf<int32_t> row_off_d, neq_d;
   gpdhg::DBuf<double> l, u, c, b, ol, ou, oc, ob, con, var;
   gpdhg::DBuf<uint8_t> ineq_flag;              // per packed row: a '>=' row
   gpdhg::DBuf<int32_t> col_inst, row_inst;     // instance of each packed column / row

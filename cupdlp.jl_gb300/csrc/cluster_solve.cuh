@@ -55,7 +55,7 @@ struct ClusterSide {
   T* val;
   unsigned long long* rows;   // 32 per tile: where the sum after each of the lane's elements goes (8
                               // bits): the row that ends there, 33 + lane if it began in an earlier lane, else 32
-  int32_t* col;               // local columns
+  int32_t* col;
   unsigned* info;             // 32 per tile: the lane's RunInfo
   Tile* tiles;
   int count;
@@ -87,27 +87,20 @@ struct RunInfo {
   static constexpr int kCountShift = 12, kSpanShift = 16, kRowShift = 24;
 };
 
-// Copies a plan CTA's tiles from `tile` on, with columns counted from col0; the caller synchronises.
+// Copies a plan CTA's tiles from `tile` on; the caller synchronises.
 template <class T>
 __device__ __forceinline__ void stage_cluster_side(const ClusterSide<T>& s, const TileView<T>& plan,
-                                                   const int32_t* row_ptr, int tile, int slots, int col0) {
+                                                   const int32_t* row_ptr, int tile, int slots) {
   const int* src = reinterpret_cast<const int*>(plan.tiles + tile);
   int* dst = reinterpret_cast<int*>(s.tiles);
-  for (int k = threadIdx.x; k < s.count * (int)(sizeof(Tile) / 4); k += kBlock) dst[k] = src[k];
+  for (int k = threadIdx.x; k < s.count * (int)(sizeof(Tile) / 4); k += kClusterThreads) dst[k] = src[k];
   // slots come in multiples of 32 from a multiple of 32, so both copies go in 16-byte pieces
   const int4* vs = reinterpret_cast<const int4*>(plan.ival + s.slot0);
   int4* vd = reinterpret_cast<int4*>(s.val);
-  for (int k = threadIdx.x; k < slots * (int)sizeof(T) / 16; k += kBlock) vd[k] = vs[k];
+  for (int k = threadIdx.x; k < slots * (int)sizeof(T) / 16; k += kClusterThreads) vd[k] = vs[k];
   const int4* cs = reinterpret_cast<const int4*>(plan.icol + s.slot0);
   int4* cd = reinterpret_cast<int4*>(s.col);
-  for (int k = threadIdx.x; k < slots / 4; k += kBlock) {
-    int4 c = cs[k];
-    c.x -= col0;   // a padding slot's column may turn negative: it is never gathered
-    c.y -= col0;
-    c.z -= col0;
-    c.w -= col0;
-    cd[k] = c;
-  }
+  for (int k = threadIdx.x; k < slots / 4; k += kClusterThreads) cd[k] = cs[k];
   const int q = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (q >= s.count) return;
   const Tile& t = plan.tiles[tile + q];
@@ -222,10 +215,6 @@ __device__ __forceinline__ void staged_tile_sums(const ClusterSide<T>& s, const 
   __syncwarp();
 }
 
-// The LP of one cluster: its instance and its columns and rows in the packed numbering.
-struct ClusterLp {
-  int32_t inst, col0, cols, row0, rows;
-};
 // Dynamic shared memory of a CTA: both vectors, the rows' terms of its rounds' sums, its tiles.
 template <class T>
 constexpr int kClusterTerms = sizeof(T) == 8 ? kBlock : kBlock / 32;   // per round and sum
@@ -242,7 +231,7 @@ struct ClusterStep {
 
 template <class T>
 __global__ void __launch_bounds__(kClusterThreads, 1)
-    cluster_kernel(PrimalArgs<T> pa, DualArgs<T> da, const int32_t* p_slot, const int32_t* d_slot, const ClusterLp* lps) {
+    cluster_kernel(PrimalArgs<T> pa, DualArgs<T> da, const int32_t* p_slot, const int32_t* d_slot, int cols, int rows) {
   extern __shared__ __align__(16) char dynamic[];
   __shared__ T rs_all[kBlock / 32][65];
   __shared__ double part[3][kClusterPlanCtas];   // every plan CTA's sums: dy . K dx, ||dy||^2, ||dx||^2
@@ -251,16 +240,14 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
   __shared__ StepState s;
   __shared__ ClusterStep now;
   const int size = (int)cluster_size(), rank = (int)cluster_rank();
-  const ClusterLp lp = lps[blockIdx.x / size];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  load_state(da.st_mut + lp.inst, s);
+  load_state(da.st_mut, s);
   __syncthreads();
   if (s.done) return;   // the whole cluster
-  const int p0 = da.p_cta_begin[lp.inst], np = da.p_cta_begin[lp.inst + 1] - p0;
-  const int d0 = da.plan.inst_cta_begin[lp.inst], nd = da.plan.inst_cta_begin[lp.inst + 1] - d0;
+  const int np = da.p_cta_begin[1], nd = da.plan.inst_cta_begin[1];   // plan CTAs of both sides
   T* xs = reinterpret_cast<T*>(dynamic);
-  T* ys = reinterpret_cast<T*>(dynamic + cluster_vector_bytes<T>(lp.cols, 0));
-  char* at = dynamic + cluster_vector_bytes<T>(lp.cols, lp.rows);
+  T* ys = reinterpret_cast<T*>(dynamic + cluster_vector_bytes<T>(cols, 0));
+  char* at = dynamic + cluster_vector_bytes<T>(cols, rows);
   constexpr int kTerms = kClusterTerms<T>;
   double* terms = reinterpret_cast<double*>(at);   // [round][sum][kTerms]
   at += sizeof(double) * kClusterRounds * 3 * kTerms;
@@ -270,21 +257,21 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
     const int b = rank + k * size;
     P[k].count = D[k].count = 0;
     if (b < np) {
-      const int tile = pa.plan.cta_tile_begin[p0 + b], slots = p_slot[p0 + b + 1] - p_slot[p0 + b];
-      P[k] = cluster_side<T>(at, pa.plan.cta_tile_begin[p0 + b + 1] - tile, slots, p_slot[p0 + b]);
-      stage_cluster_side(P[k], pa.plan, pa.At.row_ptr, tile, slots, lp.row0);
+      const int tile = pa.plan.cta_tile_begin[b], slots = p_slot[b + 1] - p_slot[b];
+      P[k] = cluster_side<T>(at, pa.plan.cta_tile_begin[b + 1] - tile, slots, p_slot[b]);
+      stage_cluster_side(P[k], pa.plan, pa.At.row_ptr, tile, slots);
       at += cluster_side_bytes(slots, sizeof(T));
     }
     if (b < nd) {
-      const int tile = da.plan.cta_tile_begin[d0 + b], slots = d_slot[d0 + b + 1] - d_slot[d0 + b];
-      D[k] = cluster_side<T>(at, da.plan.cta_tile_begin[d0 + b + 1] - tile, slots, d_slot[d0 + b]);
-      stage_cluster_side(D[k], da.plan, da.A.row_ptr, tile, slots, lp.col0);
+      const int tile = da.plan.cta_tile_begin[b], slots = d_slot[b + 1] - d_slot[b];
+      D[k] = cluster_side<T>(at, da.plan.cta_tile_begin[b + 1] - tile, slots, d_slot[b]);
+      stage_cluster_side(D[k], da.plan, da.A.row_ptr, tile, slots);
       at += cluster_side_bytes(slots, sizeof(T));
     }
   }
-  const T* y_now = (s.parity ? da.y1 : da.y0) + lp.row0;
-  for (int i = threadIdx.x; i < lp.rows; i += kBlock) ys[i] = y_now[i];
-  for (int i = threadIdx.x; i < kClusterRounds * 3 * kTerms; i += kBlock) terms[i] = 0.0;
+  const T* y_now = s.parity ? da.y1 : da.y0;
+  for (int i = threadIdx.x; i < rows; i += kClusterThreads) ys[i] = y_now[i];
+  for (int i = threadIdx.x; i < kClusterRounds * 3 * kTerms; i += kClusterThreads) terms[i] = 0.0;
   __syncthreads();
   if (threadIdx.x < kClusterRounds) {   // a row's place among the plan CTA's rows
     int at_row = 0;
@@ -347,7 +334,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
       if (lane < t.rows) {
         T out;
         d = primal_candidate(pa, tto, j, xv, ktyv, e, out);
-        for (int r = 0; r < size; ++r) remote_store(remote_address(xs + (j - lp.col0), r), out);
+        for (int r = 0; r < size; ++r) remote_store(remote_address(xs + j, r), out);
       }
       double* term = terms + (3 * k + 2) * kTerms;
       if constexpr (sizeof(T) == 8) {
@@ -372,7 +359,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
         T kdx = T(0), d = T(0);
         if (lane < t.rows) {
           const T out = dual_row(da, sc, i, i >= t.aux, rs[lane], e, kdx, d);
-          for (int r = 0; r < size; ++r) remote_store(remote_address(ys + (i - lp.row0), r), out);
+          for (int r = 0; r < size; ++r) remote_store(remote_address(ys + i, r), out);
         }
         __syncwarp();
         double* term = terms + 3 * k * kTerms;
@@ -444,7 +431,7 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
   if (decides) account(pending_before);
   __syncthreads();
   if (rank == 0) {
-    store_state(s, da.st_mut + lp.inst);
+    store_state(s, da.st_mut);
   }
 }
 
@@ -465,10 +452,9 @@ inline void cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, i
 // How an LP's intervals run on a cluster: its CTAs (0: they run as graphs of the step kernels).
 template <class T>
 struct ClusterPlan {
-  int size = 0;
+  int size = 0, cols = 0, rows = 0;
   size_t shared = 0;
   DBuf<int32_t> p_slot, d_slot;   // first slot of each plan CTA (CTAs + 1)
-  DBuf<ClusterLp> lp;
 };
 
 // First slot of every plan CTA (CTAs + 1).
@@ -517,8 +503,8 @@ void plan_cluster(ClusterPlan<T>& plan, const TilePlan<T>& p, const TilePlan<T>&
   };
   up(plan.p_slot, ps.data(), ps.size());
   up(plan.d_slot, ds.data(), ds.size());
-  const ClusterLp lp{0, 0, n, 0, m};
-  up(plan.lp, &lp, 1);
+  plan.cols = n;
+  plan.rows = m;
   CK(cudaStreamSynchronize(s));   // the host arrays die here
 }
 
@@ -528,7 +514,7 @@ void launch_cluster(const ClusterPlan<T>& plan, cudaStream_t s, const PrimalArgs
   cudaLaunchAttribute attr[1];
   cluster_config(cfg, attr, plan.size, plan.size, plan.shared, s);
   CK(cudaLaunchKernelEx(&cfg, cluster_kernel<T>, pa, da, (const int32_t*)plan.p_slot.get(),
-                        (const int32_t*)plan.d_slot.get(), (const ClusterLp*)plan.lp.get()));
+                        (const int32_t*)plan.d_slot.get(), plan.cols, plan.rows));
 }
 
 }  // namespace gpdhg
