@@ -163,7 +163,8 @@ __device__ __forceinline__ void staged_run(const U* base, int e_log2, U* d) {
 }
 
 // Row sums of the warp's tile q into rs, gathered from x (shared memory): the sums of tile_sums (same
-// elements per lane, order and scan), with the walk over rows read from the staged structure and free of branches (rs: 65 entries).
+// elements per lane, order and scan), with the walk over rows read from the staged structure and free of
+// branches (rs: 65 entries).
 template <class T>
 __device__ __forceinline__ void staged_tile_sums(const ClusterSide<T>& s, const T* x, const Tile& t, int q, T* rs) {
   constexpr int kEMax = TileTraits<T>::kEMax;
@@ -318,7 +319,8 @@ __global__ void __launch_bounds__(kClusterThreads, 1)
       const int j = t.row_begin + lane;
       PrimalIn<T> e{};
       if (lane < t.rows) primal_load(pa, pending, false, j, e);
-      if (has) rs[lane] = e.x;   // waits for the operands: left to their first use, behind the sums, an attempt takes 1.6 us more
+      // waits for the operands: left to their first use, behind the sums, an attempt takes 1.6 us more
+      if (has) rs[lane] = e.x;
       T d = T(0), xv = e.x, ktyv = e.dx;
       if (has && pending) {
         staged_tile_sums(P[k], ys, t, warp, rs);

@@ -5,7 +5,7 @@
 // (src/iteration_stats_utils_gpu.jl:23-372, src/saddle_point_gpu.jl:250-278). Here every
 // statistic of one evaluation is accumulated in FP64 in a single pass per side (n columns,
 // m rows) over fixed segments (batch_kernels.cuh), into per-segment partials that one
-// finalize CTA per instance reduces in a fixed order; the host reads back one small array.
+// finalize CTA per instance and quantity reduces in a fixed order, into the host's memory.
 // Comparisons, maxima and sign tests run on the integer pipe (bit patterns), so the FP64
 // pipe only does the arithmetic itself.
 #pragma once

@@ -13,7 +13,7 @@ namespace gpdhg {
 
 std::vector<RowItem> build_row_items(const int32_t* rp, int32_t nrows) {
   // Rows with more than kCtaRow nonzeros get a CTA each (streamed, 8 loads per thread in
-  // flight). The other rows are packed in order while their nonzeros fit the stage and there
+  // flight) unless they stand in a run (below). The other rows are packed in order while their nonzeros fit the stage and there
   // are at most kBlock of them, whatever their lengths (splitting by length would fragment a
   // power-law matrix into thousands of tiny items); such an item of at most 8 rows averaging
   // >= 64 nonzeros runs warp-per-row, any other is staged, with the largest power-of-two lane

@@ -710,10 +710,10 @@ __global__ void __launch_bounds__(kBlock, kCtas) dual_step_kernel(DualArgs<T> a)
   __syncthreads();
   if (!is_last) return;
   // The instance's last CTA: all CTAs' sums in one round of loads, the step-size factors by a warp
-  // that adds none, then thread 0 takes the decision. This tail is on every attempt's path (3-4 us
-  // of a 13 us attempt of a small LP): with the primal sum and the decision's inputs formed by the
-  // instance's first CTA after its own work, sums by one warp and the state and ranges loaded here
-  // it took more than twice as long.
+  // that adds none, then thread 0 takes the decision. This tail is on every attempt's path (3-4 us of
+  // the 13 us that an attempt of a 203 x 406 LP takes as step kernels): with the primal sum and the
+  // decision's inputs formed by the instance's first CTA after its own work, sums by one warp and the
+  // state and ranges loaded here it took more than twice as long.
   __shared__ double factors[2];
   if (threadIdx.x == 32 * (kBlock / 32 - 1)) step_factors(&s, factors);
   step_totals(a, range, s, tot, red);
@@ -730,10 +730,12 @@ __global__ void __launch_bounds__(kBlock, kCtas) dual_step_kernel(DualArgs<T> a)
 
 // The step kernels are compiled for 2, 3 and 4 resident CTAs per SM, and a launch takes the first that
 // holds all of its CTAs at once: a lane's loads in flight and its sums then have up to 128 registers
-// instead of 64 (1 per SM, 255 registers, was no faster for 128 CTAs). Per attempt, all with 4 -> as chosen: FP64 6,000 x 12,000 (128 dual
-// CTAs) 17.7 -> 15.7 us, 10,000 x 20,000 (212) 18.8 -> 16.3, 20,011 x 40,022 (425) 22.1 -> 20.3; FP32 20,000 x
-// 40,000 (204) 16.1 -> 15.9, 40,000 x 80,000 (449) 20.6 -> 18.8. One more CTA than fits is a second wave: FP64
-// 22,000 x 44,000 (467) takes 22.3 with 4 and 25.3 with 3.
+// instead of 64 (1 per SM, 255 registers, was no faster for 128 CTAs). Per attempt, all with 4 -> as
+// chosen: FP64 6,000 x 12,000 (128 dual CTAs) 17.7 -> 15.7 us, 10,000 x 20,000 (212) 18.8 -> 16.3,
+// 20,011 x 40,022 (425) 22.1 -> 20.3; FP32 20,000 x 40,000 (204) 16.1 -> 15.9, 40,000 x 80,000 (449)
+// 20.6 -> 18.8. One more CTA than fits is a second wave: FP64 22,000 x 44,000 (467) takes 22.3 with 4
+// and 25.3 with 3. The lines follow from kSms: on a part with another number of SMs a launch may
+// take another variant, with the same results.
 template <class T>
 using PrimalKernel = void (*)(PrimalArgs<T>);
 template <class T>
