@@ -4,7 +4,7 @@
 // Launched one by one (step_kernels.cuh), an attempt of a small LP is latency: two launches, loads of
 // descriptors, state and matrix, and chains of dependent FP64 operations (64 cycles each on GB300),
 // around a microsecond of work: 13.4 us for a 203 x 406 and 13.1 for a 1,000 x 2,000 LP in FP64,
-// against 7.4 and 7.7 here (launch and staging, 5-6 us an interval, included). Here a cluster
+// against 7.2 and 7.5 here (launch and staging, 5-6 us an interval, included). Here a cluster
 // of up to 16 CTAs keeps the LP on chip for the interval: every CTA holds its share of both
 // matrices in shared memory (columns, values and the lanes' row structure, staged once per
 // launch) and the whole of the two gathered vectors, x^ / dx and y, into which the CTAs write their
@@ -28,7 +28,11 @@ namespace gpdhg {
 
 constexpr int kClusterThreads = kBlock + 32;   // a warp per tile, and one that decides
 constexpr int kClusterMax = 16;       // CTAs per cluster (above 8: non-portable, GB300 takes 16)
-constexpr int kClusterRounds = 4;     // plan CTAs per CTA and side, at most
+// Plan CTAs per CTA and side, at most. Each round more is a pass of every warp through both halves of
+// an attempt: FP64 7.0-7.6 us an attempt with one, 10.1-12.4 with two, 16.1-18.0 with three, against
+// 12.5-13.2 as step kernels; FP32 5.1-6.0, 7.3-9.4 and (three) 11.1-13.1, against 11.1-11.7. Random LPs of
+// 203 to 5,500 rows with 5 to 20 nonzeros; the room for four rounds cost the others 3-10%.
+constexpr int kClusterRounds = 2;
 constexpr int kClusterPlanCtas = kClusterMax * kClusterRounds;
 constexpr size_t kClusterShared = 200 * 1024;
 // Attempts per launch at most (a chunk normally takes its 1 to 64 accepted steps and a few
