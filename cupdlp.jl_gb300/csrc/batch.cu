@@ -466,8 +466,10 @@ struct BatchWorkspace {
     if (hbeg_p.empty()) {
       hbeg_p.resize(count + 1);
       hbeg_d.resize(count + 1);
-      CK(cudaMemcpy(hbeg_p.data(), plan_p.inst_cta_begin.get(), sizeof(int32_t) * (count + 1), cudaMemcpyDeviceToHost));
-      CK(cudaMemcpy(hbeg_d.data(), plan_d.inst_cta_begin.get(), sizeof(int32_t) * (count + 1), cudaMemcpyDeviceToHost));
+      const size_t bytes = sizeof(int32_t) * (count + 1);
+      CK(cudaMemcpyAsync(hbeg_p.data(), plan_p.inst_cta_begin.get(), bytes, cudaMemcpyDeviceToHost, B->stream));
+      CK(cudaMemcpyAsync(hbeg_d.data(), plan_d.inst_cta_begin.get(), bytes, cudaMemcpyDeviceToHost, B->stream));
+      CK(cudaStreamSynchronize(B->stream));
     }
     std::vector<int32_t> mp, md;
     auto collect = [&](const std::vector<int32_t>& begin, std::vector<int32_t>& map) {
@@ -480,10 +482,11 @@ struct BatchWorkspace {
     if (mp.empty() || md.empty()) return;  // nothing runs any more
     auto up = [&](DBuf<int32_t>& d, const std::vector<int32_t>& v) {
       d.alloc(v.size());
-      CK(cudaMemcpy(d.get(), v.data(), sizeof(int32_t) * v.size(), cudaMemcpyHostToDevice));
+      CK(cudaMemcpyAsync(d.get(), v.data(), sizeof(int32_t) * v.size(), cudaMemcpyHostToDevice, B->stream));
     };
     up(map_p, mp);
     up(map_d, md);
+    CK(cudaStreamSynchronize(B->stream));   // the host maps die here
     grid_p = (int)mp.size();
     grid_d = (int)md.size();
     for (cudaGraphExec_t& g : graphs) {

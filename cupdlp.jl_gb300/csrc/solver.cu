@@ -680,9 +680,13 @@ void init_state(gpdhg_problem* P, Workspace<T>& W, const gpdhg_params& prm, Loop
     std::vector<T> h(n);
     while (fail(k) > 0.001) {
       const double nx = std::sqrt(W.dot(W.tmp_n.get(), W.tmp_n.get(), n));
-      CK(cudaMemcpy(h.data(), W.tmp_n.get(), sizeof(T) * n, cudaMemcpyDeviceToHost));
+      // on the products' own stream, which waits for no other: a plain copy of pageable memory returns
+      // before its transfer ends
+      CK(cudaMemcpyAsync(h.data(), W.tmp_n.get(), sizeof(T) * n, cudaMemcpyDeviceToHost, s));
+      CK(cudaStreamSynchronize(s));
       for (auto& v : h) v = (T)((double)v / nx);
-      CK(cudaMemcpy(W.tmp_n.get(), h.data(), sizeof(T) * n, cudaMemcpyHostToDevice));
+      CK(cudaMemcpyAsync(W.tmp_n.get(), h.data(), sizeof(T) * n, cudaMemcpyHostToDevice, s));
+      CK(cudaStreamSynchronize(s));
       W.spmv(P->A, W.tmp_n.get(), W.tmp_m.get());
       W.spmv(P->At, W.tmp_m.get(), W.dx.get());
       CK(cudaMemcpyAsync(W.tmp_n.get(), W.dx.get(), sizeof(T) * n, cudaMemcpyDeviceToDevice, s));
